@@ -170,6 +170,8 @@ struct Tables {
     uint32_t slots = 0, tris = 0, ntiles = 0;
     int tile_shift = kTileShiftPlain;
     bool eye = false, any_texture = false;
+    bool order_free = false;  // the pass renders order-free (k_tile_free.cu)
+    bool occlude = false;  // some frame's pairs may be dropped behind a covering triangle (DevFrame::occlude)
     bool defer = false;  // every record a filled triangle whose colour can be deferred (k_tile.cuh)
 };
 

@@ -72,23 +72,32 @@ struct BinArgs {
     uint32_t nframes;
     int32_t tile_shift;         // tile edge = 1 << tile_shift
     uint32_t ntiles;            // tiles of all frames
-    uint32_t *rec_tiles;        // per record tile count, then its exclusive scan (in place)
+    uint32_t units, wpg;        // bin_units(nrec): work units of the record kernels, and units per 32 records
+    uint32_t *rec_tiles;        // per unit its pair count, then the exclusive scan (in place)
     uint32_t *keys, *vals;      // pair buffers (capacity >= pairs)
     uint32_t *keys_alt, *vals_alt;
     uint32_t *tile_count;       // per tile (ntiles + 1 entries)
     uint32_t *tile_area;        // per tile: pixels of its records' boxes inside it, summed (may be null)
+    uint32_t *tile_near;        // per tile: the occlusion bound (near_key; zero at launch); null when no
+                                // frame of the pass has one
     uint32_t *tile_start;       // exclusive scan of tile_count
     uint32_t *tile_frame;       // per tile: the frame owning it (written by the range pass; may be null)
     uint32_t *radix_hist;       // radix histograms
     uint32_t *scan_temp;
     uint32_t *total_dev;        // where the pair scan writes its total: the pairs generated
     uint32_t *sort_total_dev;   // a word the sort's histogram scans may overwrite
+    int32_t order_free;         // tile lists need no order (k_tile_free.cu)
     uint32_t npairs;            // pair capacity of keys/vals (writes beyond are dropped)
     int32_t sms;                // SMs of the device (grid sizes)
     uint32_t *debug;            // status word of the debug bounds checks
 };
 
+// The count launch also takes the occlusion bounds first (where tile_near is given).
+// Ordered passes: pairs per unit, scanned, and the pair total. Order-free passes: pairs per tile
+// in tile_count, their scan in tile_start, and the total; the expand launch then writes each
+// tile's list at tile_start and leaves the list's end there.
 int launch_bin_count(const BinArgs &a, cudaStream_t s);
+uint32_t bin_units(uint32_t nrec, int sms, uint32_t *wpg);  // at most nrec + 31
 int launch_bin_expand(const BinArgs &a, cudaStream_t s);
 // Stable sort of (tile, record) pairs by tile; result in keys/vals. Uses keys_alt/vals_alt
 // as ping-pong storage.
@@ -150,11 +159,14 @@ struct TileArgs {
     int32_t defer;               // every record is a filled triangle with deferrable colour (k_tile.cuh)
     uint32_t *debug;             // status word of the debug bounds checks
     uint32_t entries_cap;        // entries tile_vals holds (debug bounds checks)
+    int32_t order_free;          // the pass renders order-free: tile_start holds each list's end
 };
 
 // K4: CTAs take tiles from the work queue; for each: clears, then every triangle of the
 // tile in order through the full fragment pipeline (raster.c:532-724), then one write-back.
 int launch_tile(const TileArgs &a, cudaStream_t s);
+// the launch of an order-free pass (k_tile_free.cu)
+int launch_tile_free(const TileArgs &a, cudaStream_t s);
 // resident CTAs per SM of the K4 variant a launch with these arguments uses
 int tile_occupancy(const TileArgs &a);
 

@@ -358,17 +358,18 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
     ClearOp *hcl = reinterpret_cast<ClearOp *>(st.p + t.off_clears);
     DevFrame *hfr = reinterpret_cast<DevFrame *>(st.p + t.off_frames);
     uint32_t di = 0, vsb = 0, rsb = 0, clb = 0, slot_base = 0, tri_base = 0, tile_base = 0;
-    bool defer = true;
+    bool defer = true, order_free = ndraws > 0;
     for (uint32_t f = 0; f < nframes; f++) {
         const Pass &p = *frames[f].pass;
         const mtgl_dev *d = frames[f].dev;
         uint8_t *data = ds + frames[f].data_off;
+        bool occlude = !p.draws.empty(), one_func = true;
         for (const PendingDraw &pd : p.draws) {
             DevDraw dd = pd.d;
             if (dd.mode < GL_TRIANGLES || dd.mode > GL_POLYGON || dd.raster >= p.rasters.size() ||
                 p.rasters[dd.raster].rs.polygon_mode_front != GL_FILL ||
                 p.rasters[dd.raster].rs.polygon_mode_back != GL_FILL)
-                defer = false;  // points and lines read the stored colour
+                defer = occlude = false;  // points and lines read the stored colour
             if (pd.off_pos >= 0) dd.pos.ptr = data + pd.off_pos;
             if (pd.off_color >= 0) dd.color.ptr = data + pd.off_color;
             if (pd.off_tex >= 0) dd.tex.ptr = data + pd.off_tex;
@@ -392,8 +393,16 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
             const uint32_t c = R.fs.ctl;
             if ((c & FC_BLEND) || ((c & FC_ALPHA) && (c & FC_TEXTURE)) || !(c & (FC_MASK_ALL | FC_MASK_NONE)))
                 defer = false;  // a fragment reads the stored colour, or may be discarded after its depth test
+            // A frame's hidden pairs may be dropped when every fragment that passes its depth test
+            // replaces colour and depth, and only nearer (or equal) fragments pass.
+            const uint32_t need = FC_DEPTH | FC_DEPTH_WRITE | FC_MASK_ALL;
+            if ((c & (need | FC_STENCIL | FC_BLEND)) != need || ((c & FC_ALPHA) && (c & FC_TEXTURE)) ||
+                (R.rs.depth_func != GL_LESS && R.rs.depth_func != GL_LEQUAL) || !R.depth_rejection)
+                occlude = false;
+            one_func = one_func && R.rs.depth_func == p.rasters[0].rs.depth_func;
             hrs[rsb + i] = R;
         }
+        order_free = order_free && (p.draws.empty() || (occlude && one_func));
         if (!p.clears.empty()) memcpy(hcl + clb, p.clears.data(), p.clears.size() * sizeof(ClearOp));
         DevFrame F;
         memset(&F, 0, sizeof(F));
@@ -407,6 +416,8 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
         F.tile_base = tile_base;
         F.clear_base = clb;
         F.nclears = (uint32_t)p.clears.size();
+        F.occlude = occlude ? 1u : 0u;
+        t.occlude = t.occlude || occlude;
         hfr[f] = F;
         vsb += (uint32_t)p.vstates.size();
         rsb += (uint32_t)p.rasters.size();
@@ -418,6 +429,7 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
     t.ndraws = (uint32_t)ndraws;
     t.nrasters = (uint32_t)nrs;
     t.defer = defer && ndraws > 0;
+    t.order_free = order_free;
     t.nclears = (uint32_t)ncl;
     t.slots = (uint32_t)slots;
     t.tris = (uint32_t)tris;
@@ -465,11 +477,13 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     // clip list, its class words, the class-sorted list, the class counters and the emit list
     uint32_t *clip_list = nullptr;
     if ((rc = sc.take(S_CLIP_LIST, 4 * (size_t)tris + kClipBuckets, &clip_list))) return rc;
-    // tile counts, then (persistent ordered launches) the per-tile record-box coverage
+    // tile counts, then per tile the record-box coverage (classified launches) or else the
+    // occlusion bound
     if ((rc = sc.take(S_TILE_COUNT, 2 * ((size_t)ntiles + 1), &tile_count))) return rc;
     // record-box coverage per tile, for the split between tiles run by rounds and per record;
     // deferred-colour passes run every tile per record (their fragments are cheap: tests only)
     uint32_t *tile_area = (c.ctas && (c.order || c.classify) && !t.defer) ? tile_count + ntiles + 1 : nullptr;
+    uint32_t *tile_near = t.occlude && !tile_area ? tile_count + ntiles + 1 : nullptr;
     if ((rc = sc.take(S_TILE_START, (size_t)ntiles + 1, &tile_start))) return rc;
     uint32_t *tile_frame = nullptr;  // batches: each tile's frame, found once by the range pass
     if (t.nframes > 1 && (rc = sc.take(S_TILE_FRAME, ntiles, &tile_frame))) return rc;
@@ -481,12 +495,14 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         scan_n = std::max<uint32_t>(scan_n, (uint32_t)radix_hist_words(c.pair_cap));
         if ((rc = sc.take(S_RECORDS, (size_t)c.rec_cap * kRecWords, &records))) return rc;
         if (eye && (rc = sc.take(S_EYE_RECORDS, (size_t)c.rec_cap * kEyeWords, &eye_records))) return rc;
-        if ((rc = sc.take(S_REC_TILES, c.rec_cap, &rec_tiles))) return rc;
-        if ((rc = sc.take(S_KEYS, c.pair_cap, &keys))) return rc;
         if ((rc = sc.take(S_VALS, c.pair_cap, &vals))) return rc;
-        if ((rc = sc.take(S_KEYS_ALT, c.pair_cap, &keys_alt))) return rc;
-        if ((rc = sc.take(S_VALS_ALT, c.pair_cap, &vals_alt))) return rc;
-        if ((rc = sc.take(S_RADIX_HIST, radix_hist_words(c.pair_cap), &radix_hist))) return rc;
+        if (!t.order_free) {
+            if ((rc = sc.take(S_REC_TILES, bin_units(c.rec_cap, x.sms, nullptr), &rec_tiles))) return rc;
+            if ((rc = sc.take(S_KEYS, c.pair_cap, &keys))) return rc;
+            if ((rc = sc.take(S_KEYS_ALT, c.pair_cap, &keys_alt))) return rc;
+            if ((rc = sc.take(S_VALS_ALT, c.pair_cap, &vals_alt))) return rc;
+            if ((rc = sc.take(S_RADIX_HIST, radix_hist_words(c.pair_cap), &radix_hist))) return rc;
+        }
     }
     if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(scan_n), &scan_temp))) return rc;
     if (alloc_only) return MTGL_OK;
@@ -535,7 +551,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         rec_cap = o.nrec = x.h_totals[0];
         if ((rc = sc.take(S_RECORDS, (size_t)rec_cap * kRecWords, &records))) return rc;
         if (eye && (rc = sc.take(S_EYE_RECORDS, (size_t)rec_cap * kEyeWords, &eye_records))) return rc;
-        if ((rc = sc.take(S_REC_TILES, rec_cap, &rec_tiles))) return rc;
+        if (!t.order_free && (rc = sc.take(S_REC_TILES, bin_units(rec_cap, x.sms, nullptr), &rec_tiles))) return rc;
         if (rec_cap > scan_n) {
             scan_n = rec_cap;
             if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(scan_n), &scan_temp))) return rc;
@@ -548,8 +564,9 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     x.prof_mark();
 
     // ---- binning
-    CK(cudaMemsetAsync(tile_count, 0, (tile_area ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
-    CK(cudaMemsetAsync(tile_start, 0, ((size_t)ntiles + 1) * sizeof(uint32_t), s));
+    CK(cudaMemsetAsync(tile_count, 0, (tile_area || tile_near ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
+    // (an order-free pass's scan writes every tile's start)
+    if (!t.order_free || !rec_cap) CK(cudaMemsetAsync(tile_start, 0, ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     BinArgs ba;
     memset(&ba, 0, sizeof(ba));
     ba.records = records;
@@ -562,30 +579,34 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ba.rec_tiles = rec_tiles;
     ba.tile_count = tile_count;
     ba.tile_area = tile_area;
+    ba.tile_near = tile_near;
     ba.tile_start = tile_start;
     ba.tile_frame = tile_frame;
     ba.total_dev = x.d_totals + 1;
     ba.sort_total_dev = x.d_totals + 3;
     ba.debug = x.d_totals + kDebugStatusWord;
+    ba.order_free = t.order_free ? 1 : 0;
     ba.scan_temp = scan_temp;
     ba.sms = x.sms;
     uint32_t pair_cap = c.pair_cap;
+    ba.units = bin_units(rec_cap, x.sms, &ba.wpg);
     if (rec_cap) {
         launches += launch_bin_count(ba, s);
-        launches += launch_scan(rec_tiles, rec_tiles, rec_cap, scan_temp, x.d_totals + 1, x.d_totals + kDebugStatusWord, s);
         CK(cudaGetLastError());
         if (c.exact) {
             CK(cudaMemcpyAsync(x.h_totals + 1, x.d_totals + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             pair_cap = o.npairs = x.h_totals[1];
-            const size_t hist = radix_hist_words(pair_cap);
-            if ((rc = sc.take(S_KEYS, pair_cap, &keys)) || (rc = sc.take(S_VALS, pair_cap, &vals)) ||
-                (rc = sc.take(S_KEYS_ALT, pair_cap, &keys_alt)) || (rc = sc.take(S_VALS_ALT, pair_cap, &vals_alt)) ||
-                (rc = sc.take(S_RADIX_HIST, hist, &radix_hist)))
-                return rc;
-            const uint32_t need = std::max<uint32_t>(std::max<uint32_t>((uint32_t)hist, rec_cap), scan_n);
-            if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(need), &scan_temp))) return rc;
-            ba.scan_temp = scan_temp;
+            if ((rc = sc.take(S_VALS, pair_cap, &vals))) return rc;
+            if (!t.order_free) {
+                const size_t hist = radix_hist_words(pair_cap);
+                if ((rc = sc.take(S_KEYS, pair_cap, &keys)) || (rc = sc.take(S_KEYS_ALT, pair_cap, &keys_alt)) ||
+                    (rc = sc.take(S_VALS_ALT, pair_cap, &vals_alt)) || (rc = sc.take(S_RADIX_HIST, hist, &radix_hist)))
+                    return rc;
+                const uint32_t need = std::max<uint32_t>(std::max<uint32_t>((uint32_t)hist, rec_cap), scan_n);
+                if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(need), &scan_temp))) return rc;
+                ba.scan_temp = scan_temp;
+            }
         }
         ba.keys = keys;
         ba.vals = vals;
@@ -594,8 +615,10 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         ba.radix_hist = radix_hist;
         ba.npairs = pair_cap;
         launches += launch_bin_expand(ba, s);
-        launches += launch_bin_sort(ba, s);
-        launches += launch_tile_ranges(ba, s);
+        if (!t.order_free) {
+            launches += launch_bin_sort(ba, s);
+            launches += launch_tile_ranges(ba, s);
+        }
     } else {
         CK(cudaMemsetAsync(x.d_totals + 1, 0, sizeof(uint32_t), s));
     }
@@ -623,7 +646,13 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ta.any_texture = t.any_texture ? 1 : 0;
     ta.defer = t.defer ? 1 : 0;
     ta.fragments = x.d_frags;
-    if (c.ctas) {
+    ta.order_free = t.order_free && rec_cap ? 1 : 0;
+    if (ta.order_free) {  // one CTA per tile: no work queue
+        if (order) {
+            launches += launch_tile_order(tile_count, nullptr, ntiles, t.tile_shift, order_aux, order, x.sms, s);
+            ta.order = order;
+        }
+    } else if (c.ctas) {
         ta.queue = order_aux + kOrderQueues;
         if (order) {  // clears the queue heads too
             launches += launch_tile_order(tile_count, tile_area, ntiles, t.tile_shift, order_aux, order, x.sms, s);

@@ -3,10 +3,12 @@
 // No counterpart in the reference, which scans every triangle's bounding box on one thread
 // (raster.c:532-724). Here each record is expanded into one (tile, record) pair per tile
 // (8, 16 or 32 pixels square) of its clamped bounding box in which it can cover a pixel (an
-// exact edge test per tile for triangles); pairs are generated in submission order and a
-// stable LSD radix sort on the tile id (warp match-any ranking plus prefix sums) groups
-// them by tile while keeping that order inside every tile. The tile kernel then walks each
-// list front to back, so blending and stencil updates happen in GL order.
+// exact edge test per tile for triangles) and is not hidden there by a triangle that covers
+// the whole tile. Pairs are generated in submission order and a stable LSD radix sort on the
+// tile id (warp match-any ranking plus prefix sums) groups them by tile while keeping that
+// order inside every tile. The tile kernel then walks each list front to back, so blending
+// and stencil updates happen in GL order. Passes whose result does not depend on that order
+// (k_tile_free.cu) skip the sort: their pairs go straight to the tiles' lists.
 #include <algorithm>
 
 #include "dev_kernels.h"
@@ -164,170 +166,298 @@ int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, u
 }
 
 // ------------------------------------------------------------------ record -> tiles
+//
+// Three kernels run over the (record, tile of its box) candidates: the occlusion bounds, the
+// pair count and the pair writes. Boxes hold from one tile to thousands, so a warp takes 32
+// records, each lane sets one up into shared memory (BoxRec), and the warp then runs over the
+// candidates of all 32 in order, 32 at a time, each lane finding its candidate's record in the
+// prefix sums of the tile counts: every lane has a candidate whatever the boxes are. Passes of
+// few records (full-screen quads, sprites) split a group's candidates over A.wpg warps in
+// contiguous parts. Both keep submission order: a part's pairs follow the earlier parts'.
 
-// The setup kernel clamps every bbox to its framebuffer; the clamps here only keep tile
-// indices inside the frame's tile grid whatever a record holds. Returns the frame.
-__device__ __forceinline__ const DevFrame &rec_tile_box(const float *rec, const BinArgs &A, int &tx0, int &ty0,
-                                                        int &tx1, int &ty1)
-{
-    const float4 b1 = __ldg(reinterpret_cast<const float4 *>(rec) + 1);
-    const float4 b2 = __ldg(reinterpret_cast<const float4 *>(rec) + 2);
-    const uint32_t f = min(__float_as_uint(__ldg(rec + R_FRAME)), A.nframes - 1);
-    const DevFrame &F = A.frames[f];
-    const int sh = A.tile_shift;
-    tx0 = min(max(__float_as_int(b1.z), 0), F.dims.width - 1) >> sh;
-    ty0 = min(max(__float_as_int(b1.w), 0), F.dims.height - 1) >> sh;
-    tx1 = max(min(__float_as_int(b2.x), F.dims.width - 1) >> sh, tx0);
-    ty1 = max(min(__float_as_int(b2.y), F.dims.height - 1) >> sh, ty0);
-    return F;
-}
+constexpr int kRecWarps = 4;  // warps per CTA of the record kernels
 
 __device__ __forceinline__ uint32_t records_in(const BinArgs &A) { return min(*A.nrec_dev, A.nrec); }
 
-// The tiles of a record's box that get a pair: every tile for points and lines; for a
-// triangle, the tiles in which its coverage test (edge functions at integer pixel positions,
-// raster.c:299-302, 534-536) can pass. k_bin_count counts them and k_bin_expand writes them,
-// with this one test.
-//
-// The record's positions and per-edge differences are integer-valued floats. When every
-// product (px - ax) * A, (py - ay) * B that the per-pixel test forms over the box's tiles is
-// below 2^24 in magnitude, those products are exact, so each edge function's sign per pixel
-// is the sign of the exact integer. Then each edge's largest value over a tile (a corner:
-// the function is affine) is an int32 stepped per tile column and row, and a tile whose
-// largest value is negative for some edge has no pixel the test passes (for a negative
-// area the signs flip). Otherwise every tile of the box gets a pair.
-struct RecTiles {
-    int tx0, ty0, w, cnt;  // the box in tiles, row-major, cnt tiles
-    int mode;              // kAll, kNone or kTest
-    int e00[3], sx[3], sy[3];  // per edge: value at the first tile's corner, steps per column / row
-};
-constexpr int kAll = 0, kNone = 1, kTest = 2;
-constexpr int kTestMinTiles = 4;  // smaller boxes keep every tile: little to drop, and the set-up dominates
-
-__device__ __forceinline__ const DevFrame &rec_tiles_of(const BinArgs &A, uint32_t r, RecTiles &t)
+// the frame that owns tile t: the last whose first tile is at or before it
+__device__ __forceinline__ uint32_t frame_of_tile(const BinArgs &A, uint32_t t)
 {
-    const float *rec = A.records + (size_t)r * kRecWords;
-    int tx1, ty1;
-    const DevFrame &F = rec_tile_box(rec, A, t.tx0, t.ty0, tx1, ty1);
-    t.w = tx1 - t.tx0 + 1;
-    t.cnt = t.w * (ty1 - t.ty0 + 1);
-    const float4 *q = reinterpret_cast<const float4 *>(rec);
-    t.mode = kAll;
-    if (t.cnt < kTestMinTiles) return F;
-    const float4 q12 = __ldg(q + 12);
-    if (((__float_as_uint(q12.x) >> kRecTypeShift) & 3u) != REC_TRI) return F;
-    const float4 q0 = __ldg(q + 0), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q13 = __ldg(q + 13);
-    const float area = q2.z;
-    if (!(area > 0.0f) && !(area < 0.0f)) {  // zero or NaN area: the test never passes
-        t.mode = kNone;
-        return F;
+    uint32_t lo = 0, hi = A.nframes - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (A.frames[mid].tile_base <= t) lo = mid;
+        else hi = mid - 1;
     }
-    const int sh = A.tile_shift, ts = 1 << sh;
-    const int xl = t.tx0 << sh, xh = (tx1 << sh) + ts - 1, yl = t.ty0 << sh, yh = (ty1 << sh) + ts - 1;
+    return lo;
+}
+
+// A triangle record's edges as integers for an exact test over pixels [xl, xh] x [yl, yh]:
+// edge k is (x - iax) * a - (y - iay) * b, sign-flipped for a negative area so that covered
+// means >= 0. The record's positions and per-edge differences are integer-valued floats; when
+// every product (px - ax) * A, (py - ay) * B that the per-pixel test (raster.c:299-302,
+// 534-536) forms there is below 2^24 in magnitude, those products are exact, so each edge
+// function's sign per pixel is the sign of the exact integer. False when one could be inexact.
+__device__ __forceinline__ bool exact_edges(const float4 &q0, const float4 &q1, const float4 &q12, const float4 &q13,
+                                            bool pos, int xl, int xh, int yl, int yh, int *iax, int *iay, int *a, int *b)
+{
     const float ax[3] = {q0.z, q1.x, q0.x}, ay[3] = {q0.w, q1.y, q0.y};
     const float ea[3] = {q12.y, q12.w, q13.y}, eb[3] = {q12.z, q13.x, q13.z};
-    const bool pos = area > 0.0f;
+    bool ok = true;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
         constexpr float kLim = 16777216.0f;  // 2^24
-        if (!(fabsf(ax[k]) < kLim && fabsf(ay[k]) < kLim && fabsf(ea[k]) < kLim && fabsf(eb[k]) < kLim)) return F;
-        const int iax = (int)ax[k], iay = (int)ay[k];
-        const int a = pos ? (int)ea[k] : -(int)ea[k], b = pos ? (int)eb[k] : -(int)eb[k];
-        const long long mx = max(llabs((long long)xl - iax), llabs((long long)xh - iax)) * llabs((long long)a);
-        const long long my = max(llabs((long long)yl - iay), llabs((long long)yh - iay)) * llabs((long long)b);
-        if (mx >= (1ll << 24) || my >= (1ll << 24)) return F;
-        // (x - ax) * a - (y - ay) * b is largest over a tile at x = right edge when a >= 0,
-        // y = top row when b >= 0
-        const int cx = xl + (a >= 0 ? ts - 1 : 0), cy = yl + (b >= 0 ? 0 : ts - 1);
-        t.e00[k] = (cx - iax) * a - (cy - iay) * b;
-        t.sx[k] = a * ts;
-        t.sy[k] = b * ts;
+        ok = ok && fabsf(ax[k]) < kLim && fabsf(ay[k]) < kLim && fabsf(ea[k]) < kLim && fabsf(eb[k]) < kLim;
+        iax[k] = (int)ax[k];
+        iay[k] = (int)ay[k];
+        a[k] = pos ? (int)ea[k] : -(int)ea[k];
+        b[k] = pos ? (int)eb[k] : -(int)eb[k];
+        const long long mx = max(llabs((long long)xl - iax[k]), llabs((long long)xh - iax[k])) * llabs((long long)a[k]);
+        const long long my = max(llabs((long long)yl - iay[k]), llabs((long long)yh - iay[k])) * llabs((long long)b[k]);
+        ok = ok && mx < (1ll << 24) && my < (1ll << 24);
     }
-    t.mode = kTest;
-    return F;
-}
-
-// the i-th tile of the box (row-major) gets a pair
-__device__ __forceinline__ bool tile_gets_pair(const RecTiles &t, int i)
-{
-    if (t.mode != kTest) return t.mode == kAll;
-    const int col = i % t.w, row = i / t.w;
-    bool ok = true;
-#pragma unroll
-    for (int k = 0; k < 3; k++) ok = ok && t.e00[k] + col * t.sx[k] - row * t.sy[k] >= 0;
     return ok;
 }
 
-constexpr uint32_t kCountLanes = 2;  // lanes per record in k_bin_count (16 records per warp)
-
-// pairs per record; records past the real count get 0 so the scan over the capacity is exact
-__global__ void __launch_bounds__(256) k_bin_count(BinArgs A)
+__device__ __forceinline__ bool has_depth_bound(uint32_t flags)
 {
-    const uint32_t n = records_in(A);
-    constexpr uint32_t L = kCountLanes, G = 32 / kCountLanes;
-    const uint32_t lane = threadIdx.x & 31u, sub = lane / L, sl = lane % L;
-    const uint32_t gmask = ((1u << L) - 1u) << (sub * L);
-    const uint32_t groups = gridDim.x * (blockDim.x >> 5) * G;
-    for (uint32_t r0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G; r0 < A.nrec; r0 += groups) {
-        const uint32_t r = r0 + sub;
-        if (r >= A.nrec) continue;
-        uint32_t c = 0;
-        if (r < n) {
-            RecTiles t;
-            rec_tiles_of(A, r, t);
-            if (t.mode == kAll) {
-                c = sl == 0 ? (uint32_t)t.cnt : 0u;
-            } else if (t.mode == kTest) {
-                for (int i = (int)sl; i < t.cnt; i += (int)L) c += tile_gets_pair(t, i) ? 1u : 0u;
-            }
-        }
-        c = __reduce_add_sync(gmask, c);
-        if (sl == 0) A.rec_tiles[r] = c;
-    }
+    const uint32_t zc = (flags >> 1) & 3u;
+    return ((flags >> kRecTypeShift) & 3u) == REC_TRI && (zc == ZC_LESS || zc == ZC_LEQUAL);
 }
 
-// A group of L lanes per record (L = 32 / G, G records per warp from the average pairs per
-// record: 1 for large triangles, up to 8 for small ones, so that a warp has several records'
-// loads in flight): the group tests its record's box tiles row-major and writes the pairs of
-// those that get one, in that order (pairs stay in submission order within every tile).
-__global__ void __launch_bounds__(256) k_bin_expand(BinArgs A)
+// A record's candidate tiles, row-major: `w` per row from (tx0, ty0).
+enum BoxMode : uint32_t {
+    BOX_TEST = 1u,  // some tile may fail the edge test: e00 + col * sx - row * sy per edge decides
+    BOX_HIDE = 2u,  // the tile's occlusion bound may hide the record
+};
+struct BoxRec {
+    int tx0, ty0, w;
+    uint32_t mode;
+    int e00[3];
+    float dmin;              // lower bound of the record's depths
+    int sx[3];
+    uint32_t mn;             // the record's box in pixels, x | y << 16
+    int sy[3];
+    uint32_t mx;
+    float4 zp;               // depth plane
+    uint32_t tile0, tiles_x; // global tile id at (tx0, ty0), tiles per row of its frame
+    float inv_w;
+    uint32_t pad;
+};
+static_assert(sizeof(BoxRec) % 16 == 0, "16-byte shared-memory words");
+
+__device__ __forceinline__ uint32_t pack_xy(int x, int y) { return (uint32_t)x | ((uint32_t)y << 16); }
+
+constexpr int kTestMinTiles = 4;  // smaller boxes keep every tile: little to drop, and the set-up dominates
+
+// Sets up record r; returns its candidate count. OCCLUDE: the tiles it may cover whole.
+// Otherwise the tiles of its box; the pairs are those where its coverage test can pass (a tile
+// in which some edge function is negative at its largest, a corner, holds no covered pixel),
+// less the hidden ones; points, lines and small boxes keep every tile not hidden.
+template <bool OCCLUDE>
+__device__ __forceinline__ int box_of(const BinArgs &A, uint32_t r, BoxRec &t)
 {
-    const uint32_t n = records_in(A);
-    const uint32_t avg = n ? max(1u, *A.total_dev / n) : 1u;
-    const uint32_t G = avg >= 32u ? 1u : (avg >= 16u ? 2u : (avg >= 8u ? 4u : 8u));
-    const uint32_t L = 32u / G;
-    const uint32_t lane = threadIdx.x & 31u, sub = lane / L, sl = lane % L;
-    const uint32_t lmask = L == 32u ? 0xFFFFFFFFu : (1u << L) - 1u;
-    const uint32_t gmask = lmask << (sub * L);
-    const uint32_t groups = gridDim.x * (blockDim.x >> 5) * G;
-    const int sh = A.tile_shift;
-    for (uint32_t r = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * G + sub; r < n; r += groups) {
-        RecTiles t;
-        const DevFrame &F = rec_tiles_of(A, r, t);
-        const float *rec = A.records + (size_t)r * kRecWords;
-        const float4 b1 = __ldg(reinterpret_cast<const float4 *>(rec) + 1);
-        const float4 b2 = __ldg(reinterpret_cast<const float4 *>(rec) + 2);
-        const int bx0 = __float_as_int(b1.z), by0 = __float_as_int(b1.w);
-        const int bx1 = __float_as_int(b2.x), by1 = __float_as_int(b2.y);
-        const uint32_t base = A.rec_tiles[r];
-        uint32_t run = 0;  // pairs of this record written so far
-        for (int i0 = 0; i0 < t.cnt; i0 += (int)L) {
-            const int i = i0 + (int)sl;
-            const int tx = t.tx0 + i % t.w, ty = t.ty0 + i / t.w;
-            const bool get = i < t.cnt && tile_gets_pair(t, i);
-            const uint32_t m = (__ballot_sync(gmask, get) >> (sub * L)) & lmask;
-            const uint32_t at = base + run + (uint32_t)__popc(m & ((1u << sl) - 1u));
-            run += (uint32_t)__popc(m);
-            if (!get || at >= A.npairs) continue;
-            const uint32_t tile = F.tile_base + (uint32_t)(ty * F.dims.tiles_x + tx);
-            A.keys[at] = tile;
-            A.vals[at] = r;
-            if (A.tile_area) {  // pixels of the record's box inside this tile
-                const int ox = min(bx1, ((tx + 1) << sh) - 1) - max(bx0, tx << sh) + 1;
-                const int oy = min(by1, ((ty + 1) << sh) - 1) - max(by0, ty << sh) + 1;
-                atomicAdd(A.tile_area + tile, (uint32_t)(ox * oy));
-            }
+    const float4 *q = reinterpret_cast<const float4 *>(A.records + (size_t)r * kRecWords);
+    const float4 q1 = __ldg(q + 1), q2 = __ldg(q + 2), q12 = __ldg(q + 12), q13 = __ldg(q + 13);
+    const DevFrame &F = A.frames[min(__float_as_uint(q13.w), A.nframes - 1)];
+    const int sh = A.tile_shift, ts = 1 << sh;
+    const int W = F.dims.width, H = F.dims.height;
+    // set-up clamps every box to its framebuffer; the clamps here only keep tile indices inside
+    // the frame's grid whatever a record holds
+    const int mnx = min(max(__float_as_int(q1.z), 0), W - 1), mny = min(max(__float_as_int(q1.w), 0), H - 1);
+    const int mxx = max(min(__float_as_int(q2.x), W - 1), mnx), mxy = max(min(__float_as_int(q2.y), H - 1), mny);
+    const uint32_t flags = __float_as_uint(q12.x);
+    const bool bounded = A.tile_near && F.occlude && has_depth_bound(flags);
+    const float area = q2.z;
+    int tx1, ty1;
+    if (OCCLUDE) {
+        // the tiles wholly inside the box, whose right and bottom sides may be the framebuffer's
+        t.tx0 = (mnx + ts - 1) >> sh;
+        t.ty0 = (mny + ts - 1) >> sh;
+        tx1 = mxx == W - 1 ? (W - 1) >> sh : ((mxx + 1) >> sh) - 1;
+        ty1 = mxy == H - 1 ? (H - 1) >> sh : ((mxy + 1) >> sh) - 1;
+        if (!bounded || tx1 < t.tx0 || ty1 < t.ty0 || !(area > 0.0f || area < 0.0f)) return 0;
+        t.zp = __ldg(q + 14);
+        if (!isfinite(t.zp.w)) return 0;  // no plane
+    } else {
+        t.tx0 = mnx >> sh;
+        t.ty0 = mny >> sh;
+        tx1 = mxx >> sh;
+        ty1 = mxy >> sh;
+    }
+    t.w = tx1 - t.tx0 + 1;
+    const int cnt = t.w * (ty1 - t.ty0 + 1);
+    t.tile0 = F.tile_base + (uint32_t)(t.ty0 * F.dims.tiles_x + t.tx0);
+    t.tiles_x = (uint32_t)F.dims.tiles_x;
+    t.inv_w = 1.0f / (float)t.w;
+    t.mn = pack_xy(mnx, mny);
+    t.mx = pack_xy(mxx, mxy);
+    t.mode = 0u;
+    if (!OCCLUDE) {
+        if (bounded) {
+            t.mode = BOX_HIDE;
+            t.dmin = __ldg(reinterpret_cast<const float *>(q) + R_DMIN);
+            t.zp = __ldg(q + 14);
         }
+        if (cnt < kTestMinTiles || ((flags >> kRecTypeShift) & 3u) != REC_TRI) return cnt;
+        if (!(area > 0.0f) && !(area < 0.0f)) return 0;  // zero or NaN area: the test never passes
+    }
+    const float4 q0 = __ldg(q + 0);
+    int iax[3], iay[3], a[3], b[3];
+    const int xl = t.tx0 << sh, yl = t.ty0 << sh;
+    if (!exact_edges(q0, q1, q12, q13, area > 0.0f, xl, (tx1 << sh) + ts - 1, yl, (ty1 << sh) + ts - 1, iax, iay, a, b))
+        return OCCLUDE ? 0 : cnt;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        // (x - ax) * a - (y - ay) * b is largest over a tile at its right edge when a >= 0 and its
+        // top row when b >= 0; smallest at the opposite corner
+        const bool right = (a[k] >= 0) != OCCLUDE, bottom = (b[k] >= 0) == OCCLUDE;
+        t.e00[k] = (xl + (right ? ts - 1 : 0) - iax[k]) * a[k] - (yl + (bottom ? ts - 1 : 0) - iay[k]) * b[k];
+        t.sx[k] = a[k] * ts;
+        t.sy[k] = b[k] * ts;
+    }
+    t.mode |= BOX_TEST;
+    return cnt;
+}
+
+// the box's i-th candidate as a column and row
+__device__ __forceinline__ void box_tile(const BoxRec &t, int i, int &col, int &row)
+{
+    // (i + 1/2) / w lies at least 1/(2w) from an integer, and the float result is within
+    // i / w * 2^-22 of it: exact below 2^20
+    row = i < (1 << 20) ? (int)(((float)i + 0.5f) * t.inv_w) : i / t.w;
+    col = i - row * t.w;
+}
+
+// the record gets a pair in this tile
+__device__ __forceinline__ bool tile_gets_pair(const BinArgs &A, const BoxRec &t, int col, int row)
+{
+    if (t.mode & BOX_TEST) {
+        bool ok = true;
+#pragma unroll
+        for (int k = 0; k < 3; k++) ok = ok && t.e00[k] + col * t.sx[k] - row * t.sy[k] >= 0;
+        if (!ok) return false;
+    }
+    if (!(t.mode & BOX_HIDE)) return true;
+    const uint32_t bound = __ldg(A.tile_near + t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col);
+    const int sh = A.tile_shift, x = (t.tx0 + col) << sh, y = (t.ty0 + row) << sh, ts = 1 << sh;
+    const int mnx = (int)(t.mn & 0xFFFFu), mny = (int)(t.mn >> 16), mxx = (int)(t.mx & 0xFFFFu), mxy = (int)(t.mx >> 16);
+    const float lo = fmaxf(t.dmin, depth_plane_bound(t.zp, mnx, mny, max(x, mnx), min(x + ts - 1, mxx), max(y, mny),
+                                                     min(y + ts - 1, mxy)));
+    return near_key(lo) >= bound;  // else strictly beyond it: no fragment of the record survives the tile
+}
+
+// Occlusion bounds (frames with DevFrame::occlude: every passing fragment replaces colour and
+// depth, and only nearer or equal ones pass). A triangle that covers every pixel of a tile
+// leaves no stored depth there beyond its own largest depth in the tile, whatever else is
+// drawn before or after it; so a record whose smallest depth in the tile is beyond that
+// changes nothing there, and its pair is dropped. Coverage is the exact edge test at the
+// tile's corners (clipped to the framebuffer and inside the record's box), the depths are the
+// plane's bounds. The bound of a tile is the nearest such depth (near_key, atomicMax).
+__device__ __forceinline__ void take_bound(const BinArgs &A, const BoxRec &t, int col, int row)
+{
+    const int sh = A.tile_shift, ts = 1 << sh;
+    const int xl = (t.tx0 + col) << sh, yl = (t.ty0 + row) << sh;
+    const int W = (int)(t.mx & 0xFFFFu) + 1, H = (int)(t.mx >> 16) + 1;  // the box holds the tile's pixels
+    const int cx = max(xl + ts - W, 0), cy = max(yl + ts - H, 0);        // those beyond the framebuffer
+    bool all = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        // the corner moves in by the clipped pixels
+        const int e = t.e00[k] + col * t.sx[k] - row * t.sy[k] + max(-(t.sx[k] >> sh), 0) * cx +
+                      max(t.sy[k] >> sh, 0) * cy;
+        all = all && e >= 0;
+    }
+    if (!all) return;
+    const float up = depth_plane_upper(t.zp, (int)(t.mn & 0xFFFFu), (int)(t.mn >> 16), xl, xl + ts - 1 - cx, yl,
+                                       yl + ts - 1 - cy);
+    if (!(up < INFINITY)) return;
+    const uint32_t key = near_key(up);
+    uint32_t *at = A.tile_near + t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
+    // most records of a deep tile are not the nearest by then: look before the atomic (an old
+    // value only costs an atomic)
+    if (key > __ldcg(at)) atomicMax(at, key);
+}
+
+// The passes over the candidates: occlusion bounds; pairs per unit and the pair writes (ordered
+// passes, sorted by tile afterwards); and, for order-free passes (k_tile_free.cu), pairs per
+// tile and the record indices straight into the tiles' lists, in whatever order they come.
+enum RecPass { PASS_OCCLUDE, PASS_COUNT, PASS_EXPAND, PASS_COUNT_FREE, PASS_EXPAND_FREE };
+
+template <RecPass PASS>
+__global__ void __launch_bounds__(kRecWarps * 32) k_bin_records(BinArgs A)
+{
+    __shared__ BoxRec s_box[kRecWarps][32];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    const uint32_t n = records_in(A);
+    BoxRec *box = s_box[warp];
+    if (PASS == PASS_COUNT_FREE && A.tile_frame)
+        for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.ntiles; t += gridDim.x * blockDim.x)
+            A.tile_frame[t] = frame_of_tile(A, t);
+    for (uint32_t u = blockIdx.x * kRecWarps + warp; u < A.units; u += gridDim.x * kRecWarps) {
+        // unit u: part u % wpg of the candidates of records [r0, r0 + 32)
+        const uint32_t r0 = u / A.wpg * 32u, part = u % A.wpg;
+        uint32_t kept = 0;
+        if (r0 < n) {
+            BoxRec b;
+            const int cnt = r0 + lane < n ? box_of<PASS == PASS_OCCLUDE>(A, r0 + lane, b) : 0;
+            uint32_t incl = warp_incl_scan((uint32_t)cnt);
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            if (cnt) box[lane] = b;
+            __syncwarp();
+            const uint32_t per = ((total + A.wpg - 1) / A.wpg + 31u) & ~31u;
+            const uint32_t lo = min(part * per, total), hi = min(lo + per, total);
+            uint32_t at = PASS == PASS_EXPAND ? A.rec_tiles[u] : 0u;
+            for (uint32_t c0 = lo; c0 < hi; c0 += 32) {
+                const uint32_t c = c0 + lane;
+                // the record: the first lane whose inclusive sum exceeds c
+                uint32_t j = 0;
+#pragma unroll
+                for (uint32_t step = 16; step; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= c) j += step;
+                const uint32_t before = __shfl_sync(0xffffffffu, incl - (uint32_t)cnt, j & 31u);
+                bool get = false;
+                int col = 0, row = 0;
+                if (c < hi) {
+                    const BoxRec &t = box[j];
+                    box_tile(t, (int)(c - before), col, row);
+                    if (PASS == PASS_OCCLUDE) take_bound(A, t, col, row);
+                    else get = tile_gets_pair(A, t, col, row);
+                }
+                if (PASS == PASS_OCCLUDE) continue;
+                if (PASS == PASS_COUNT_FREE || PASS == PASS_EXPAND_FREE) {
+                    if (!get) continue;
+                    const BoxRec &t = box[j];
+                    const uint32_t tile = t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
+                    if (!debug_check(A.debug, tile < A.ntiles, DBG_BIN_TILE)) continue;
+                    if (PASS == PASS_COUNT_FREE) {
+                        atomicAdd(A.tile_count + tile, 1u);
+                    } else {
+                        const uint32_t pos = atomicAdd(A.tile_start + tile, 1u);
+                        if (pos < A.npairs) A.vals[pos] = r0 + j;
+                    }
+                    continue;
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, get);
+                if (PASS == PASS_EXPAND && get) {
+                    const uint32_t pos = at + kept + (uint32_t)__popc(m & below);
+                    if (pos < A.npairs) {
+                        const BoxRec &t = box[j];
+                        const uint32_t tile = t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
+                        A.keys[pos] = tile;
+                        A.vals[pos] = r0 + j;
+                        if (A.tile_area) {  // pixels of the record's box inside this tile
+                            const int sh = A.tile_shift, x = (t.tx0 + col) << sh, y = (t.ty0 + row) << sh;
+                            const int ox = min((int)(t.mx & 0xFFFFu), x + (1 << sh) - 1) - max((int)(t.mn & 0xFFFFu), x) + 1;
+                            const int oy = min((int)(t.mx >> 16), y + (1 << sh) - 1) - max((int)(t.mn >> 16), y) + 1;
+                            atomicAdd(A.tile_area + tile, (uint32_t)(ox * oy));
+                        }
+                    }
+                }
+                kept += (uint32_t)__popc(m);
+            }
+            __syncwarp();
+        }
+        if (PASS == PASS_COUNT && lane == 0) A.rec_tiles[u] = kept;  // units past the records: none
     }
 }
 
@@ -353,21 +483,13 @@ __global__ void __launch_bounds__(256) k_tile_bounds(BinArgs A)
 }
 
 // end position - start = count; a tile without pairs has both still zero. Also the frame
-// that owns each tile (the last frame whose first tile is at or before it), so the tile
-// kernel reads it instead of searching the frame table per tile.
+// that owns each tile, so the tile kernel reads it instead of searching the frame table per
+// tile.
 __global__ void __launch_bounds__(256) k_tile_counts(BinArgs A)
 {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.ntiles; t += gridDim.x * blockDim.x) {
         A.tile_count[t] -= A.tile_start[t];
-        if (A.tile_frame) {
-            uint32_t lo = 0, hi = A.nframes - 1;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi + 1) >> 1;
-                if (A.frames[mid].tile_base <= t) lo = mid;
-                else hi = mid - 1;
-            }
-            A.tile_frame[t] = lo;
-        }
+        if (A.tile_frame) A.tile_frame[t] = frame_of_tile(A, t);
     }
 }
 
@@ -378,18 +500,42 @@ int launch_tile_ranges(const BinArgs &a, cudaStream_t s)
     return a.npairs ? 2 : 1;
 }
 
+// Warps per group of 32 records: the group count alone fills the GPU (64 warps per SM) from
+// about 300,000 records up; fewer groups split their candidates, up to 32 ways.
+uint32_t bin_units(uint32_t nrec, int sms, uint32_t *wpg)
+{
+    const uint32_t groups = (nrec + 31u) / 32u, warps = (uint32_t)(sms > 0 ? sms : 1) * 64u;
+    uint32_t k = 1;
+    while (k < 32 && (uint64_t)groups * k < warps) k *= 2;
+    if (wpg) *wpg = k;
+    return groups * k;
+}
+
+namespace {
+
+template <RecPass PASS>
+int launch_records(const BinArgs &a, cudaStream_t s)
+{
+    k_bin_records<PASS><<<stride_grid((uint64_t)a.units * 32, kRecWarps * 32, 2 * a.sms), kRecWarps * 32, 0, s>>>(a);
+    return 1;
+}
+
+}  // namespace
+
 int launch_bin_count(const BinArgs &a, cudaStream_t s)
 {
     if (!a.nrec) return 0;
-    k_bin_count<<<stride_grid((uint64_t)a.nrec * kCountLanes, 256, a.sms), 256, 0, s>>>(a);
-    return 1;
+    const int occlude = a.tile_near ? launch_records<PASS_OCCLUDE>(a, s) : 0;
+    if (!a.order_free) return occlude + launch_records<PASS_COUNT>(a, s) +
+                              launch_scan(a.rec_tiles, a.rec_tiles, a.units, a.scan_temp, a.total_dev, a.debug, s);
+    return occlude + launch_records<PASS_COUNT_FREE>(a, s) +
+           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.total_dev, a.debug, s);
 }
 
 int launch_bin_expand(const BinArgs &a, cudaStream_t s)
 {
     if (!a.nrec) return 0;
-    k_bin_expand<<<stride_grid((uint64_t)a.nrec * 32, 256, a.sms), 256, 0, s>>>(a);
-    return 1;
+    return a.order_free ? launch_records<PASS_EXPAND_FREE>(a, s) : launch_records<PASS_EXPAND>(a, s);
 }
 
 // ------------------------------------------------------------------ persistent work order

@@ -6,6 +6,7 @@ namespace mtgl {
 int launch_tile(const TileArgs &a, cudaStream_t s)
 {
     if (a.ntiles == 0) return 0;
+    if (a.order_free) return launch_tile_free(a, s);
     return a.defer ? dispatch_tile_deferred(a, s, false) : dispatch_tile_size<false>(a, s, false);
 }
 

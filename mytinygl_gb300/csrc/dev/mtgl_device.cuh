@@ -119,6 +119,25 @@ __device__ __forceinline__ float depth_plane_bound(const float4 &zp, int minx, i
     return (z + 1.0f) * 0.5f;
 }
 
+// Upper bound of the same fragment depths, from the same plane: its maximum over the
+// rectangle plus the margin, which bounds the errors on either side. +inf without a plane.
+__device__ __forceinline__ float depth_plane_upper(const float4 &zp, int minx, int miny, int xl, int xh, int yl,
+                                                   int yh)
+{
+    const float dx = (float)((zp.y >= 0.0f ? xh : xl) - minx);
+    const float dy = (float)((zp.z >= 0.0f ? yh : yl) - miny);
+    const float z = (zp.x + zp.y * dx) + zp.z * dy + zp.w;
+    return (z + 1.0f) * 0.5f;
+}
+
+// Float order as unsigned order, reversed: a nearer depth has the larger key, and 0 is beyond
+// every depth (the tile occlusion bounds of binning start at zero bytes and take a maximum).
+__device__ __forceinline__ uint32_t near_key(float f)
+{
+    const uint32_t b = __float_as_uint(f);
+    return ~(b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u));
+}
+
 // Post-transform vertices (vertex_t, graphics.h:438-446, without the unused object normal)
 // are stored as three streams of 16-byte words, one word per vertex slot each: the clip
 // position, the colour, and (u, v, eye z, 0). The count pass of set-up reads only the first.
@@ -239,7 +258,7 @@ struct DevFrame {
     FrameDims dims;
     uint32_t tile_base;
     uint32_t clear_base, nclears;
-    uint32_t pad_;
+    uint32_t occlude;  // binning may drop pairs hidden behind a triangle covering their tile (k_bin.cu)
 };
 
 // ------------------------------------------------------------------ scalar helpers

@@ -379,3 +379,54 @@ def test_depth_plane_bound_is_below_every_covered_fragment():
                 if kind == 0 and dmin - lo < 1e-4:
                     tight += 1
     assert blocks > 20000 and tight > 1000
+
+
+def _depth_plane_upper_f32(zp, minx, miny, xl, xh, yl, yh):
+    """depth_plane_upper (mtgl_device.cuh) in float32."""
+    f = np.float32
+    p0, gx, gy, m = zp
+    dx = f((xh if gx >= 0 else xl) - minx)
+    dy = f((yh if gy >= 0 else yl) - miny)
+    zz = (p0 + gx * dx) + gy * dy + m
+    return (zz + f(1)) * f(0.5)
+
+
+def test_depth_plane_upper_is_above_every_covered_fragment():
+    """The occlusion bound of binning: over random 16x16 tiles of random integer triangles, the
+    plane's upper bound is at least the depth of every covered pixel in the tile, and near it."""
+    f = np.float32
+    rng = np.random.default_rng(12)
+    tiles = tight = 0
+    for k in range(600):
+        scale = [12, 60, 200, 400][k % 4]
+        xs = [150 + int(v) for v in rng.integers(-scale, scale + 1, 3)]
+        ys = [150 + int(v) for v in rng.integers(-scale, scale + 1, 3)]
+        z = [rng.uniform(-1, 1, 3), 0.3 + rng.uniform(-1e-6, 1e-6, 3), rng.uniform(-1, 1, 3) * 1e4,
+             rng.uniform(0.9, 1.0, 3)][(k // 4) % 4]
+        z = [f(v) for v in z]
+        X0, Y0, X1, Y1, X2, Y2 = (f(v) for v in (xs[0], ys[0], xs[1], ys[1], xs[2], ys[2]))
+        area = (X2 - X0) * (Y1 - Y0) - (Y2 - Y0) * (X1 - X0)
+        if abs(area) < 0.5:
+            continue
+        inv_area = f(1) / area
+        minx, maxx = max(min(xs), 0), min(max(xs), 511)
+        miny, maxy = max(min(ys), 0), min(max(ys), 511)
+        zp = _depth_plane_f32(z, xs, ys, area, inv_area, minx, miny, maxx, maxy)
+        gx, gy = np.meshgrid(np.arange(minx, maxx + 1, dtype=f), np.arange(miny, maxy + 1, dtype=f))
+        e = [(gx - ax) * A - (gy - ay) * B for ax, ay, A, B in _edges(xs[0], ys[0], xs[1], ys[1], xs[2], ys[2])]
+        cov = (e[0] >= 0) & (e[1] >= 0) & (e[2] >= 0) if area > 0 else (e[0] <= 0) & (e[1] <= 0) & (e[2] <= 0)
+        b = [ei * inv_area for ei in e]
+        depth = ((b[0] * z[0] + b[1] * z[1] + b[2] * z[2]) + f(1)) * f(0.5)
+        for by in range(miny - miny % 16, maxy + 1, 16):
+            for bx in range(minx - minx % 16, maxx + 1, 16):
+                xl, xh, yl, yh = max(bx, minx), min(bx + 15, maxx), max(by, miny), min(by + 15, maxy)
+                sub = cov[yl - miny:yh - miny + 1, xl - minx:xh - minx + 1]
+                if not sub.any():
+                    continue
+                up = _depth_plane_upper_f32(zp, minx, miny, xl, xh, yl, yh)
+                dmax = depth[yl - miny:yh - miny + 1, xl - minx:xh - minx + 1][sub].max()
+                assert up >= dmax, (k, bx, by, float(up), float(dmax))
+                tiles += 1
+                if sub.all() and up - dmax < 1e-4:
+                    tight += 1
+    assert tiles > 10000 and tight > 1000
