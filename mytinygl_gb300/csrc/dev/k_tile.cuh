@@ -113,8 +113,7 @@ __device__ __forceinline__ bool frag_color(const DevRaster &R, uint32_t ctl, con
         c = c2;
     } else {
         const float4 c0 = __ldg(r4 + 5), c1 = __ldg(r4 + 6);  // C0, C1
-        c = make_float4(c0.x * b0 + c1.x * b1 + c2.x * b2, c0.y * b0 + c1.y * b1 + c2.y * b2,
-                        c0.z * b0 + c1.z * b1 + c2.z * b2, c0.w * b0 + c1.w * b1 + c2.w * b2);
+        c = add4(add4(scale4(c0, b0), scale4(c1, b1)), scale4(c2, b2));
     }
     if (EYE && have_eye) {
         const mtgl_raster_state &rs = R.rs;
@@ -151,7 +150,7 @@ __device__ __forceinline__ bool frag_color(const DevRaster &R, uint32_t ctl, con
             u = b0 * q8.x + b1 * q8.z + b2 * q9.x;
             v = b0 * q8.y + b1 * q8.w + b2 * q9.y;
         }
-        const float4 tc = unpack_rgba(sample_lod(S, u, v, q4.w));
+        const float4 tc = sample_lod(S, u, v, q4.w);
         // the alpha test applies to textured fragments only (raster.c:639-643)
         if ((ctl & FC_ALPHA) && !cmp_pass(__ldg(&S.alpha_func), tc.w, __ldg(&S.alpha_ref))) return false;
         switch (__ldg(&S.tex_env_mode)) {
@@ -164,7 +163,7 @@ __device__ __forceinline__ bool frag_color(const DevRaster &R, uint32_t ctl, con
             break;
         }
         case GL_ADD: c = make_float4(c.x + tc.x, c.y + tc.y, c.z + tc.z, c.w * tc.w); break;
-        default: c = make_float4(c.x * tc.x, c.y * tc.y, c.z * tc.z, c.w * tc.w); break;
+        default: c = mul4(c, tc); break;
         }
     }
     if (ctl & FC_FOG) {
@@ -205,7 +204,6 @@ __device__ __forceinline__ uint32_t pending_color(const TileArgs &A, uint32_t ri
     const DevRaster &R = A.rasters[min(__float_as_uint(q11.w), A.nrasters - 1)];
     float4 c;
     frag_color<TEX, EYE>(R, __ldg(&R.fs.ctl), r4, e, have_eye, b0, b1, b2, c);
-    c = clamp4(c);
     return pack_rgba(c.x, c.y, c.z, c.w);
 }
 
@@ -302,7 +300,6 @@ __device__ __forceinline__ bool shade_pixel(const TileArgs &A, uint32_t ridx, co
         wrote = true;
     }
     if (ctl & FC_BLEND) c = blend(__ldg(&S.blend_src), __ldg(&S.blend_dst), c, unpack_rgba(col));
-    c = clamp4(c);
     if (ctl & FC_MASK_ALL) col = pack_rgba(c.x, c.y, c.z, c.w);
     else if (!(ctl & FC_MASK_NONE)) col = masked_write(__ldg(&S.color_mask), col, c);
     return wrote;
@@ -380,7 +377,7 @@ static __device__ __noinline__ PixelOut shade_prim(const TileArgs &A, const floa
     if (R.tex) {
         const float u = r[R_UV0] + t * (r[R_UV1] - r[R_UV0]);
         const float v = r[R_UV0 + 1] + t * (r[R_UV1 + 1] - r[R_UV0 + 1]);
-        const float4 tc = unpack_rgba(sample_lod(R.fs, u, v, 0.0f));
+        const float4 tc = sample_lod(R.fs, u, v, 0.0f);
         // the reference never leaves its loop when this test fails (raster.c:175, 183 skip the
         // Bresenham step); here the pixel is dropped
         if (rs.alpha_test && !cmp_pass(rs.alpha_func, tc.w, rs.alpha_ref)) return none;

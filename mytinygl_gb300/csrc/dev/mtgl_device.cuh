@@ -285,37 +285,92 @@ __device__ __forceinline__ int32_t small_floor(float f, float *fl)
     return __float_as_int(s) - 0x4B400000;
 }
 
-// (float)v / 255.0f (graphics.h:350-357, textures.c:294-307) for v in [0, 255], without a
-// division: the product with the rounded reciprocal, corrected once by its exact residual
-// (Markstein's FMA correction). The result equals the IEEE quotient for every byte value
-// (checked exhaustively with exact rational arithmetic in tests/test_arith.py).
-__device__ __forceinline__ float u8f(uint32_t v)
+// Two IEEE single operations in one instruction (the packed f32x2 forms): each half rounds as
+// the scalar operation does. The colour stages work on four channels at a time and are bound
+// by issue slots, so they use these throughout.
+#define MTGL_OP2(name, ptx)                                                                               \
+    __device__ __forceinline__ float2 name(float2 a, float2 b)                                            \
+    {                                                                                                     \
+        float2 r;                                                                                         \
+        asm("{\n .reg .b64 a, b, r;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n " ptx             \
+            " r, a, b;\n mov.b64 {%0, %1}, r;\n}"                                                       \
+            : "=f"(r.x), "=f"(r.y)                                                                        \
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));                                                    \
+        return r;                                                                                         \
+    }
+MTGL_OP2(add2_rz, "add.rz.f32x2")
+MTGL_OP2(mul2, "mul.rn.f32x2")
+#undef MTGL_OP2
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c)
 {
-    const float x = small_u2f(v);
-    const float r = 0x1.010102p-8f;  // 1.0f / 255.0f rounded to float
-    const float q = x * r;
-    const float e = __fmaf_rn(-q, 255.0f, x);
-    return __fmaf_rn(e, r, q);
+    float2 r;
+    asm("{\n .reg .b64 a, b, c, r;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n mov.b64 c, {%6, %7};\n "
+        "fma.rn.f32x2 r, a, b, c;\n mov.b64 {%0, %1}, r;\n}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return r;
+}
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+// Sums as fma with a factor of one or minus one, which rounds once, as the sum does. The factor
+// is read from constant memory, where the assembler cannot know its value: it contracts a
+// packed mul.rn followed by add.rn, or by an fma with a literal one, into a single fma (a
+// rounding less) whatever -fmad says (tests/test_gpu_colour.py sees the difference).
+static __constant__ float2 k_plus_one = {1.0f, 1.0f};
+static __constant__ float2 k_minus_one = {-1.0f, -1.0f};
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return fma2(a, k_plus_one, b); }
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return fma2(b, k_minus_one, a); }
+__device__ __forceinline__ float2 lo2(float4 v) { return make_float2(v.x, v.y); }
+__device__ __forceinline__ float2 hi2(float4 v) { return make_float2(v.z, v.w); }
+__device__ __forceinline__ float4 join(float2 a, float2 b) { return make_float4(a.x, a.y, b.x, b.y); }
+__device__ __forceinline__ float4 mul4(float4 a, float4 b) { return join(mul2(lo2(a), lo2(b)), mul2(hi2(a), hi2(b))); }
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return join(add2(lo2(a), lo2(b)), add2(hi2(a), hi2(b))); }
+__device__ __forceinline__ float4 scale4(float4 a, float t)
+{
+    return join(mul2(lo2(a), both(t)), mul2(hi2(a), both(t)));
 }
 
-// one channel of color_to_rgba32: the reference clamps with two compares, which pass a
-// NaN through to a conversion giving INT32_MIN, whose low byte is 0; fmaxf / fminf map a NaN
-// to 0 first, and every other input to the same clamped value (a -0 may come out as +0,
-// which truncates to the same byte)
-__device__ __forceinline__ uint32_t pack_channel(float c)
+// x / 255.0f (graphics.h:350-357, textures.c:294-307) for x an integer in [0, 255], without a
+// division: 1/255 as the sum of two floats, fma(x, hi, x * lo). The result equals the IEEE
+// quotient for every byte value (checked exhaustively with exact rational arithmetic in
+// tests/test_arith.py).
+constexpr float kInv255Hi = 0x1.010102p-8f, kInv255Lo = -0x1.fdfdfep-33f;
+__device__ __forceinline__ float over_255(float x) { return __fmaf_rn(x, kInv255Hi, x * kInv255Lo); }
+__device__ __forceinline__ float2 over_255(float2 x) { return fma2(x, both(kInv255Hi), mul2(x, both(kInv255Lo))); }
+__device__ __forceinline__ float u8f(uint32_t v) { return over_255(small_u2f(v)); }
+
+// The byte v that color_to_rgba32 stores per channel (graphics.h:337-348), as the float
+// 2^23 + v, whose low byte is v: clamp, times 255, truncate. The reference clamps with two
+// compares, which pass a NaN through to a conversion giving INT32_MIN, whose low byte is 0;
+// saturation maps a NaN to 0 first, and every other input to the same clamped value (a -0 may
+// come out as +0, which truncates to the same byte).
+__device__ __forceinline__ float2 byte_bits(float a, float b)
 {
-    return (uint32_t)small_trunc(fminf(fmaxf(c, 0.0f), 1.0f) * 255.0f) & 0xFFu;
+    return add2_rz(mul2(make_float2(__saturatef(a), __saturatef(b)), both(255.0f)), both(0x1p23f));
 }
 
 // color_to_rgba32 (graphics.h:337-348)
 __device__ __forceinline__ uint32_t pack_rgba(float r, float g, float b, float a)
 {
-    return (pack_channel(a) << 24) | (pack_channel(b) << 16) | (pack_channel(g) << 8) | pack_channel(r);
+    const float2 rg = byte_bits(r, g), ba = byte_bits(b, a);
+    const uint32_t lo = __byte_perm(__float_as_uint(rg.x), __float_as_uint(rg.y), 0x0040);
+    const uint32_t hi = __byte_perm(__float_as_uint(ba.x), __float_as_uint(ba.y), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
 }
 
 __device__ __forceinline__ float4 unpack_rgba(uint32_t p)
 {
-    return make_float4(u8f(p & 0xFFu), u8f((p >> 8) & 0xFFu), u8f((p >> 16) & 0xFFu), u8f((p >> 24) & 0xFFu));
+    // a byte under the exponent of 2^23: 2^23 + v
+    const float2 rg = make_float2(__uint_as_float(__byte_perm(p, 0x4B000000u, 0x7440)),
+                                  __uint_as_float(__byte_perm(p, 0x4B000000u, 0x7441)));
+    const float2 ba = make_float2(__uint_as_float(__byte_perm(p, 0x4B000000u, 0x7442)),
+                                  __uint_as_float(__byte_perm(p, 0x4B000000u, 0x7443)));
+    return join(over_255(sub2(rg, both(0x1p23f))), over_255(sub2(ba, both(0x1p23f))));
+}
+
+// unpack_rgba(pack_rgba(c)): a colour through its stored bytes
+__device__ __forceinline__ float4 quantize(float4 c)
+{
+    return join(over_255(sub2(byte_bits(c.x, c.y), both(0x1p23f))), over_255(sub2(byte_bits(c.z, c.w), both(0x1p23f))));
 }
 
 __device__ __forceinline__ float clamp01(float v) { return v < 0.0f ? 0.0f : (v > 1.0f ? 1.0f : v); }
@@ -327,14 +382,14 @@ __device__ __forceinline__ float4 clamp4(float4 c)
 // color_lerp (graphics.h:293-296): a*(1-t) + b*t
 __device__ __forceinline__ float4 lerp_col(float4 a, float4 b, float t)
 {
-    float s = 1.0f - t;
-    return make_float4(a.x * s + b.x * t, a.y * s + b.y * t, a.z * s + b.z * t, a.w * s + b.w * t);
+    return add4(scale4(a, 1.0f - t), scale4(b, t));
 }
 
 // color_lerp_rgb (graphics.h:298-305): a + (b-a)*t, keeps a's alpha
 __device__ __forceinline__ float4 lerp_rgb(float4 a, float4 b, float t)
 {
-    return make_float4(a.x + (b.x - a.x) * t, a.y + (b.y - a.y) * t, a.z + (b.z - a.z) * t, a.w);
+    const float2 xy = add2(lo2(a), mul2(sub2(lo2(b), lo2(a)), both(t)));
+    return make_float4(xy.x, xy.y, a.z + (b.z - a.z) * t, a.w);
 }
 
 __device__ __forceinline__ float3 normalize3(float x, float y, float z)
@@ -464,7 +519,8 @@ __device__ __forceinline__ uint32_t texel_at(const TexView &t, int32_t x, int32_
     return __ldg(t.px + (size_t)y * t.w + x);
 }
 
-__device__ __forceinline__ uint32_t sample_level(const TexView &t, int32_t ws, int32_t wt, float u, float v, bool linear)
+// texture_sample_nearest / _linear on one level, as the colour of the stored bytes
+__device__ __forceinline__ float4 sample_level(const TexView &t, int32_t ws, int32_t wt, float u, float v, bool linear)
 {
     float tx = u * (float)t.w - 0.5f;
     float ty = v * (float)t.h - 0.5f;
@@ -486,14 +542,11 @@ __device__ __forceinline__ uint32_t sample_level(const TexView &t, int32_t ws, i
         const bool rs = ws == GL_REPEAT, rt = wt == GL_REPEAT;
         const int32_t xa = wrap_coord(x0, t.w, rs), xb = wrap_next(xa, x0, t.w, rs);
         const int32_t ya = wrap_coord(y0, t.h, rt), yb = wrap_next(ya, y0, t.h, rt);
-        float4 c00 = unpack_rgba(texel_at(t, xa, ya));
-        float4 c10 = unpack_rgba(texel_at(t, xb, ya));
-        float4 c01 = unpack_rgba(texel_at(t, xa, yb));
-        float4 c11 = unpack_rgba(texel_at(t, xb, yb));
-        float4 top = lerp_col(c00, c10, fx);
-        float4 bot = lerp_col(c01, c11, fx);
-        float4 r = lerp_col(top, bot, fy);
-        return pack_rgba(r.x, r.y, r.z, r.w);
+        const uint32_t *ra = t.px + (size_t)ya * t.w, *rb = t.px + (size_t)yb * t.w;
+        const uint32_t p00 = __ldg(ra + xa), p10 = __ldg(ra + xb), p01 = __ldg(rb + xa), p11 = __ldg(rb + xb);
+        const float4 top = lerp_col(unpack_rgba(p00), unpack_rgba(p10), fx);
+        const float4 bot = lerp_col(unpack_rgba(p01), unpack_rgba(p11), fx);
+        return quantize(lerp_col(top, bot, fy));
     }
     const float hx = tx + 0.5f, hy = ty + 0.5f;
     int32_t x, y;
@@ -509,23 +562,13 @@ __device__ __forceinline__ uint32_t sample_level(const TexView &t, int32_t ws, i
     if (x >= t.w) x = t.w - 1;
     if (y < 0) y = 0;
     if (y >= t.h) y = t.h - 1;
-    return __ldg(t.px + (size_t)y * t.w + x);
+    return unpack_rgba(__ldg(t.px + (size_t)y * t.w + x));
 }
 
 // a pointer field through the read-only path
 __device__ __forceinline__ const uint32_t *ldg_ptr(const uint32_t *const *p)
 {
     return reinterpret_cast<const uint32_t *>(__ldg(reinterpret_cast<const unsigned long long *>(p)));
-}
-
-__device__ __forceinline__ uint32_t sample_mip1(const FragState &S, int32_t ws, int32_t wt, float u, float v,
-                                                int32_t filter)
-{
-    const uint32_t *mip1 = ldg_ptr(&S.mip1);
-    if (!mip1) return 0xFFFFFFFFu;  // level 1 cannot be built (textures.c:317, 416-419)
-    TexView m{mip1, __ldg(&S.mip_w), __ldg(&S.mip_h)};
-    bool lin = filter == GL_LINEAR || filter == GL_LINEAR_MIPMAP_NEAREST || filter == GL_LINEAR_MIPMAP_LINEAR;
-    return sample_level(m, ws, wt, u, v, lin);
 }
 
 // (float)x86_f2i(f): the truncated value as a float (INT32_MIN outside the int range)
@@ -537,8 +580,8 @@ __device__ __forceinline__ float trunc_f2i_f(float f)
     return f < 0.0f ? -t : t;  // a -0 here only meets u - t, where it acts as +0
 }
 
-// Level d of a texture with a chain (0: base, 1: mip1, 2..: the chain).
-__device__ __forceinline__ TexView chain_level(const FragState &S, int d)
+// Level d of a texture (0: base, 1: mip1, null when it cannot be built; 2..: the chain).
+__device__ __forceinline__ TexView tex_level(const FragState &S, int d)
 {
     if (d == 0) return TexView{ldg_ptr(&S.tex), __ldg(&S.tex_w), __ldg(&S.tex_h)};
     if (d == 1) return TexView{ldg_ptr(&S.mip1), __ldg(&S.mip_w), __ldg(&S.mip_h)};
@@ -546,30 +589,19 @@ __device__ __forceinline__ TexView chain_level(const FragState &S, int d)
     return TexView{ldg_ptr(&m[d - 2].px), __ldg(&m[d - 2].w), __ldg(&m[d - 2].h)};
 }
 
-// The mipmap filters over a whole chain (MTGL_OPT_MIPMAP_CHAIN; no counterpart in the
-// reference): levels 0 .. top, lod > 0. *_MIPMAP_NEAREST takes level floor(lod + 0.5);
-// *_MIPMAP_LINEAR blends levels floor(lod) and floor(lod) + 1 by the fraction, as the
-// reference blends levels 0 and 1 (lerp of the unpacked texels, repacked); from the top
-// level up, that level alone.
-static __device__ __noinline__ uint32_t sample_chain(const FragState &S, int32_t ws, int32_t wt, float u, float v, float lod,
-                                              int32_t filter, int top)
-{
-    const bool lin = filter == GL_LINEAR_MIPMAP_NEAREST || filter == GL_LINEAR_MIPMAP_LINEAR;
-    if (filter == GL_NEAREST_MIPMAP_NEAREST || filter == GL_LINEAR_MIPMAP_NEAREST) {
-        const int d = lod >= (float)top ? top : (int)(lod + 0.5f);
-        return sample_level(chain_level(S, min(d, top)), ws, wt, u, v, lin);
-    }
-    if (lod >= (float)top) return sample_level(chain_level(S, top), ws, wt, u, v, lin);
-    const int d = (int)lod;
-    const float t = lod - (float)d;
-    const uint32_t c0 = sample_level(chain_level(S, d), ws, wt, u, v, lin);
-    const uint32_t c1 = sample_level(chain_level(S, d + 1), ws, wt, u, v, lin);
-    const float4 r = lerp_col(unpack_rgba(c0), unpack_rgba(c1), t);
-    return pack_rgba(r.x, r.y, r.z, r.w);
-}
-
-// texture_sample_lod (textures.c:457-557) on the packed texture state
-__device__ inline uint32_t sample_lod(const FragState &S, float u, float v, float lod)
+// texture_sample_lod (textures.c:457-557) on the packed texture state, as the colour of the
+// sampled bytes. The filter picks one level, or two and a weight:
+// - GL_NEAREST / GL_LINEAR (and any filter at lod <= 0): the base level;
+// - *_MIPMAP_NEAREST: level 1 from lod 0.5 up;
+// - *_MIPMAP_LINEAR: levels 0 and 1 blended by lod; from lod 1 up level 1 alone: lerp_col(c0,
+//   c1, 1) gives c1's channels exactly (c0 * 0 + c1 * 1), and their bytes are c1's again
+//   (truncating ((float)b / 255) * 255 returns b for every byte).
+// With a whole chain (MTGL_OPT_MIPMAP_CHAIN; no counterpart in the reference) and lod > 0:
+// level floor(lod + 0.5), or levels floor(lod) and floor(lod) + 1 blended by the fraction, and
+// from the top level up that level alone.
+// The levels go through one copy of the filter code, in a loop: the tile kernels spill out of
+// the instruction cache otherwise (no_instruction was the largest stall of a textured frame).
+__device__ inline float4 sample_lod(const FragState &S, float u, float v, float lod)
 {
     const int4 mode = __ldg(reinterpret_cast<const int4 *>(&S.wrap_s));  // wrap s, wrap t, min, mag filter
     const int32_t ws = mode.x, wt = mode.y;
@@ -587,31 +619,31 @@ __device__ inline uint32_t sample_lod(const FragState &S, float u, float v, floa
         if (v < 0.0f) v = 0.0f;
         if (v > 1.0f) v = 1.0f;
     }
-    int32_t filter = (lod > 0.0f) ? mode.z : mode.w;
+    const int32_t filter = (lod > 0.0f) ? mode.z : mode.w;
+    const bool linear = filter == GL_LINEAR || filter == GL_LINEAR_MIPMAP_NEAREST || filter == GL_LINEAR_MIPMAP_LINEAR;
+    int d = 0, last = 0;
+    float t = 0.0f;
     if (lod > 0.0f && filter != GL_NEAREST && filter != GL_LINEAR) {
-        const int chain = __ldg(&S.chain_levels);
-        if (chain > 0) return sample_chain(S, ws, wt, u, v, lod, filter, 1 + chain);
-    }
-    if (filter == GL_NEAREST_MIPMAP_NEAREST || filter == GL_LINEAR_MIPMAP_NEAREST) {
-        if (lod >= 0.5f) return sample_mip1(S, ws, wt, u, v, filter);
-        filter = (filter == GL_NEAREST_MIPMAP_NEAREST) ? GL_NEAREST : GL_LINEAR;
-    } else if (filter == GL_NEAREST_MIPMAP_LINEAR || filter == GL_LINEAR_MIPMAP_LINEAR) {
-        // From lod 1 up the weight of level 1 is 1: lerp_col(c0, c1, 1) gives c1's channels
-        // exactly (c0 * 0 + c1 * 1), and packing them gives c1 back (truncating
-        // ((float)b / 255) * 255 returns b for every byte), so level 0 is not sampled.
-        if (lod >= 1.0f) return sample_mip1(S, ws, wt, u, v, filter);
-        if (lod > 0.0f) {
-            float cl = (lod > 1.0f) ? 1.0f : lod;
-            const TexView base{ldg_ptr(&S.tex), __ldg(&S.tex_w), __ldg(&S.tex_h)};
-            uint32_t c0 = sample_level(base, ws, wt, u, v, filter == GL_LINEAR_MIPMAP_LINEAR);
-            uint32_t c1 = sample_mip1(S, ws, wt, u, v, filter);
-            float4 r = lerp_col(unpack_rgba(c0), unpack_rgba(c1), cl);
-            return pack_rgba(r.x, r.y, r.z, r.w);
+        const int top = 1 + __ldg(&S.chain_levels);
+        if (filter == GL_NEAREST_MIPMAP_NEAREST || filter == GL_LINEAR_MIPMAP_NEAREST) {
+            if (top == 1) d = lod >= 0.5f ? 1 : 0;
+            else d = lod >= (float)top ? top : min((int)(lod + 0.5f), top);
+            last = d;
+        } else {
+            d = lod >= (float)top ? top : (int)lod;
+            last = min(d + 1, top);
+            t = lod - (float)d;
         }
-        filter = (filter == GL_NEAREST_MIPMAP_LINEAR) ? GL_NEAREST : GL_LINEAR;
     }
-    const TexView base{ldg_ptr(&S.tex), __ldg(&S.tex_w), __ldg(&S.tex_h)};
-    return sample_level(base, ws, wt, u, v, filter == GL_LINEAR);
+    float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll 1
+    for (int k = d; k <= last; k++) {
+        const TexView view = tex_level(S, k);
+        // a level 1 that cannot be built samples as white (textures.c:317, 416-419)
+        const float4 s = view.px ? sample_level(view, ws, wt, u, v, linear) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        c = k == d ? s : quantize(lerp_col(c, s, t));
+    }
+    return c;
 }
 
 // ------------------------------------------------------------------ fragment helpers (raster.c:343-448, 672-705)
@@ -637,12 +669,13 @@ __device__ __forceinline__ float4 blend_factor(uint32_t f, float4 s, float4 d)
     }
 }
 
+// The result is clamped where it is stored (pack_rgba): the reference's clamp before that
+// changes nothing, and a masked write keeps the same channels.
 __device__ __forceinline__ float4 blend(uint32_t src, uint32_t dst, float4 s, float4 d)
 {
-    float4 sf = blend_factor(src, s, d);
-    float4 df = blend_factor(dst, s, d);
-    return clamp4(make_float4(s.x * sf.x + d.x * df.x, s.y * sf.y + d.y * df.y, s.z * sf.z + d.z * df.z,
-                              s.w * sf.w + d.w * df.w));
+    if (src == GL_SRC_ALPHA && dst == GL_ONE_MINUS_SRC_ALPHA)  // the common pair, without the two switches
+        return add4(scale4(s, s.w), scale4(d, 1 - s.w));
+    return add4(mul4(s, blend_factor(src, s, d)), mul4(d, blend_factor(dst, s, d)));
 }
 
 __device__ __forceinline__ float4 blend(const mtgl_raster_state &rs, float4 s, float4 d)

@@ -430,3 +430,39 @@ def test_depth_plane_upper_is_above_every_covered_fragment():
                 if sub.all() and up - dmax < 1e-4:
                     tight += 1
     assert tiles > 10000 and tight > 1000
+
+
+def test_byte_over_255_as_two_floats_is_exact_for_every_byte():
+    """over_255 (mtgl_device.cuh): fma(v, hi, v * lo) with hi + lo the two-float 1/255 is the
+    IEEE quotient v / 255 for every byte value."""
+    hi, lo = float.fromhex("0x1.010102p-8"), float.fromhex("-0x1.fdfdfep-33")
+    assert Fr(hi) == round_f32(Fr(1, 255)) and Fr(lo) == round_f32(Fr(1, 255) - Fr(hi))
+    for v in range(256):
+        t = round_f32(v * Fr(lo))
+        assert round_f32(v * Fr(hi) + t) == round_f32(Fr(v, 255)), v
+
+
+def _warp_transpose(v):
+    """warp_transpose (k_tile_free.cu) over 32 lanes."""
+    v, mask, s = list(v), 0x0000FFFF, 16
+    while s:
+        o = [v[lane ^ s] for lane in range(32)]
+        for lane in range(32):
+            keep, other = v[lane], o[lane]
+            if lane & s:
+                v[lane] = (keep & ~mask & 0xFFFFFFFF) | ((other & ~mask & 0xFFFFFFFF) >> s)
+            else:
+                v[lane] = (keep & mask) | ((other & mask) << s)
+        mask ^= (mask << (s >> 1)) & 0xFFFFFFFF
+        s >>= 1
+    return v
+
+
+def test_warp_transpose():
+    rng = np.random.default_rng(13)
+    for _ in range(50):
+        v = [int(x) for x in rng.integers(0, 1 << 32, 32)]
+        t = _warp_transpose(v)
+        for i in range(32):
+            for j in range(32):
+                assert t[i] >> j & 1 == v[j] >> i & 1
