@@ -179,6 +179,10 @@ int mtgl_dev_buffer_destroy(mtgl_dev *d, mtgl_handle h);
 int mtgl_dev_texture_create(mtgl_dev *d, mtgl_handle *out);
 /* rgba32: packed a<<24|b<<16|g<<8|r texels (graphics.h:420-434). Builds mip level 1. */
 int mtgl_dev_texture_image(mtgl_dev *d, mtgl_handle h, int32_t width, int32_t height, const uint32_t *rgba32);
+/* The same from client bytes, `comps` per texel: 1 luminance, 2 luminance and alpha, 3 RGB,
+ * 4 RGBA (texture_upload_*, textures.c:141-269). pixels is borrowed for the call only. */
+int mtgl_dev_texture_pixels(mtgl_dev *d, mtgl_handle h, int32_t width, int32_t height, int32_t comps,
+                            const uint8_t *pixels);
 int mtgl_dev_texture_destroy(mtgl_dev *d, mtgl_handle h);
 /* Replace level `level` (>= 1) of a texture whose chain was built under
  * MTGL_OPT_MIPMAP_CHAIN; the size must be the level's. No counterpart in the reference.

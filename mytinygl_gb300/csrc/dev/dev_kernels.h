@@ -173,6 +173,9 @@ int tile_occupancy(const TileArgs &a);
 // glClear without draws (gl_api.c:409-457)
 void launch_clear(const ClearOp *ops_host, int nops, FrameDims dims, uint32_t *color, float *depth, uint8_t *stencil,
                   cudaStream_t s);
+// packed RGBA8 texels from 1 (luminance), 2 (luminance, alpha) or 3 (RGB) bytes per texel
+// (texture_upload_*, textures.c:141-269)
+void launch_expand_texels(const uint8_t *raw, int comps, int64_t n, uint32_t *texels, cudaStream_t s);
 // mip level 1 (textures.c:311-354)
 void launch_mip1(const uint32_t *base, int32_t w, int32_t h, uint32_t *mip, cudaStream_t s);
 // glDrawPixels blit (gl_api.c:1287-1376)

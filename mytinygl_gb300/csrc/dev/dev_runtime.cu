@@ -416,39 +416,76 @@ int mtgl_dev_texture_create(mtgl_dev *d, mtgl_handle *out)
     return MTGL_OK;
 }
 
-int mtgl_dev_texture_image(mtgl_dev *d, mtgl_handle h, int32_t w, int32_t hgt, const uint32_t *rgba32)
+// Stores an image of w x hgt texels: `comps` client bytes per texel (4: packed texels as they
+// are), expanded on the device where they are fewer. Storage of the same size is kept.
+static int texture_store(mtgl_dev *d, DevTextureObj *t, int32_t w, int32_t hgt, int32_t comps, const void *pixels)
 {
-    DevTextureObj *t = reinterpret_cast<DevTextureObj *>(h);
-    if (!d || !t || w <= 0 || hgt <= 0 || !rgba32) return MTGL_ERR_INVALID;
     CK(cudaSetDevice(d->device));
     int st = flush_if_drawing(d);
     if (st || (st = mtgl_dev_enter(d))) return st;
     cudaStream_t s = d->x.stream;
-    if (t->base) CK(cudaFreeAsync(t->base, s));
-    if (t->mip1) CK(cudaFreeAsync(t->mip1, s));
     if (t->chain) CK(cudaFreeAsync(t->chain, s));
     if (t->chain_tab) CK(cudaFreeAsync(t->chain_tab, s));
-    t->base = nullptr;
-    t->mip1 = nullptr;
     t->chain = nullptr;
     t->chain_tab = nullptr;
     t->levels.clear();
     const size_t n = (size_t)w * (size_t)hgt;
-    CK(cudaMallocAsync((void **)&t->base, n * 4, s));
-    CK(cudaMemcpyAsync(t->base, rgba32, n * 4, cudaMemcpyHostToDevice, s));
-    t->w = w;
-    t->h = hgt;
-    t->mw = t->mh = 0;
-    if (w >= 2 && hgt >= 2) {
-        t->mw = w / 2;
-        t->mh = hgt / 2;
-        CK(cudaMallocAsync((void **)&t->mip1, (size_t)t->mw * t->mh * 4, s));
+    if (t->base && (t->w != w || t->h != hgt)) {
+        uint32_t *base = t->base, *mip1 = t->mip1;
+        t->base = t->mip1 = nullptr;
+        CK(cudaFreeAsync(base, s));
+        if (mip1) CK(cudaFreeAsync(mip1, s));
+    }
+    if (!t->base) {
+        t->mw = t->mh = 0;
+        CK(cudaMallocAsync((void **)&t->base, n * 4, s));
+        t->w = w;
+        t->h = hgt;
+        if (w >= 2 && hgt >= 2) {
+            const cudaError_t e = cudaMallocAsync((void **)&t->mip1, (size_t)(w / 2) * (hgt / 2) * 4, s);
+            if (e != cudaSuccess) {  // an image has both levels or neither
+                t->mip1 = nullptr;
+                cudaFreeAsync(t->base, s);
+                t->base = nullptr;
+                return fail_cuda("cudaMallocAsync", e);
+            }
+            t->mw = w / 2;
+            t->mh = hgt / 2;
+        }
+    }
+    if (comps == 4) {
+        CK(cudaMemcpyAsync(t->base, pixels, n * 4, cudaMemcpyHostToDevice, s));
+    } else {
+        uint8_t *raw = nullptr;
+        CK(cudaMallocAsync((void **)&raw, n * (size_t)comps, s));
+        const cudaError_t e = cudaMemcpyAsync(raw, pixels, n * (size_t)comps, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) launch_expand_texels(raw, comps, (int64_t)n, t->base, s);
+        CK(cudaFreeAsync(raw, s));
+        if (e != cudaSuccess) return fail_cuda("cudaMemcpyAsync", e);
+        d->stats.kernel_launches++;
+    }
+    if (t->mip1) {
         launch_mip1(t->base, w, hgt, t->mip1, s);
         CK(cudaGetLastError());
         d->stats.kernel_launches++;
     }
+    CK(cudaStreamSynchronize(s));  // the copy has read the caller's memory
     if (d->mipmap_chain && t->mip1) return build_chain(d, t);
     return MTGL_OK;
+}
+
+int mtgl_dev_texture_image(mtgl_dev *d, mtgl_handle h, int32_t w, int32_t hgt, const uint32_t *rgba32)
+{
+    DevTextureObj *t = reinterpret_cast<DevTextureObj *>(h);
+    if (!d || !t || w <= 0 || hgt <= 0 || !rgba32) return MTGL_ERR_INVALID;
+    return texture_store(d, t, w, hgt, 4, rgba32);
+}
+
+int mtgl_dev_texture_pixels(mtgl_dev *d, mtgl_handle h, int32_t w, int32_t hgt, int32_t comps, const uint8_t *pixels)
+{
+    DevTextureObj *t = reinterpret_cast<DevTextureObj *>(h);
+    if (!d || !t || w <= 0 || hgt <= 0 || comps < 1 || comps > 4 || !pixels) return MTGL_ERR_INVALID;
+    return texture_store(d, t, w, hgt, comps, pixels);
 }
 
 int mtgl_dev_texture_level(mtgl_dev *d, mtgl_handle h, int32_t level, int32_t w, int32_t hgt, const uint32_t *rgba32)
@@ -613,6 +650,7 @@ int mtgl_dev_draw_pixels(mtgl_dev *d, int32_t rx, int32_t ry, int32_t w, int32_t
     CK(cudaMallocAsync((void **)&dr, sizeof(DevRaster), s));
     CK(cudaMemcpyAsync(img, rgba32, n * 4, cudaMemcpyHostToDevice, s));
     CK(cudaMemcpyAsync(dr, &R, sizeof(R), cudaMemcpyHostToDevice, s));
+    CK(cudaStreamSynchronize(s));  // the copies have read the caller's memory and this frame's
     FrameDims dims;
     dims.width = d->width;
     dims.height = d->height;

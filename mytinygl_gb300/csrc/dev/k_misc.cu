@@ -41,6 +41,21 @@ void launch_clear(const ClearOp *ops, int nops, FrameDims dims, uint32_t *color,
     }
 }
 
+__global__ void __launch_bounds__(256) k_expand_texels(const uint8_t *raw, int comps, int64_t n, uint32_t *texels)
+{
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const uint8_t *p = raw + i * comps;
+        const uint32_t r = p[0], g = comps == 3 ? p[1] : r, b = comps == 3 ? p[2] : r, a = comps == 2 ? p[1] : 255u;
+        texels[i] = (a << 24) | (b << 16) | (g << 8) | r;
+    }
+}
+
+void launch_expand_texels(const uint8_t *raw, int comps, int64_t n, uint32_t *texels, cudaStream_t s)
+{
+    if (n <= 0) return;
+    k_expand_texels<<<(unsigned)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, s>>>(raw, comps, n, texels);
+}
+
 // texture_generate_mip1 (textures.c:311-354): 2x2 box filter in float, truncated to RGBA8.
 // Built when the image is uploaded; the reference builds it on first use, with the same result.
 __global__ void __launch_bounds__(256) k_mip1(const uint32_t *base, int32_t w, int32_t h, uint32_t *mip)

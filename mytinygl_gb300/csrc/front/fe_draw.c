@@ -686,6 +686,12 @@ void glDrawPixels(GLsizei width, GLsizei height, GLenum format, GLenum type, con
     if (type != GL_UNSIGNED_BYTE || !pixels || !c->raster_valid) return;
     if (format != GL_RGBA && format != GL_RGB && format != GL_LUMINANCE && format != GL_LUMINANCE_ALPHA) return;
     if (width <= 0 || height <= 0) return;
+    mtgl_raster_state rs;
+    fe_snapshot_raster(c, &rs);
+    if (format == GL_RGBA && ((uintptr_t)pixels & 3u) == 0) { /* packed texels are the client's bytes as they are */
+        fe_dev_error(c, mtgl_dev_draw_pixels(c->dev, c->raster_x, c->raster_y, width, height, (const uint32_t *)pixels, &rs));
+        return;
+    }
     size_t n = (size_t)width * (size_t)height;
     uint32_t *packed = (uint32_t *)malloc(n * sizeof(uint32_t));
     if (!packed) {
@@ -701,8 +707,6 @@ void glDrawPixels(GLsizei width, GLsizei height, GLenum format, GLenum type, con
         else { r = g = b = s[2 * i]; a = s[2 * i + 1]; }
         packed[i] = (a << 24) | (b << 16) | (g << 8) | r;
     }
-    mtgl_raster_state rs;
-    fe_snapshot_raster(c, &rs);
     fe_dev_error(c, mtgl_dev_draw_pixels(c->dev, c->raster_x, c->raster_y, width, height, packed, &rs));
     free(packed);
 }

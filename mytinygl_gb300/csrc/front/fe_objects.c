@@ -145,6 +145,20 @@ void glTexImage2D(GLenum target, GLint level, GLint internalformat, GLsizei widt
     }
     /* upload failures (empty or oversized image) leave the texture unchanged */
     if (width <= 0 || height <= 0 || width > FE_MAX_TEXTURE_SIZE || height > FE_MAX_TEXTURE_SIZE) return;
+    int st = MTGL_OK;
+    if (level == 0 && pixels) { /* the back end takes the client's bytes */
+        if (!t->dev) st = mtgl_dev_texture_create(c->dev, &t->dev);
+        if (st == MTGL_OK)
+            st = mtgl_dev_texture_pixels(c->dev, t->dev, width, height, comps, (const uint8_t *)pixels);
+        if (st != MTGL_OK) {
+            fe_dev_error(c, st);
+            return;
+        }
+        t->width = width;
+        t->height = height;
+        t->has_image = 1;
+        return;
+    }
     size_t n = (size_t)width * (size_t)height;
     uint32_t *texels = (uint32_t *)malloc(n * sizeof(uint32_t));
     if (!texels) return;
@@ -159,7 +173,6 @@ void glTexImage2D(GLenum target, GLint level, GLint internalformat, GLsizei widt
         }
         texels[i] = (a << 24) | (b << 16) | (g << 8) | r;
     }
-    int st = MTGL_OK;
     if (level > 0) {
         if (!t->has_image || !t->dev) {
             free(texels);

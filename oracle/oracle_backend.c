@@ -309,6 +309,24 @@ int mtgl_dev_texture_image(mtgl_dev *d, mtgl_handle h, int32_t width, int32_t he
     return MTGL_OK;
 }
 
+int mtgl_dev_texture_pixels(mtgl_dev *d, mtgl_handle h, int32_t width, int32_t height, int32_t comps,
+                            const uint8_t *pixels)
+{
+    if (!pixels || width <= 0 || height <= 0 || comps < 1 || comps > 4) return MTGL_ERR_INVALID;
+    const size_t n = (size_t)width * (size_t)height;
+    uint32_t *texels = (uint32_t *)malloc(n * sizeof(uint32_t));
+    if (!texels) return MTGL_ERR_OOM;
+    for (size_t i = 0; i < n; i++) {
+        const uint8_t *s = pixels + i * (size_t)comps;
+        const uint32_t r = s[0], g = comps >= 3 ? s[1] : s[0], b = comps >= 3 ? s[2] : s[0];
+        const uint32_t a = comps == 4 ? s[3] : (comps == 2 ? s[1] : 255u);
+        texels[i] = (a << 24) | (b << 16) | (g << 8) | r;
+    }
+    const int st = mtgl_dev_texture_image(d, h, width, height, texels);
+    free(texels);
+    return st;
+}
+
 int mtgl_dev_texture_level(mtgl_dev *d, mtgl_handle h, int32_t level, int32_t width, int32_t height,
                            const uint32_t *rgba32)
 {
