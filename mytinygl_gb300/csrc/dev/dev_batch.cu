@@ -438,7 +438,9 @@ int mtgl_dev_batch_launch(mtgl_batch *b)
     b->run.exact = false;
     b->run.rec_cap = rec_cap;
     b->run.pair_cap = pair_cap;
-    b->run.ctas = persistent_ctas(b->x, b->t, b->cfg.ctas_per_sm);
+    bool limited = false;
+    const int resident = resident_ctas(b->x, b->t, b->cfg.ctas_per_sm, &limited);
+    b->run.ctas = limited ? resident : 0;
     b->run.order = b->cfg.order_by_cost != 0;
     if ((st = launch_run(b))) return st;
     if ((st = b->stage.mark_uploaded(b->x.stream))) return st;
@@ -453,7 +455,7 @@ int mtgl_dev_batch_launch(mtgl_batch *b)
         b->stats.vertices += p.slots;
         b->stats.vertex_bytes += p.vbytes;
     }
-    b->stats.ctas = b->run.ctas;
+    b->stats.ctas = resident;
     return MTGL_OK;
 }
 

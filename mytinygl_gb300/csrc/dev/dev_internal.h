@@ -169,7 +169,7 @@ struct Tables {
     uint32_t ndraws = 0, nrasters = 0, nclears = 0, nframes = 0;
     uint32_t slots = 0, tris = 0, ntiles = 0;
     int tile_shift = kTileShiftPlain;
-    bool eye = false, any_texture = false;
+    bool eye = false, any_texture = false, any_stencil = false;
     bool order_free = false;  // the pass renders order-free (k_tile_free.cu)
     bool occlude = false;  // some frame's pairs may be dropped behind a covering triangle (DevFrame::occlude)
     bool defer = false;  // every record a filled triangle whose colour can be deferred (k_tile.cuh)
@@ -181,16 +181,15 @@ struct Tables {
 int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframes, int tile_shift, bool may_grow,
                  Tables &t, size_t direct = 0);
 
-// CTAs of a persistent tile launch for these tables: per_sm per SM (0: all that fit)
-int persistent_ctas(const Exec &x, const Tables &t, int per_sm);
+// Resident tile CTAs for these tables: per_sm per SM (0: all that fit). *limited: fewer than fit.
+int resident_ctas(const Exec &x, const Tables &t, int per_sm, bool *limited);
 
 struct PipeConfig {
     bool exact = true;       // wait for the record and pair totals and size scratch from them
     uint32_t rec_cap = 0;    // capacity mode: records and tile pairs the scratch holds
     uint32_t pair_cap = 0;
-    int32_t ctas = 0;        // persistent tile CTAs (0: one CTA per tile)
-    bool order = false;      // hand out tiles costliest first (classified: small-record tiles first)
-    bool classify = false;   // without an order: small-record tiles by rounds, the rest per record
+    int32_t ctas = 0;        // tile CTAs that step through the tiles (0: one CTA per tile)
+    bool order = false;      // hand out tiles costliest first
 };
 
 struct PipeOut {

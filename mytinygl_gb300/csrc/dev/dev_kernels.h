@@ -77,7 +77,6 @@ struct BinArgs {
     uint32_t *keys, *vals;      // pair buffers (capacity >= pairs)
     uint32_t *keys_alt, *vals_alt;
     uint32_t *tile_count;       // per tile (ntiles + 1 entries)
-    uint32_t *tile_area;        // per tile: pixels of its records' boxes inside it, summed (may be null)
     uint32_t *tile_near;        // per tile: the occlusion bound (near_key; zero at launch); null when no
                                 // frame of the pass has one
     uint32_t *tile_start;       // exclusive scan of tile_count
@@ -108,32 +107,16 @@ size_t radix_hist_words(uint32_t npairs);
 // be zero for every tile on entry.
 int launch_tile_ranges(const BinArgs &a, cudaStream_t s);
 
-// Work order of the persistent tile launches. Tiles whose records are small (their boxes
-// cover on average less than a quarter of the tile) come first, then the others; each group
-// by descending record count (coarse log buckets), so the longest tiles start first. The
-// split point is written to aux[kOrderSplit]. order holds ntiles words, aux kOrderAuxWords.
-int launch_tile_order(const uint32_t *tile_count, const uint32_t *tile_area, uint32_t ntiles, int tile_shift,
-                      uint32_t *aux, uint32_t *order, int sms, cudaStream_t s);
-constexpr size_t kOrderSplit = 1024;      // aux word: number of small-record tiles
-constexpr size_t kOrderQueues = 1028;     // aux words: work-queue heads of the tile launches
-constexpr size_t kOrderAuxWords = 1040;
-
-// A tile's class: 0 when its records are small (their boxes cover on average under a quarter
-// of the tile), else 1. Empty tiles are class 1.
-__device__ __forceinline__ uint32_t tile_class(const uint32_t *tile_count, const uint32_t *tile_area, uint32_t t,
-                                               int tile_shift)
-{
-    const uint32_t c = tile_count[t];
-    if (c == 0 || !tile_area) return 1u;
-    return (uint64_t)tile_area[t] * 4u < ((uint64_t)c << (2 * tile_shift)) ? 0u : 1u;
-}
+// Work order of a tile launch, by descending record count (coarse log buckets), so that the
+// longest tiles start first. order holds ntiles words, aux kOrderAuxWords.
+int launch_tile_order(const uint32_t *tile_count, uint32_t ntiles, uint32_t *aux, uint32_t *order, int sms,
+                      cudaStream_t s);
+constexpr size_t kOrderAuxWords = 512;
 
 struct TileArgs {
     const float *records;
     const float *eye_records;
     const uint32_t *tile_vals;   // record indices sorted by tile, submission order within a tile
-    uint32_t *pair_mask;         // per entry of tile_vals: the warp blocks that walk it (written
-                                 // by the tile's CTA; binning's sorted keys, no longer read)
     const uint32_t *tile_start;  // per tile
     const uint32_t *tile_count;
     const uint32_t *tile_frame;  // per tile: its frame (null: found by a search of the frame table)
@@ -144,13 +127,10 @@ struct TileArgs {
     uint32_t nframes;
     uint32_t ntiles;             // work items: global tile ids
     const uint32_t *order;       // item -> tile (null: item i is tile i)
-    const uint32_t *split;       // items [0, *split) have small records (null: no split)
-    const uint32_t *tile_area;   // without an order: per-tile record-box coverage; each launch
-                                 // takes the tiles of its class in tile order (null: no classes)
-    uint32_t *queue;             // work-queue heads (two), zero at launch
-    int32_t ctas;                // persistent CTAs (0: one per tile)
+    int32_t ctas;                // CTAs that step through the tiles (0: one per tile)
     int32_t tile_shift;
     int32_t any_texture;         // some raster state of the pass samples a texture
+    int32_t any_stencil;         // some raster state of the pass tests the stencil
     // capacity check: when guard[0] > records_cap or guard[1] > pairs_cap the binning
     // dropped entries, and the launch leaves every framebuffer untouched
     const uint32_t *guard;
@@ -162,11 +142,9 @@ struct TileArgs {
     int32_t order_free;          // the pass renders order-free: tile_start holds each list's end
 };
 
-// K4: CTAs take tiles from the work queue; for each: clears, then every triangle of the
-// tile in order through the full fragment pipeline (raster.c:532-724), then one write-back.
+// K4: per tile the clears, then its triangles through the full fragment pipeline
+// (raster.c:532-724), then one write-back.
 int launch_tile(const TileArgs &a, cudaStream_t s);
-// the launch of an order-free pass (k_tile_free.cu)
-int launch_tile_free(const TileArgs &a, cudaStream_t s);
 // resident CTAs per SM of the K4 variant a launch with these arguments uses
 int tile_occupancy(const TileArgs &a);
 

@@ -391,6 +391,7 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
             R.frame = f;
             t.any_texture = t.any_texture || R.tex != nullptr;
             const uint32_t c = R.fs.ctl;
+            t.any_stencil = t.any_stencil || (c & FC_STENCIL);
             if ((c & FC_BLEND) || ((c & FC_ALPHA) && (c & FC_TEXTURE)) || !(c & (FC_MASK_ALL | FC_MASK_NONE)))
                 defer = false;  // a fragment reads the stored colour, or may be discarded after its depth test
             // A frame's hidden pairs may be dropped when every fragment that passes its depth test
@@ -437,17 +438,18 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
     return MTGL_OK;
 }
 
-int persistent_ctas(const Exec &x, const Tables &t, int per_sm)
+int resident_ctas(const Exec &x, const Tables &t, int per_sm, bool *limited)
 {
     TileArgs probe;
     memset(&probe, 0, sizeof(probe));
     probe.tile_shift = t.tile_shift;
     probe.any_texture = t.any_texture ? 1 : 0;
     probe.defer = t.defer ? 1 : 0;
+    probe.order_free = t.order_free ? 1 : 0;
     probe.eye_records = t.eye ? reinterpret_cast<const float *>(1) : nullptr;
     const int occ = tile_occupancy(probe);
-    const int n = per_sm > 0 ? std::min(per_sm, occ) : occ;
-    return std::max(1, n) * x.sms;
+    *limited = per_sm > 0 && per_sm < occ;
+    return std::max(1, *limited ? per_sm : occ) * x.sms;
 }
 
 // ------------------------------------------------------------------ the pipeline
@@ -477,18 +479,14 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     // clip list, its class words, the class-sorted list, the class counters and the emit list
     uint32_t *clip_list = nullptr;
     if ((rc = sc.take(S_CLIP_LIST, 4 * (size_t)tris + kClipBuckets, &clip_list))) return rc;
-    // tile counts, then per tile the record-box coverage (classified launches) or else the
-    // occlusion bound
+    // tile counts, then the occlusion bounds
     if ((rc = sc.take(S_TILE_COUNT, 2 * ((size_t)ntiles + 1), &tile_count))) return rc;
-    // record-box coverage per tile, for the split between tiles run by rounds and per record;
-    // deferred-colour passes run every tile per record (their fragments are cheap: tests only)
-    uint32_t *tile_area = (c.ctas && (c.order || c.classify) && !t.defer) ? tile_count + ntiles + 1 : nullptr;
-    uint32_t *tile_near = t.occlude && !tile_area ? tile_count + ntiles + 1 : nullptr;
+    uint32_t *tile_near = t.occlude ? tile_count + ntiles + 1 : nullptr;
     if ((rc = sc.take(S_TILE_START, (size_t)ntiles + 1, &tile_start))) return rc;
     uint32_t *tile_frame = nullptr;  // batches: each tile's frame, found once by the range pass
     if (t.nframes > 1 && (rc = sc.take(S_TILE_FRAME, ntiles, &tile_frame))) return rc;
-    if (c.ctas && c.order && (rc = sc.take(S_ORDER, ntiles, &order))) return rc;
-    if (c.ctas && (rc = sc.take(S_ORDER_AUX, kOrderAuxWords, &order_aux))) return rc;
+    if (c.order && ((rc = sc.take(S_ORDER, ntiles, &order)) || (rc = sc.take(S_ORDER_AUX, kOrderAuxWords, &order_aux))))
+        return rc;
     uint32_t scan_n = std::max<uint32_t>(std::max(tris, ntiles), 1);
     if (!c.exact) {
         scan_n = std::max<uint32_t>(scan_n, c.rec_cap);
@@ -564,7 +562,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     x.prof_mark();
 
     // ---- binning
-    CK(cudaMemsetAsync(tile_count, 0, (tile_area || tile_near ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
+    CK(cudaMemsetAsync(tile_count, 0, (tile_near ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     // (an order-free pass's scan writes every tile's start)
     if (!t.order_free || !rec_cap) CK(cudaMemsetAsync(tile_start, 0, ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     BinArgs ba;
@@ -578,7 +576,6 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ba.ntiles = ntiles;
     ba.rec_tiles = rec_tiles;
     ba.tile_count = tile_count;
-    ba.tile_area = tile_area;
     ba.tile_near = tile_near;
     ba.tile_start = tile_start;
     ba.tile_frame = tile_frame;
@@ -629,7 +626,6 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ta.records = records;
     ta.eye_records = eye_records;
     ta.tile_vals = rec_cap ? ba.vals : nullptr;
-    ta.pair_mask = rec_cap ? ba.keys : nullptr;
     ta.debug = x.d_totals + kDebugStatusWord;
     ta.records_cap = rec_cap;
     ta.entries_cap = rec_cap ? pair_cap : 0u;
@@ -644,25 +640,14 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ta.ntiles = ntiles;
     ta.tile_shift = t.tile_shift;
     ta.any_texture = t.any_texture ? 1 : 0;
+    ta.any_stencil = t.any_stencil ? 1 : 0;
     ta.defer = t.defer ? 1 : 0;
     ta.fragments = x.d_frags;
     ta.order_free = t.order_free && rec_cap ? 1 : 0;
-    if (ta.order_free) {  // one CTA per tile: no work queue
-        if (order) {
-            launches += launch_tile_order(tile_count, nullptr, ntiles, t.tile_shift, order_aux, order, x.sms, s);
-            ta.order = order;
-        }
-    } else if (c.ctas) {
-        ta.queue = order_aux + kOrderQueues;
-        if (order) {  // clears the queue heads too
-            launches += launch_tile_order(tile_count, tile_area, ntiles, t.tile_shift, order_aux, order, x.sms, s);
-            ta.order = order;
-            ta.split = order_aux + kOrderSplit;
-        } else {
-            CK(cudaMemsetAsync(ta.queue, 0, 2 * sizeof(uint32_t), s));
-            ta.tile_area = tile_area;  // classes, tile order
-        }
-        ta.ctas = c.ctas;
+    ta.ctas = c.ctas;
+    if (order) {
+        launches += launch_tile_order(tile_count, ntiles, order_aux, order, x.sms, s);
+        ta.order = order;
     }
     if (!c.exact) {
         ta.guard = x.d_totals;

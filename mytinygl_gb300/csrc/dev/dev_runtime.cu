@@ -86,12 +86,8 @@ void pack_frag_state(DevRaster &R)
     f.color_mask = mask;
     memcpy(f.fog_color, rs.fog_color, sizeof(f.fog_color));
     memcpy(f.tex_env_color, rs.tex_env_color, sizeof(f.tex_env_color));
-    f.tex = R.tex;
-    f.mip1 = R.mip1;
-    f.tex_w = R.tex_w;
-    f.tex_h = R.tex_h;
-    f.mip_w = R.mip_w;
-    f.mip_h = R.mip_h;
+    f.level[0] = DevMip{R.tex, R.tex_w, R.tex_h};
+    f.level[1] = DevMip{R.mip1, R.mip_w, R.mip_h};
     f.wrap_s = rs.tex_wrap_s;
     f.wrap_t = rs.tex_wrap_t;
     f.min_filter = rs.tex_min_filter;
@@ -187,19 +183,6 @@ int run_clears_only(mtgl_dev *d)
     return MTGL_OK;
 }
 
-// Exact sizing. A large pass runs the tile kernel persistently in two launches, tiles of
-// small records by rounds and the rest per record, each in tile order; a small one, where
-// those extra launches would cost more than they save, with one CTA per tile.
-PipeConfig plain_config(mtgl_dev *d, const Tables &t)
-{
-    PipeConfig c;
-    if (t.tris >= 32768) {
-        c.ctas = persistent_ctas(d->x, t, 0);
-        c.classify = true;  // one frame: tile order keeps neighbouring tiles' records in cache together
-    }
-    return c;
-}
-
 int flush_pass(mtgl_dev *d)
 {
     int st = mtgl_dev_enter(d);
@@ -209,7 +192,7 @@ int flush_pass(mtgl_dev *d)
     FrameSrc fs{d, &P, 0};
     Tables t;
     if ((st = build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, true, t))) return st;
-    PipeConfig c = plain_config(d, t);
+    PipeConfig c;  // exact sizing
     PipeOut o;
     if ((st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o))) return st;
     if ((st = d->stage.mark_uploaded(d->x.stream))) return st;
@@ -906,7 +889,7 @@ int flush_pass_noalloc(mtgl_dev *d)
     }
     // the previous call's kernels (any context, any stream) are done with the array first
     if (nd->pending) CK(cudaStreamWaitEvent(d->x.stream, nd->done, 0));
-    PipeConfig c = plain_config(d, t);
+    PipeConfig c;  // exact sizing
     PipeOut o;
     st = run_pipeline(d->x, cv, d->stage, t, c, &o);
     // whatever this call enqueued, the next call waits for it

@@ -445,12 +445,6 @@ __global__ void __launch_bounds__(kRecWarps * 32) k_bin_records(BinArgs A)
                         const uint32_t tile = t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
                         A.keys[pos] = tile;
                         A.vals[pos] = r0 + j;
-                        if (A.tile_area) {  // pixels of the record's box inside this tile
-                            const int sh = A.tile_shift, x = (t.tx0 + col) << sh, y = (t.ty0 + row) << sh;
-                            const int ox = min((int)(t.mx & 0xFFFFu), x + (1 << sh) - 1) - max((int)(t.mn & 0xFFFFu), x) + 1;
-                            const int oy = min((int)(t.mx >> 16), y + (1 << sh) - 1) - max((int)(t.mn >> 16), y) + 1;
-                            atomicAdd(A.tile_area + tile, (uint32_t)(ox * oy));
-                        }
                     }
                 }
                 kept += (uint32_t)__popc(m);
@@ -549,64 +543,49 @@ __device__ __forceinline__ uint32_t cost_bucket(uint32_t c)
     return min(1u + (uint32_t)lg * 8u + frac, 255u);
 }
 
-// aux[0..511]: tiles per (class, bucket); aux[512..1023]: placement cursors; all zero at launch
-__global__ void __launch_bounds__(256) k_order_hist(const uint32_t *tile_count, const uint32_t *tile_area,
-                                                    uint32_t ntiles, int tile_shift, uint32_t *aux)
+// aux[0..255]: tiles per bucket; aux[256..511]: placement cursors; all zero at launch
+__global__ void __launch_bounds__(256) k_order_hist(const uint32_t *tile_count, uint32_t ntiles, uint32_t *aux)
 {
-    __shared__ uint32_t h[512];
+    __shared__ uint32_t h[256];
     h[threadIdx.x] = 0;
-    h[threadIdx.x + 256] = 0;
     __syncthreads();
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x)
-        atomicAdd(&h[tile_class(tile_count, tile_area, t, tile_shift) * 256 + cost_bucket(tile_count[t])], 1u);
+        atomicAdd(&h[cost_bucket(tile_count[t])], 1u);
     __syncthreads();
     if (h[threadIdx.x]) atomicAdd(&aux[threadIdx.x], h[threadIdx.x]);
-    if (h[threadIdx.x + 256]) atomicAdd(&aux[threadIdx.x + 256], h[threadIdx.x + 256]);
 }
 
-// Places every tile after all tiles of earlier groups: class 0 before class 1, costlier
-// buckets first within a class. The order inside a bucket is whatever the atomics give:
-// tiles are independent, so it changes timing only.
-__global__ void __launch_bounds__(256) k_order_scatter(const uint32_t *tile_count, const uint32_t *tile_area,
-                                                       uint32_t ntiles, int tile_shift, uint32_t *aux,
+// Places every tile after all tiles of costlier buckets. The order inside a bucket is whatever
+// the atomics give: tiles are independent, so it changes timing only.
+__global__ void __launch_bounds__(256) k_order_scatter(const uint32_t *tile_count, uint32_t ntiles, uint32_t *aux,
                                                        uint32_t *order)
 {
-    __shared__ uint32_t start[512];
+    __shared__ uint32_t start[256];
     __shared__ uint32_t warp_tot[8];
-    // positions p = 2*thread, 2*thread+1 in placement order: class p / 256, bucket 255 - p % 256
-    const int p0 = 2 * (int)threadIdx.x, p1 = p0 + 1;
-    const int e0 = (p0 / 256) * 256 + (255 - p0 % 256), e1 = (p1 / 256) * 256 + (255 - p1 % 256);
-    const uint32_t v0 = aux[e0], v1 = aux[e1];
+    const int e = 255 - (int)threadIdx.x;  // costliest first
+    const uint32_t v = aux[e];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t x = v0 + v1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
+    const uint32_t x = warp_incl_scan(v);
     if (lane == 31) warp_tot[warp] = x;
     __syncthreads();
     uint32_t before = 0;
     for (int w = 0; w < warp; w++) before += warp_tot[w];
-    const uint32_t excl = before + x - (v0 + v1);
-    start[e0] = excl;
-    start[e1] = excl + v0;
-    if (blockIdx.x == 0 && threadIdx.x == 127) aux[kOrderSplit] = before + x;  // end of class 0
+    start[e] = before + x - v;
     __syncthreads();
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += gridDim.x * blockDim.x) {
-        const uint32_t e = tile_class(tile_count, tile_area, t, tile_shift) * 256 + cost_bucket(tile_count[t]);
-        order[start[e] + atomicAdd(&aux[512 + e], 1u)] = t;
+        const uint32_t k = cost_bucket(tile_count[t]);
+        order[start[k] + atomicAdd(&aux[256 + k], 1u)] = t;
     }
 }
 
-int launch_tile_order(const uint32_t *tile_count, const uint32_t *tile_area, uint32_t ntiles, int tile_shift,
-                      uint32_t *aux, uint32_t *order, int sms, cudaStream_t s)
+int launch_tile_order(const uint32_t *tile_count, uint32_t ntiles, uint32_t *aux, uint32_t *order, int sms,
+                      cudaStream_t s)
 {
     if (!ntiles) return 0;
     cudaMemsetAsync(aux, 0, kOrderAuxWords * sizeof(uint32_t), s);
     const unsigned g = stride_grid(ntiles, 256, sms);
-    k_order_hist<<<g, 256, 0, s>>>(tile_count, tile_area, ntiles, tile_shift, aux);
-    k_order_scatter<<<g, 256, 0, s>>>(tile_count, tile_area, ntiles, tile_shift, aux, order);
+    k_order_hist<<<g, 256, 0, s>>>(tile_count, ntiles, aux);
+    k_order_scatter<<<g, 256, 0, s>>>(tile_count, ntiles, aux, order);
     return 2;
 }
 

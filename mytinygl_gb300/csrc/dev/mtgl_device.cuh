@@ -187,8 +187,8 @@ enum FragCtl : uint32_t {
     FC_AFFINE_UV = 1u << 5, FC_FOG = 1u << 6, FC_BLEND = 1u << 7, FC_DEFAULT_RANGE = 1u << 8,
     FC_MASK_ALL = 1u << 9, FC_MASK_NONE = 1u << 10, FC_TEXTURE = 1u << 11
 };
-// A texture level beyond 1 (MTGL_OPT_MIPMAP_CHAIN): packed RGBA8 texels, row-major.
-struct DevMip {
+// A texture level: packed RGBA8 texels, row-major (px null: a level that cannot be built).
+struct __align__(16) DevMip {
     const uint32_t *px;
     int32_t w, h;
 };
@@ -206,8 +206,7 @@ struct __align__(16) FragState {
     uint32_t pad0;
     float fog_color[4];
     float tex_env_color[4];
-    const uint32_t *tex, *mip1;            // texture: levels 0 and 1 (see DevRaster)
-    int32_t tex_w, tex_h, mip_w, mip_h;
+    DevMip level[2];                       // texture: levels 0 and 1 (see DevRaster)
     int32_t wrap_s, wrap_t, min_filter, mag_filter;
     const DevMip *chain;                   // levels 2.. (MTGL_OPT_MIPMAP_CHAIN), or null
     int32_t chain_levels, pad1;            // how many (0: the reference's two levels)
@@ -216,8 +215,8 @@ struct __align__(16) FragState {
 static_assert(sizeof(FragState) == 176 && offsetof(FragState, chain) == 160 && offsetof(FragState, stencil_func) == 16 &&
                   offsetof(FragState, stencil_fail) == 32 && offsetof(FragState, blend_src) == 48 &&
                   offsetof(FragState, fog_start) == 64 && offsetof(FragState, fog_color) == 80 &&
-                  offsetof(FragState, tex_env_color) == 96 && offsetof(FragState, tex) == 112 &&
-                  offsetof(FragState, tex_w) == 128 && offsetof(FragState, wrap_s) == 144,
+                  offsetof(FragState, tex_env_color) == 96 && offsetof(FragState, level) == 112 &&
+                  sizeof(DevMip) == 16 && offsetof(FragState, wrap_s) == 144,
               "FragState groups are read as 16-byte words");
 
 // Raster state with the bound texture resolved to device pointers.
@@ -411,17 +410,16 @@ __device__ __forceinline__ float4 mul_m4(const float *m, float x, float y, float
 
 __device__ __forceinline__ bool cmp_pass(uint32_t func, float a, float b)
 {
-    switch (func) {
-    case GL_NEVER: return false;
-    case GL_LESS: return a < b;
-    case GL_EQUAL: return a == b;
-    case GL_LEQUAL: return a <= b;
-    case GL_GREATER: return a > b;
-    case GL_NOTEQUAL: return a != b;
-    case GL_GEQUAL: return a >= b;
-    default: return true;
-    }
+    // the comparison functions are GL_NEVER + a mask of less (1), equal (2) and greater (4); an
+    // unordered pair passes GL_NOTEQUAL and GL_ALWAYS, the two with less and greater
+    const uint32_t r = a < b ? 1u : (a == b ? 2u : (a > b ? 4u : 8u));
+    const uint32_t f = func & 7u;
+    return ((f | ((f & 5u) == 5u ? 8u : 0u)) & r) != 0u;
 }
+static_assert(GL_LESS == GL_NEVER + 1 && GL_EQUAL == GL_NEVER + 2 && GL_LEQUAL == GL_NEVER + 3 &&
+                  GL_GREATER == GL_NEVER + 4 && GL_NOTEQUAL == GL_NEVER + 5 && GL_GEQUAL == GL_NEVER + 6 &&
+                  GL_ALWAYS == GL_NEVER + 7 && (GL_NEVER & 7) == 0,
+              "comparison functions as masks");
 
 // ------------------------------------------------------------------ lighting (lighting.h:53-142)
 
@@ -514,39 +512,43 @@ __device__ __forceinline__ int32_t wrap_next(int32_t xa, int32_t x, int32_t n, b
     return wrap_coord(x + 1, n, false);
 }
 
-__device__ __forceinline__ uint32_t texel_at(const TexView &t, int32_t x, int32_t y)
+// One axis of a bilinear sample at texel coordinate t of an n-texel axis: the two texels and the
+// weight of the second.
+struct TexAxis {
+    int32_t a, b;
+    float f;
+};
+static __device__ __noinline__ TexAxis tex_axis_any(float t, int32_t n, bool repeat)
 {
-    return __ldg(t.px + (size_t)y * t.w + x);
+    const int32_t i = x86_f2i(floorf(t));
+    const int32_t a = wrap_coord(i, n, repeat);
+    return TexAxis{a, wrap_next(a, i, n, repeat), t - (float)i};
+}
+// A wrapped or clamped coordinate u in [0, 1] gives t = u * n - 0.5 in [-0.5, n - 0.5], whose
+// texels need a wrap only past the ends; anything else (NaN, infinities) goes the general way.
+__device__ __forceinline__ TexAxis tex_axis(float t, int32_t n, float fn, bool repeat)
+{
+    if (!(t >= -1.0f && t < fminf(fn, 0x1p22f))) return tex_axis_any(t, n, repeat);
+    float fl;
+    const int32_t i = small_floor(t, &fl);  // -1 .. n - 1
+    return TexAxis{i < 0 ? (repeat ? n - 1 : 0) : i, i + 1 < n ? i + 1 : (repeat ? 0 : n - 1), t - fl};
 }
 
 // texture_sample_nearest / _linear on one level, as the colour of the stored bytes
 __device__ __forceinline__ float4 sample_level(const TexView &t, int32_t ws, int32_t wt, float u, float v, bool linear)
 {
-    float tx = u * (float)t.w - 0.5f;
-    float ty = v * (float)t.h - 0.5f;
+    const float fw = (float)t.w, fh = (float)t.h;
+    float tx = u * fw - 0.5f;
+    float ty = v * fh - 0.5f;
     if (linear) {
-        int32_t x0, y0;
-        float fx, fy;
-        if (fabsf(tx) < 0x1p22f && fabsf(ty) < 0x1p22f) {  // every in-range coordinate
-            float flx, fly;
-            x0 = small_floor(tx, &flx);
-            y0 = small_floor(ty, &fly);
-            fx = tx - flx;
-            fy = ty - fly;
-        } else {
-            x0 = x86_f2i(floorf(tx));
-            y0 = x86_f2i(floorf(ty));
-            fx = tx - (float)x0;
-            fy = ty - (float)y0;
-        }
-        const bool rs = ws == GL_REPEAT, rt = wt == GL_REPEAT;
-        const int32_t xa = wrap_coord(x0, t.w, rs), xb = wrap_next(xa, x0, t.w, rs);
-        const int32_t ya = wrap_coord(y0, t.h, rt), yb = wrap_next(ya, y0, t.h, rt);
-        const uint32_t *ra = t.px + (size_t)ya * t.w, *rb = t.px + (size_t)yb * t.w;
-        const uint32_t p00 = __ldg(ra + xa), p10 = __ldg(ra + xb), p01 = __ldg(rb + xa), p11 = __ldg(rb + xb);
-        const float4 top = lerp_col(unpack_rgba(p00), unpack_rgba(p10), fx);
-        const float4 bot = lerp_col(unpack_rgba(p01), unpack_rgba(p11), fx);
-        return quantize(lerp_col(top, bot, fy));
+        const TexAxis x = tex_axis(tx, t.w, fw, ws == GL_REPEAT), y = tex_axis(ty, t.h, fh, wt == GL_REPEAT);
+        // a level holds at most 2^32 texels: 32-bit offsets
+        const uint32_t ra = (uint32_t)y.a * (uint32_t)t.w, rb = (uint32_t)y.b * (uint32_t)t.w;
+        const uint32_t p00 = __ldg(t.px + (ra + x.a)), p10 = __ldg(t.px + (ra + x.b));
+        const uint32_t p01 = __ldg(t.px + (rb + x.a)), p11 = __ldg(t.px + (rb + x.b));
+        const float4 top = lerp_col(unpack_rgba(p00), unpack_rgba(p10), x.f);
+        const float4 bot = lerp_col(unpack_rgba(p01), unpack_rgba(p11), x.f);
+        return quantize(lerp_col(top, bot, y.f));
     }
     const float hx = tx + 0.5f, hy = ty + 0.5f;
     int32_t x, y;
@@ -562,13 +564,7 @@ __device__ __forceinline__ float4 sample_level(const TexView &t, int32_t ws, int
     if (x >= t.w) x = t.w - 1;
     if (y < 0) y = 0;
     if (y >= t.h) y = t.h - 1;
-    return unpack_rgba(__ldg(t.px + (size_t)y * t.w + x));
-}
-
-// a pointer field through the read-only path
-__device__ __forceinline__ const uint32_t *ldg_ptr(const uint32_t *const *p)
-{
-    return reinterpret_cast<const uint32_t *>(__ldg(reinterpret_cast<const unsigned long long *>(p)));
+    return unpack_rgba(__ldg(t.px + (uint32_t)y * (uint32_t)t.w + x));
 }
 
 // (float)x86_f2i(f): the truncated value as a float (INT32_MIN outside the int range)
@@ -583,10 +579,12 @@ __device__ __forceinline__ float trunc_f2i_f(float f)
 // Level d of a texture (0: base, 1: mip1, null when it cannot be built; 2..: the chain).
 __device__ __forceinline__ TexView tex_level(const FragState &S, int d)
 {
-    if (d == 0) return TexView{ldg_ptr(&S.tex), __ldg(&S.tex_w), __ldg(&S.tex_h)};
-    if (d == 1) return TexView{ldg_ptr(&S.mip1), __ldg(&S.mip_w), __ldg(&S.mip_h)};
-    const DevMip *m = reinterpret_cast<const DevMip *>(__ldg(reinterpret_cast<const unsigned long long *>(&S.chain)));
-    return TexView{ldg_ptr(&m[d - 2].px), __ldg(&m[d - 2].w), __ldg(&m[d - 2].h)};
+    const DevMip *m = S.level + d;
+    if (d > 1)
+        m = reinterpret_cast<const DevMip *>(__ldg(reinterpret_cast<const unsigned long long *>(&S.chain))) + (d - 2);
+    const int4 q = __ldg(reinterpret_cast<const int4 *>(m));
+    const uint64_t px = (uint64_t)(uint32_t)q.x | ((uint64_t)(uint32_t)q.y << 32);
+    return TexView{reinterpret_cast<const uint32_t *>(px), q.z, q.w};
 }
 
 // texture_sample_lod (textures.c:457-557) on the packed texture state, as the colour of the
@@ -685,18 +683,9 @@ __device__ __forceinline__ float4 blend(const mtgl_raster_state &rs, float4 s, f
 
 __device__ __forceinline__ bool stencil_pass(uint32_t func, int32_t ref, uint32_t mask, uint32_t val)
 {
-    int32_t mr = (int32_t)((uint32_t)ref & mask);
-    int32_t mv = (int32_t)(val & mask);
-    switch (func) {
-    case GL_NEVER: return false;
-    case GL_LESS: return mr < mv;
-    case GL_EQUAL: return mr == mv;
-    case GL_LEQUAL: return mr <= mv;
-    case GL_GREATER: return mr > mv;
-    case GL_NOTEQUAL: return mr != mv;
-    case GL_GEQUAL: return mr >= mv;
-    default: return true;
-    }
+    const int32_t mr = (int32_t)((uint32_t)ref & mask);
+    const int32_t mv = (int32_t)(val & mask);
+    return (func & (mr < mv ? 1u : (mr == mv ? 2u : 4u))) != 0u;  // see cmp_pass
 }
 
 __device__ __forceinline__ uint32_t stencil_apply(uint32_t op, uint32_t v, int32_t ref)
