@@ -315,6 +315,8 @@ namespace {
 int involve(mtgl_batch *b, mtgl_dev *d, bool write)
 {
     if (d->device != b->x.device) return MTGL_ERR_INVALID;
+    int settled = mtgl_dev_settle(d);
+    if (settled) return settled;
     bool known = false;
     for (mtgl_dev *e : b->devs) known = known || e == d;
     for (mtgl_dev *e : b->sources) known = known || e == d;

@@ -139,7 +139,8 @@ struct Exec {
     uint64_t allocs = 0;  // device allocations of the staging copy
     uint32_t *d_totals = nullptr;  // [0] records, [1] pairs, [2] tiles' records, [3] sort scratch, [4] clip list, [5] emit list (GeomArgs::list_counts),
                                    // [kDebugStatusWord] the debug bounds checks' status
-    uint32_t *h_totals = nullptr;  // pinned copy of [0..1]
+    uint32_t *h_totals = nullptr;  // page-locked copy of [0..1]
+    uint32_t rec_seen = 0, pair_seen = 0;  // largest totals of this Exec's passes: later passes' capacities
     unsigned long long *d_frags = nullptr;
     // per-phase profiling: 5 events per pass (before K1, after K1, after K2, after K3, after K4)
     bool profile = false;
@@ -219,6 +220,11 @@ struct mtgl_dev {
     uint64_t alloc_base = 0;  // allocation count at the last reset of the counters
     bool depth_rejection = true;
     bool mipmap_chain = false;  // MTGL_OPT_MIPMAP_CHAIN
+    // the last flushed pass ran with capacities and has not been checked against its totals; its
+    // tables are still staged
+    bool unsettled = false;
+    mtgl::Tables ran_t;
+    mtgl::PipeConfig ran_c;
     // ordering against batches, which run on their own streams: work of this context's
     // stream that a batch must wait for, and a batch this context's stream must wait for
     cudaEvent_t tail = nullptr;
@@ -231,3 +237,7 @@ struct mtgl_dev {
 
 // Every entry that enqueues work on a context's stream goes through here first.
 int mtgl_dev_enter(mtgl_dev *d);
+// Settles the context's last flushed pass (waits for it, renders it again with exact sizing if
+// its capacities did not hold): before its staging area is written, its stream is used or its
+// framebuffer is read.
+int mtgl_dev_settle(mtgl_dev *d);

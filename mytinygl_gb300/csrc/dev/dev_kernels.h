@@ -58,8 +58,9 @@ int launch_setup_emit(const GeomArgs &a, cudaStream_t s);
 // 8-byte aligned; debug is the
 // status word its bounded waits report to (may be null).
 size_t scan_temp_words(uint32_t n);
+// With `host` (two page-locked words) the launch also writes *rec_total and the total there.
 int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
-                cudaStream_t s);
+                cudaStream_t s, const uint32_t *rec_total = nullptr, uint32_t *host = nullptr);
 
 // Element counts of the binning stage live on the device (written by the scans), so the
 // stage runs without the host knowing them. `nrec` / `npairs` on the host are capacities:
@@ -84,6 +85,7 @@ struct BinArgs {
     uint32_t *radix_hist;       // radix histograms
     uint32_t *scan_temp;
     uint32_t *total_dev;        // where the pair scan writes its total: the pairs generated
+    uint32_t *totals_host;      // page-locked words that get the record and pair totals (may be null)
     uint32_t *sort_total_dev;   // a word the sort's histogram scans may overwrite
     int32_t order_free;         // tile lists need no order (k_tile_free.cu)
     uint32_t npairs;            // pair capacity of keys/vals (writes beyond are dropped)

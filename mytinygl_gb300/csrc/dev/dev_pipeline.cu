@@ -581,6 +581,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ba.tile_frame = tile_frame;
     ba.total_dev = x.d_totals + 1;
     ba.sort_total_dev = x.d_totals + 3;
+    ba.totals_host = c.exact ? nullptr : x.h_totals;
     ba.debug = x.d_totals + kDebugStatusWord;
     ba.order_free = t.order_free ? 1 : 0;
     ba.scan_temp = scan_temp;
@@ -618,6 +619,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         }
     } else {
         CK(cudaMemsetAsync(x.d_totals + 1, 0, sizeof(uint32_t), s));
+        if (!c.exact) CK(cudaMemcpyAsync(x.h_totals, x.d_totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     }
     x.prof_mark();
 
@@ -656,7 +658,6 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     launches += launch_tile(ta, s);
     x.prof_mark();
     CK(cudaGetLastError());
-    if (!c.exact) CK(cudaMemcpyAsync(x.h_totals, x.d_totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     o.launches = launches;
     if (out) *out = o;
     return MTGL_OK;

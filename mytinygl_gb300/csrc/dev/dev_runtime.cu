@@ -183,6 +183,33 @@ int run_clears_only(mtgl_dev *d)
     return MTGL_OK;
 }
 
+// Capacities of a pass's records and pairs: the largest totals the context has seen, or for its
+// first passes an estimate: 9/8 records per filled triangle, 25/8 for polygon modes drawn as
+// points or lines; four pairs per record, and at least 2^18 (a few megabytes) unless the frame
+// cannot have that many. Totals beyond them cost one more run of the pass (mtgl_dev_settle).
+// A pass of more than 2^22 primitives, whose records may be gigabytes of which few are
+// needed, takes exact sizes instead: its two waits are nothing beside it.
+PipeConfig capacities(const mtgl_dev *d, const Tables &t)
+{
+    const Pass &P = d->pass;
+    if (P.tris > (1u << 22)) return PipeConfig();
+    uint64_t recs = 64;
+    for (const PendingDraw &pd : P.draws) {
+        const mtgl_raster_state &rs = P.rasters[pd.d.raster].rs;
+        const bool fill = pd.d.mode < GL_TRIANGLES ||
+                          (rs.polygon_mode_front == GL_FILL && rs.polygon_mode_back == GL_FILL);
+        recs += (uint64_t)pd.d.tri_count * (fill ? 1u : 3u) + pd.d.tri_count / 8;  // clipping splits some
+    }
+    recs = std::max<uint64_t>(recs, d->x.rec_seen);
+    uint64_t pairs = std::max<uint64_t>(std::max<uint64_t>(4 * recs, d->x.pair_seen), 1u << 18);
+    pairs = std::min<uint64_t>(pairs, recs * std::max<uint32_t>(t.ntiles, 1u));
+    PipeConfig c;
+    c.exact = false;
+    c.rec_cap = (uint32_t)std::min<uint64_t>(recs, 0x7FFFFF00ull);
+    c.pair_cap = (uint32_t)std::min<uint64_t>(pairs, 0xFFFFFF00ull);
+    return c;
+}
+
 int flush_pass(mtgl_dev *d)
 {
     int st = mtgl_dev_enter(d);
@@ -192,19 +219,25 @@ int flush_pass(mtgl_dev *d)
     FrameSrc fs{d, &P, 0};
     Tables t;
     if ((st = build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, true, t))) return st;
-    PipeConfig c;  // exact sizing
+    const PipeConfig c = capacities(d, t);
     PipeOut o;
     if ((st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o))) return st;
     if ((st = d->stage.mark_uploaded(d->x.stream))) return st;
+    if (c.exact) {
+        d->stats.setup_triangles += o.nrec;
+        d->stats.bin_entries += o.npairs;
+        d->stage.used = 0;
+    } else {
+        d->unsettled = true;
+        d->ran_t = t;
+        d->ran_c = c;
+    }
     d->stats.passes++;
     d->stats.input_triangles += P.tris;
     d->stats.vertices += P.slots;
     d->stats.vertex_bytes += P.vbytes;
-    d->stats.setup_triangles += o.nrec;
-    d->stats.bin_entries += o.npairs;
     d->stats.kernel_launches += (uint64_t)o.launches;
     P.reset();
-    d->stage.used = 0;
     return MTGL_OK;
 }
 
@@ -226,8 +259,37 @@ extern "C" int dev_current_device(void)
     return cudaGetDevice(&d) == cudaSuccess ? d : -1;
 }
 
+int mtgl_dev_settle(mtgl_dev *d)
+{
+    if (!d->unsettled) return MTGL_OK;
+    d->unsettled = false;  // a failure below leaves nothing to retry
+    const int st = d->stage.wait();
+    if (st) return st;
+    uint32_t nrec = d->x.h_totals[0], npairs = d->x.h_totals[1];
+    if (nrec > d->ran_c.rec_cap || npairs > d->ran_c.pair_cap) {
+        // the tile launch left the framebuffer untouched: run the staged tables again
+        PipeConfig c;
+        PipeOut o;
+        int rc = run_pipeline(d->x, d->x.pool, d->stage, d->ran_t, c, &o);
+        if (rc || (rc = d->stage.mark_uploaded(d->x.stream)) || (rc = d->stage.wait())) return rc;
+        nrec = o.nrec;
+        npairs = o.npairs;
+        d->stats.kernel_launches += (uint64_t)o.launches;
+    }
+    d->x.rec_seen = std::max(d->x.rec_seen, nrec);
+    d->x.pair_seen = std::max(d->x.pair_seen, npairs);
+    d->stats.setup_triangles += nrec;
+    d->stats.bin_entries += npairs;
+    d->stage.used = 0;
+    return MTGL_OK;
+}
+
 int mtgl_dev_enter(mtgl_dev *d)
 {
+    if (d->unsettled) {
+        int st = mtgl_dev_settle(d);
+        if (st) return st;
+    }
     if (d->batch) {
         int st = mtgl_dev_batch_wait(d->batch);  // verifies (and if needed re-runs) the batch
         if (st) return st;
@@ -544,9 +606,9 @@ int mtgl_dev_draw(mtgl_dev *d, const mtgl_draw *dr)
         if (st) return st;
         if (ntri > 0x7FFFFFFFull) return MTGL_ERR_INVALID;
     }
+    int st = mtgl_dev_settle(d);
+    if (st || (st = d->stage.wait())) return st;
     const size_t staged0 = d->stage.used;
-    int st = d->stage.wait();
-    if (st) return st;
 
     PendingDraw p;
     memset(&p.d, 0, sizeof(p.d));
@@ -621,7 +683,7 @@ int mtgl_dev_draw_pixels(mtgl_dev *d, int32_t rx, int32_t ry, int32_t w, int32_t
     if (w <= 0 || h <= 0 || !rgba32) return MTGL_OK;
     CK(cudaSetDevice(d->device));
     int st = flush_pass(d);
-    if (st) return st;
+    if (st || (st = mtgl_dev_settle(d))) return st;
     DevRaster R;
     memset(&R, 0, sizeof(R));
     R.rs = *rs;
@@ -658,7 +720,7 @@ int mtgl_dev_finish(mtgl_dev *d)
     if (!d) return MTGL_ERR_INVALID;
     CK(cudaSetDevice(d->device));
     int st = flush_pass(d);
-    if (st) return st;
+    if (st || (st = mtgl_dev_settle(d))) return st;
     CK(cudaStreamSynchronize(d->x.stream));
     return MTGL_OK;
 }

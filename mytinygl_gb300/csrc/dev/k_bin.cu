@@ -71,7 +71,7 @@ __device__ __forceinline__ void st_status(uint64_t *p, uint64_t v) { *(volatile 
 
 __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint32_t *out, uint32_t n,
                                                       uint64_t *status, uint32_t *ticket, uint32_t *total_dev,
-                                                      uint32_t *debug)
+                                                      uint32_t *debug, const uint32_t *rec_total, uint32_t *host)
 {
     __shared__ uint32_t s_tile, s_prefix;
     if (threadIdx.x == 0) s_tile = gridDim.x == 1 ? 0u : atomicAdd(ticket, 1u);
@@ -121,7 +121,13 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
         }
         if (lane == 0) {
             s_prefix = prefix;
-            if (tile + 1 == gridDim.x) *total_dev = prefix + agg;
+            if (tile + 1 == gridDim.x) {
+                *total_dev = prefix + agg;
+                if (host) {  // page-locked: the pass's record and pair totals, without a copy behind it
+                    host[0] = *rec_total;
+                    host[1] = prefix + agg;
+                }
+            }
         }
     }
     __syncthreads();
@@ -149,7 +155,7 @@ size_t scan_temp_words(uint32_t n)
 }
 
 int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
-                cudaStream_t s)
+                cudaStream_t s, const uint32_t *rec_total, uint32_t *host)
 {
     if (n == 0) {
         cudaMemsetAsync(total_dev, 0, sizeof(uint32_t), s);
@@ -161,7 +167,7 @@ int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, u
     uint64_t *status = reinterpret_cast<uint64_t *>(temp);
     uint32_t *ticket = temp + 2 * (size_t)nb;
     if (nb > 1) cudaMemsetAsync(temp, 0, (2 * (size_t)nb + 1) * sizeof(uint32_t), s);
-    k_scan<<<nb, kScanThreads, 0, s>>>(in, out, n, status, ticket, total_dev, debug);
+    k_scan<<<nb, kScanThreads, 0, s>>>(in, out, n, status, ticket, total_dev, debug, rec_total, host);
     return 1;
 }
 
@@ -521,9 +527,10 @@ int launch_bin_count(const BinArgs &a, cudaStream_t s)
     if (!a.nrec) return 0;
     const int occlude = a.tile_near ? launch_records<PASS_OCCLUDE>(a, s) : 0;
     if (!a.order_free) return occlude + launch_records<PASS_COUNT>(a, s) +
-                              launch_scan(a.rec_tiles, a.rec_tiles, a.units, a.scan_temp, a.total_dev, a.debug, s);
+                              launch_scan(a.rec_tiles, a.rec_tiles, a.units, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev,
+                                          a.totals_host);
     return occlude + launch_records<PASS_COUNT_FREE>(a, s) +
-           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.total_dev, a.debug, s);
+           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev, a.totals_host);
 }
 
 int launch_bin_expand(const BinArgs &a, cudaStream_t s)
