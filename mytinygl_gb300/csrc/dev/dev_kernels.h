@@ -42,6 +42,11 @@ struct GeomArgs {
                                       // by the count launch)
     int32_t sms;
     uint32_t *debug;                  // status word of the debug bounds checks
+    // order-free set-up
+    uint32_t *rec_total;              // records made (device; zeroed by the vertex launch)
+    uint32_t *rec_seq;                // per record: its place in the submission order
+    uint32_t *zero;                   // words the vertex launch clears, beside list_counts and rec_total
+    uint32_t zero_words;              // (0: none of them)
 };
 
 // K1: per-vertex stage (gl_api.c:263-348) for every vertex slot of the pass.
@@ -50,6 +55,10 @@ int launch_vertex(const GeomArgs &a, cudaStream_t s);
 // (raster.c:451-529, 729-1017, 1199-1231); count pass then emit pass.
 int launch_setup_count(const GeomArgs &a, cudaStream_t s);
 int launch_setup_emit(const GeomArgs &a, cudaStream_t s);
+// K2 of an order-free pass with record capacity: one pass, records in any order with their place
+// in rec_seq. Without clip_sorted straddling triangles are clipped in the same launch.
+int launch_setup_free(const GeomArgs &a, cudaStream_t s);
+constexpr uint32_t kInlineClipTris = 16384;  // passes up to this many triangles do so
 
 // Every launcher returns the number of kernels it launched.
 
@@ -60,7 +69,7 @@ int launch_setup_emit(const GeomArgs &a, cudaStream_t s);
 size_t scan_temp_words(uint32_t n);
 // With `host` (two page-locked words) the launch also writes *rec_total and the total there.
 int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
-                cudaStream_t s, const uint32_t *rec_total = nullptr, uint32_t *host = nullptr);
+                cudaStream_t s, const uint32_t *rec_total = nullptr, uint32_t *host = nullptr, bool temp_zeroed = false);
 
 // Element counts of the binning stage live on the device (written by the scans), so the
 // stage runs without the host knowing them. `nrec` / `npairs` on the host are capacities:
@@ -87,6 +96,7 @@ struct BinArgs {
     uint32_t *total_dev;        // where the pair scan writes its total: the pairs generated
     uint32_t *totals_host;      // page-locked words that get the record and pair totals (may be null)
     uint32_t *sort_total_dev;   // a word the sort's histogram scans may overwrite
+    int32_t scan_zeroed;        // scan_temp is zero already
     int32_t order_free;         // tile lists need no order (k_tile_free.cu)
     uint32_t npairs;            // pair capacity of keys/vals (writes beyond are dropped)
     int32_t sms;                // SMs of the device (grid sizes)
@@ -118,6 +128,7 @@ constexpr size_t kOrderAuxWords = 512;
 struct TileArgs {
     const float *records;
     const float *eye_records;
+    const uint32_t *rec_seq;     // order-free passes: a record's place in the submission order (null: its index)
     const uint32_t *tile_vals;   // record indices sorted by tile, submission order within a tile
     const uint32_t *tile_start;  // per tile
     const uint32_t *tile_count;

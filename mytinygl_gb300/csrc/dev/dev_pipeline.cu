@@ -363,13 +363,14 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
         const Pass &p = *frames[f].pass;
         const mtgl_dev *d = frames[f].dev;
         uint8_t *data = ds + frames[f].data_off;
-        bool occlude = !p.draws.empty(), one_func = true;
+        bool occlude = !p.draws.empty(), triangles = true;
+        uint32_t frame_rule = 0;
         for (const PendingDraw &pd : p.draws) {
             DevDraw dd = pd.d;
             if (dd.mode < GL_TRIANGLES || dd.mode > GL_POLYGON || dd.raster >= p.rasters.size() ||
                 p.rasters[dd.raster].rs.polygon_mode_front != GL_FILL ||
                 p.rasters[dd.raster].rs.polygon_mode_back != GL_FILL)
-                defer = occlude = false;  // points and lines read the stored colour
+                defer = occlude = triangles = false;  // points and lines read the stored colour
             if (pd.off_pos >= 0) dd.pos.ptr = data + pd.off_pos;
             if (pd.off_color >= 0) dd.color.ptr = data + pd.off_color;
             if (pd.off_tex >= 0) dd.tex.ptr = data + pd.off_tex;
@@ -396,14 +397,22 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
                 defer = false;  // a fragment reads the stored colour, or may be discarded after its depth test
             // A frame's hidden pairs may be dropped when every fragment that passes its depth test
             // replaces colour and depth, and only nearer (or equal) fragments pass.
-            const uint32_t need = FC_DEPTH | FC_DEPTH_WRITE | FC_MASK_ALL;
-            if ((c & (need | FC_STENCIL | FC_BLEND)) != need || ((c & FC_ALPHA) && (c & FC_TEXTURE)) ||
-                (R.rs.depth_func != GL_LESS && R.rs.depth_func != GL_LEQUAL) || !R.depth_rejection)
-                occlude = false;
-            one_func = one_func && R.rs.depth_func == p.rasters[0].rs.depth_func;
+            // It renders order-free when its draws agree on what decides: the nearest fragment, by one
+            // depth function, or the last (k_tile_free.cu).
+            const bool replaces = (c & (FC_MASK_ALL | FC_STENCIL | FC_BLEND)) == FC_MASK_ALL &&
+                                  !((c & FC_ALPHA) && (c & FC_TEXTURE));
+            uint32_t rule = 0;  // GL_LESS, GL_LEQUAL, or last with (3) or without (4) a depth write
+            if (replaces && (c & FC_DEPTH) && (c & FC_DEPTH_WRITE) && R.depth_rejection &&
+                (R.rs.depth_func == GL_LESS || R.rs.depth_func == GL_LEQUAL))
+                rule = R.rs.depth_func == GL_LESS ? 1 : 2;
+            else if (replaces && (!(c & FC_DEPTH) || R.rs.depth_func == GL_ALWAYS))
+                rule = (c & FC_DEPTH_WRITE) ? 3 : 4;
+            if (rule != 1 && rule != 2) occlude = false;
+            if (i == 0) frame_rule = rule;
+            else if (rule != frame_rule) frame_rule = 0;
             hrs[rsb + i] = R;
         }
-        order_free = order_free && (p.draws.empty() || (occlude && one_func));
+        order_free = order_free && (p.draws.empty() || (triangles && frame_rule));
         if (!p.clears.empty()) memcpy(hcl + clb, p.clears.data(), p.clears.size() * sizeof(ClearOp));
         DevFrame F;
         memset(&F, 0, sizeof(F));
@@ -430,7 +439,7 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
     t.ndraws = (uint32_t)ndraws;
     t.nrasters = (uint32_t)nrs;
     t.defer = defer && ndraws > 0;
-    t.order_free = order_free;
+    t.order_free = order_free && tris < (1ull << 28);  // 16 places per primitive
     t.nclears = (uint32_t)ncl;
     t.slots = (uint32_t)slots;
     t.tris = (uint32_t)tris;
@@ -474,13 +483,26 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     uint32_t *radix_hist = nullptr;
     if ((rc = sc.take(S_VERTS, 3 * (size_t)slots, &verts))) return rc;
     if (eye && (rc = sc.take(S_EYES, slots, &eyes))) return rc;
-    if ((rc = sc.take(S_TRI_COUNTS, tris, &tri_counts))) return rc;
-    if ((rc = sc.take(S_TRI_OFFSETS, tris, &tri_offsets))) return rc;
+    // order-free set-up (capacity mode): no counts, no scan, no emit list
+    const bool free_setup = t.order_free && !c.exact && c.rec_cap && slots;
+    const bool inline_clip = free_setup && tris <= kInlineClipTris;
+    uint32_t *rec_seq = nullptr;
+    if (!free_setup) {
+        if ((rc = sc.take(S_TRI_COUNTS, tris, &tri_counts))) return rc;
+        if ((rc = sc.take(S_TRI_OFFSETS, tris, &tri_offsets))) return rc;
+    } else if ((rc = sc.take(S_REC_SEQ, c.rec_cap, &rec_seq))) {
+        return rc;
+    }
     // clip list, its class words, the class-sorted list, the class counters and the emit list
     uint32_t *clip_list = nullptr;
-    if ((rc = sc.take(S_CLIP_LIST, 4 * (size_t)tris + kClipBuckets, &clip_list))) return rc;
-    // tile counts, then the occlusion bounds
-    if ((rc = sc.take(S_TILE_COUNT, 2 * ((size_t)ntiles + 1), &tile_count))) return rc;
+    if (!inline_clip && (rc = sc.take(S_CLIP_LIST, (free_setup ? 3 : 4) * (size_t)tris + kClipBuckets, &clip_list)))
+        return rc;
+    // tile counts, then the occlusion bounds; an order-free set-up's vertex launch clears both, and
+    // behind them the clip class counters and the tile scan's temporaries
+    const size_t tile_words = 2 * ((size_t)ntiles + 1), class_words = free_setup && !inline_clip ? kClipBuckets : 0;
+    const size_t scan_at = (tile_words + class_words + 1) & ~(size_t)1;  // 8-byte aligned
+    const size_t zero_words = free_setup ? scan_at + scan_temp_words(ntiles) : 0;
+    if ((rc = sc.take(S_TILE_COUNT, std::max(tile_words, zero_words), &tile_count))) return rc;
     uint32_t *tile_near = t.occlude ? tile_count + ntiles + 1 : nullptr;
     if ((rc = sc.take(S_TILE_START, (size_t)ntiles + 1, &tile_start))) return rc;
     uint32_t *tile_frame = nullptr;  // batches: each tile's frame, found once by the range pass
@@ -525,24 +547,31 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ga.total_tris = tris;
     ga.tri_counts = tri_counts;
     ga.tri_offsets = tri_offsets;
-    ga.clip_list = clip_list;
-    ga.clip_class = clip_list + tris;
-    // sort by class below 2^24 triangles: a bucket then holds under 2^20 entries (its blocks
-    // are every kClipSlots-th of 128 triangles), so a rank fits the class word's 20 bits
-    ga.clip_sorted = tris < (1u << 24) ? clip_list + 2 * (size_t)tris : nullptr;
-    ga.class_count = clip_list + 3 * (size_t)tris;
-    ga.emit_list = clip_list + 3 * (size_t)tris + kClipBuckets;
+    if (!inline_clip) {
+        ga.clip_list = clip_list;
+        ga.clip_class = clip_list + tris;
+        // sort by class below 2^24 triangles: a bucket then holds under 2^20 entries (its blocks
+        // are every kClipSlots-th of 128 triangles), so a rank fits the class word's 20 bits
+        ga.clip_sorted = tris < (1u << 24) ? clip_list + 2 * (size_t)tris : nullptr;
+        ga.class_count = free_setup ? tile_count + tile_words : clip_list + 3 * (size_t)tris;
+        ga.emit_list = clip_list + 3 * (size_t)tris + kClipBuckets;
+    }
     ga.list_counts = x.d_totals + 4;
     ga.debug = x.d_totals + kDebugStatusWord;
     ga.sms = x.sms;
+    ga.rec_total = x.d_totals + 0;
+    ga.rec_seq = rec_seq;
+    ga.zero = tile_count;
+    ga.zero_words = (uint32_t)zero_words;
     int launches = 0;
     launches += launch_vertex(ga, s);
     x.prof_mark();
-    launches += launch_setup_count(ga, s);
-    launches += launch_scan(tri_counts, tri_offsets, tris, scan_temp, x.d_totals + 0, x.d_totals + kDebugStatusWord, s);
-    CK(cudaGetLastError());
-
     uint32_t rec_cap = c.rec_cap;
+    if (!free_setup) {
+        launches += launch_setup_count(ga, s);
+        launches += launch_scan(tri_counts, tri_offsets, tris, scan_temp, x.d_totals + 0, x.d_totals + kDebugStatusWord, s);
+    }
+    CK(cudaGetLastError());
     if (c.exact) {
         CK(cudaMemcpyAsync(x.h_totals, x.d_totals, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
@@ -558,11 +587,12 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ga.records = records;
     ga.eye_records = eye_records;
     ga.records_cap = rec_cap;
-    launches += launch_setup_emit(ga, s);
+    launches += free_setup ? launch_setup_free(ga, s) : launch_setup_emit(ga, s);
     x.prof_mark();
 
     // ---- binning
-    CK(cudaMemsetAsync(tile_count, 0, (tile_near ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
+    if (!free_setup)
+        CK(cudaMemsetAsync(tile_count, 0, (tile_near ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     // (an order-free pass's scan writes every tile's start)
     if (!t.order_free || !rec_cap) CK(cudaMemsetAsync(tile_start, 0, ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     BinArgs ba;
@@ -584,7 +614,8 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ba.totals_host = c.exact ? nullptr : x.h_totals;
     ba.debug = x.d_totals + kDebugStatusWord;
     ba.order_free = t.order_free ? 1 : 0;
-    ba.scan_temp = scan_temp;
+    ba.scan_temp = free_setup ? tile_count + scan_at : scan_temp;
+    ba.scan_zeroed = free_setup ? 1 : 0;
     ba.sms = x.sms;
     uint32_t pair_cap = c.pair_cap;
     ba.units = bin_units(rec_cap, x.sms, &ba.wpg);
@@ -627,6 +658,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     memset(&ta, 0, sizeof(ta));
     ta.records = records;
     ta.eye_records = eye_records;
+    ta.rec_seq = rec_seq;
     ta.tile_vals = rec_cap ? ba.vals : nullptr;
     ta.debug = x.d_totals + kDebugStatusWord;
     ta.records_cap = rec_cap;

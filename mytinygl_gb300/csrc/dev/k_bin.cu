@@ -155,7 +155,7 @@ size_t scan_temp_words(uint32_t n)
 }
 
 int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
-                cudaStream_t s, const uint32_t *rec_total, uint32_t *host)
+                cudaStream_t s, const uint32_t *rec_total, uint32_t *host, bool temp_zeroed)
 {
     if (n == 0) {
         cudaMemsetAsync(total_dev, 0, sizeof(uint32_t), s);
@@ -166,7 +166,7 @@ int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, u
     // neither tickets nor statuses (and so no clearing)
     uint64_t *status = reinterpret_cast<uint64_t *>(temp);
     uint32_t *ticket = temp + 2 * (size_t)nb;
-    if (nb > 1) cudaMemsetAsync(temp, 0, (2 * (size_t)nb + 1) * sizeof(uint32_t), s);
+    if (nb > 1 && !temp_zeroed) cudaMemsetAsync(temp, 0, (2 * (size_t)nb + 1) * sizeof(uint32_t), s);
     k_scan<<<nb, kScanThreads, 0, s>>>(in, out, n, status, ticket, total_dev, debug, rec_total, host);
     return 1;
 }
@@ -530,7 +530,8 @@ int launch_bin_count(const BinArgs &a, cudaStream_t s)
                               launch_scan(a.rec_tiles, a.rec_tiles, a.units, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev,
                                           a.totals_host);
     return occlude + launch_records<PASS_COUNT_FREE>(a, s) +
-           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev, a.totals_host);
+           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev, a.totals_host,
+                       a.scan_zeroed != 0);
 }
 
 int launch_bin_expand(const BinArgs &a, cudaStream_t s)

@@ -92,6 +92,10 @@ __global__ void __launch_bounds__(128) k_vertex(GeomArgs A)
     static_assert(sizeof(mtgl_vertex_state) % 4 == 0 && alignof(mtgl_vertex_state) == 4, "copied as 32-bit words");
     __shared__ uint32_t s_vs[sizeof(mtgl_vertex_state) / 4];
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
+    // the later stages' counters, cleared here instead of by memsets of their own
+    for (uint32_t i = g; i < A.zero_words; i += gridDim.x * blockDim.x) A.zero[i] = 0u;
+    if (A.zero_words && g < 2) A.list_counts[g] = 0u;
+    if (A.zero_words && g == 2) *A.rec_total = 0u;
     const bool live = g < A.total_slots;
     int d = 0;
     uint32_t k = 0, vsi = 0;
@@ -1275,10 +1279,186 @@ __global__ void __launch_bounds__(256) k_clip_sort(GeomArgs A)
     }
 }
 
+// ------------------------------------------------------------------ K2 of order-free passes
+//
+// Where records need no order (k_tile_free.cu) set-up counts nothing first: records take the
+// next free slots as they are made, and carry their place in the submission order
+// (rec_seq: 16 * primitive + fan triangle) for the one use it has, ties of equal depths. One
+// pass over the triangles instead of two and a scan: the vertices are read once and straddling
+// triangles are clipped once.
+
+// The record slots [base, base + n) of this thread's triangle.
+__device__ __forceinline__ RecOut slots_of(const GeomArgs &A, bool eye, uint32_t base)
+{
+    return RecOut{A.records, eye ? A.eye_records : nullptr, base, A.records_cap};
+}
+__device__ __forceinline__ void put_seq(const GeomArgs &A, uint32_t at, uint32_t t, uint32_t fan)
+{
+    if (at < A.records_cap) A.rec_seq[at] = 16u * t + min(fan, 15u);
+}
+
+// A warp's allocation of n slots per lane; every lane calls.
+__device__ __forceinline__ uint32_t take_slots(const GeomArgs &A, uint32_t n)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if ((int)lane >= o) incl += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    uint32_t base = 0;
+    if (lane == 0 && total) base = atomicAdd(A.rec_total, total);
+    return __shfl_sync(0xffffffffu, base, 0) + incl - n;
+}
+
+// Clips, divides and fans the straddling triangle t (listed false: no triangle), with its
+// records' slots taken by the whole warp at once; every lane calls.
+template <bool EYE>
+__device__ __forceinline__ void clip_emit(const GeomArgs &A, bool listed, uint32_t t)
+{
+    using V = CVx<EYE>;
+    V buf[kClipMax];
+    int nv = 0;
+    Prim<EYE> P;
+    uint32_t n = 0;
+    if (listed) {
+        P = prim_of<EYE>(A, t);
+        uint32_t e0, e1, e2;
+        element_triple(P.D->mode, P.k, e0, e1, e2);
+        V v0, v1, v2;
+        load_cv(A, element_slot(*P.D, e0), v0);
+        load_cv(A, element_slot(*P.D, e1), v1);
+        load_cv(A, element_slot(*P.D, e2), v2);
+        const int start = clip_start(inside_mask(v0.clip), inside_mask(v1.clip), inside_mask(v2.clip));
+        if (start < kClipNone) {
+            nv = clip_one_plane(v0, v1, v2, start, buf[0], buf[1], buf[2], buf[3]);
+            if (!nv) {
+                V other[kClipMax];
+                buf[0] = v0;
+                buf[1] = v1;
+                buf[2] = v2;
+                nv = clip_triangle(buf, other, start);
+            }
+        }
+        for (int j = 0; j < nv; j++) persp_divide(buf[j]);
+        for (int j = 1; j + 1 < nv; j++) {
+            TriBox tb;
+            n += tri_box(P.R->rs, P.dims, buf[0].clip, buf[j].clip, buf[j + 1].clip, tb) == kTriFill ? 1u : 0u;
+        }
+    }
+    const uint32_t base = take_slots(A, n);
+    if (!n) return;
+    const RecOut o = slots_of(A, EYE, base);
+    uint32_t made = 0;
+    for (int j = 1; j + 1 < nv; j++) {
+        const uint32_t one = setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, buf[0], buf[j], buf[j + 1], o, made);
+        if (one) put_seq(A, base + made, t, (uint32_t)j - 1u);
+        made += one;
+    }
+}
+
+// One thread per triangle decides (positions alone); the block's triangles that make a record
+// are then packed to its first threads, which write them; straddling ones are packed the same
+// way and clipped in place (INLINE_CLIP: passes of few triangles, where two more launches cost
+// more than idle lanes) or listed for k_clip_free.
+template <bool EYE, bool INLINE_CLIP>
+__global__ void __launch_bounds__(128) k_setup_free(GeomArgs A)
+{
+    constexpr uint32_t kB = 128, kWarps = kB / 32;
+    __shared__ uint32_t s_list[2][kB];               // records, straddling triangles
+    __shared__ uint32_t s_n[2][kWarps], s_base[2];   // per warp, then where the block's entries go
+    const uint32_t t = blockIdx.x * kB + threadIdx.x;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
+    bool make = false, straddles = false;
+    uint32_t cls = 0;
+    if (t < A.total_tris) {
+        const Prim<EYE> P = prim_of<EYE>(A, t);
+        uint32_t e0, e1, e2;
+        element_triple(P.D->mode, P.k, e0, e1, e2);
+        ClipPos v0{A.verts.clip[element_slot(*P.D, e0)]}, v1{A.verts.clip[element_slot(*P.D, e1)]},
+            v2{A.verts.clip[element_slot(*P.D, e2)]};
+        const uint32_t m0 = inside_mask(v0.clip), m1 = inside_mask(v1.clip), m2 = inside_mask(v2.clip);
+        const int start = clip_start(m0, m1, m2);
+        if (start == kClipNone) {
+            persp_divide(v0);
+            persp_divide(v1);
+            persp_divide(v2);
+            TriBox tb;
+            make = tri_box(P.R->rs, P.dims, v0.clip, v1.clip, v2.clip, tb) == kTriFill;
+        } else if (start != kClipEmpty) {
+            straddles = true;
+            cls = clip_class(m0, m1, m2, start);
+        }
+    }
+    const uint32_t makes = __ballot_sync(0xffffffffu, make), want = __ballot_sync(0xffffffffu, straddles);
+    if (lane == 0) {
+        s_n[0][warp] = (uint32_t)__popc(makes);
+        s_n[1][warp] = (uint32_t)__popc(want);
+    }
+    __syncthreads();
+    uint32_t n[2] = {0, 0}, before[2] = {0, 0};
+    for (uint32_t w = 0; w < kWarps; w++)
+        for (int l = 0; l < 2; l++) {
+            if (w < warp) before[l] += s_n[l][w];
+            n[l] += s_n[l][w];
+        }
+    if (make) s_list[0][before[0] + (uint32_t)__popc(makes & below)] = t;
+    if (INLINE_CLIP && straddles) s_list[1][before[1] + (uint32_t)__popc(want & below)] = t;
+    if (threadIdx.x == 0) s_base[0] = n[0] ? atomicAdd(A.rec_total, n[0]) : 0u;
+    if (!INLINE_CLIP && threadIdx.x == 32) s_base[1] = n[1] ? atomicAdd(A.list_counts, n[1]) : 0u;
+    __syncthreads();
+    if (threadIdx.x < n[0]) {
+        using V = CVx<EYE>;
+        const uint32_t u = s_list[0][threadIdx.x], at = s_base[0] + threadIdx.x;
+        const Prim<EYE> P = prim_of<EYE>(A, u);
+        uint32_t e0, e1, e2;
+        element_triple(P.D->mode, P.k, e0, e1, e2);
+        V v0, v1, v2;
+        load_cv(A, element_slot(*P.D, e0), v0);
+        load_cv(A, element_slot(*P.D, e1), v1);
+        load_cv(A, element_slot(*P.D, e2), v2);
+        persp_divide(v0);
+        persp_divide(v1);
+        persp_divide(v2);
+        if (setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, v0, v1, v2, slots_of(A, EYE, at), 0)) put_seq(A, at, u, 0);
+    }
+    if (INLINE_CLIP) {
+        if (warp * 32 < n[1]) clip_emit<EYE>(A, threadIdx.x < n[1], threadIdx.x < n[1] ? s_list[1][threadIdx.x] : 0u);
+    } else if (want) {
+        // the clip list, grouped later by class (k_clip_sort)
+        const uint32_t bucket = cls * kClipSlots + (blockIdx.x & (kClipSlots - 1));
+        const uint32_t peers = __match_any_sync(0xffffffffu, straddles ? bucket : 0xFFFFFFFFu);
+        const int leader = __ffs(peers) - 1;
+        uint32_t rb = 0;
+        if (straddles && (int)lane == leader) rb = atomicAdd(A.class_count + bucket, (uint32_t)__popc(peers));
+        rb = __shfl_sync(0xffffffffu, rb, leader);
+        const uint32_t slot = s_base[1] + before[1] + (uint32_t)__popc(want & below);
+        if (straddles && slot < A.total_tris) {
+            A.clip_list[slot] = t;
+            A.clip_class[slot] = (bucket << 20) | (rb + (uint32_t)__popc(peers & below));
+        }
+    }
+}
+
+// the listed triangles (grid capped as k_clip's)
+template <bool EYE>
+__global__ void __launch_bounds__(64) k_clip_free(GeomArgs A)
+{
+    const uint32_t n = min(A.list_counts[0], A.total_tris);
+    for (uint32_t i0 = (blockIdx.x * 64u + threadIdx.x) & ~31u; i0 < n; i0 += gridDim.x * 64u) {
+        const uint32_t i = i0 + (threadIdx.x & 31u);
+        clip_emit<EYE>(A, i < n, i < n ? A.clip_sorted[i] : 0u);
+    }
+}
+
 int launch_vertex(const GeomArgs &a, cudaStream_t s)
 {
     if (!a.total_slots) return 0;
-    k_vertex<<<(a.total_slots + 127) / 128, 128, 0, s>>>(a);
+    // a block per 128 vertices; a few vertices over many tiles take more, for the words to clear
+    const uint32_t clear = std::min<uint32_t>((a.zero_words + 1023) / 1024, 4u * (uint32_t)std::max(1, a.sms));
+    k_vertex<<<std::max((a.total_slots + 127) / 128, clear), 128, 0, s>>>(a);
     return 1;
 }
 
@@ -1308,6 +1488,23 @@ int launch_setup(const GeomArgs &a, cudaStream_t s)
 }
 
 }  // namespace
+
+int launch_setup_free(const GeomArgs &a, cudaStream_t s)
+{
+    if (!a.total_tris) return 0;
+    const unsigned g = (a.total_tris + 127) / 128;
+    if (!a.clip_sorted) {
+        if (a.eyes) k_setup_free<true, true><<<g, 128, 0, s>>>(a);
+        else k_setup_free<false, true><<<g, 128, 0, s>>>(a);
+        return 1;
+    }
+    if (a.eyes) k_setup_free<true, false><<<g, 128, 0, s>>>(a);
+    else k_setup_free<false, false><<<g, 128, 0, s>>>(a);
+    k_clip_sort<<<clip_grid(a), 256, 0, s>>>(a);
+    if (a.eyes) k_clip_free<true><<<clip_grid(a), 64, 0, s>>>(a);
+    else k_clip_free<false><<<clip_grid(a), 64, 0, s>>>(a);
+    return 3;
+}
 
 int launch_setup_count(const GeomArgs &a, cudaStream_t s)
 {

@@ -4,9 +4,10 @@
 // (or GL_LEQUAL, one function per frame), has no stencil test, blending or discards and writes
 // all four channels, a pixel ends with the depth and colour of its nearest fragment: of equal
 // depths the first in submission order under GL_LESS, the last under GL_LEQUAL. That is the
-// smallest (depth, record index) pair (or the largest index), whatever order the fragments are
-// taken in, so binning neither sorts nor orders the tile lists, records may be skipped on any
-// sound bound, and the colour stages run once per pixel.
+// smallest (depth, place) pair (or the largest place), whatever order the fragments are taken
+// in, so set-up and binning order nothing, records may be skipped on any sound bound, and the
+// colour stages run once per pixel. Frames without a depth test (or with GL_ALWAYS) end with
+// the last fragment: the largest place alone.
 //
 // One CTA per tile, one thread per pixel, one warp per 8x4 block. The tile's records are staged
 // 64 at a time into shared memory with asynchronous copies, the next chunk in flight while one
@@ -29,12 +30,13 @@ namespace {
 constexpr int kStage = 64;         // records staged at a time
 constexpr int kStageWords = 9;     // 16-byte words per staged record: 7 used, stride free of bank conflicts
 // record words in stage order: q0 q1 q2 q3 q12 q13 q14, then the record index
-enum StageWord { SW_Q0, SW_Q1, SW_Q2, SW_Q3, SW_Q12, SW_Q13, SW_Q14, SW_INDEX };
+enum StageWord { SW_Q0, SW_Q1, SW_Q2, SW_Q3, SW_Q12, SW_Q13, SW_Q14, SW_INDEX };  // SW_INDEX: index, place + 1
 constexpr int kPerRecordMax = 6;   // records of a step taken one by one; more go by masks
 
 struct Nearest {
     float dep;     // the pixel's depth
-    uint32_t rec;  // 1 + the record that holds it, 0: none
+    uint32_t rec;  // the record that holds it
+    uint32_t seq;  // 1 + its place in the submission order, 0: none holds it
 };
 
 // One fragment: the reference's depth at the pixel, kept when it is the nearer.
@@ -48,17 +50,21 @@ __device__ __forceinline__ bool take_fragment(const TileArgs &A, const float4 *q
     const float z = b0 * q3.x + b1 * q3.y + b2 * q3.z;
     float depth = (z + 1.0f) * 0.5f;
     const uint32_t flags = __float_as_uint(q12.x), idx = __float_as_uint(q[SW_INDEX].x);
-    if (!((flags >> kRecCtlShift) & FC_DEFAULT_RANGE)) {
+    const uint32_t seq = __float_as_uint(q[SW_INDEX].y), ctl = flags >> kRecCtlShift;
+    if (!(ctl & FC_DEFAULT_RANGE)) {
         const uint32_t rs = __float_as_uint(__ldg(A.records + (size_t)idx * kRecWords + R_RASTER));
         const DevRaster &R = A.rasters[min(rs, A.nrasters - 1)];
         depth = map_depth_range(depth, R.rs.depth_near, R.rs.depth_far);
     }
-    const bool less = ((flags >> kRecDepthFuncShift) & 7u) == GL_LESS - GL_NEVER;
-    const bool tie = less ? idx + 1u < n.rec : idx + 1u > n.rec;
-    const bool pass = depth < n.dep || (depth == n.dep && tie);
+    const uint32_t func = (flags >> kRecDepthFuncShift) & 7u;  // a mask, see cmp_pass
+    const bool later = seq > n.seq;
+    bool pass = later;  // no depth test, or one that always passes
+    if ((ctl & FC_DEPTH) && func != 7u)
+        pass = depth < n.dep || (depth == n.dep && (func == 1u ? seq < n.seq : later));
     if (pass) {
-        n.dep = depth;
-        n.rec = idx + 1u;
+        if (ctl & FC_DEPTH_WRITE) n.dep = depth;
+        n.rec = idx;
+        n.seq = seq;
     }
     return pass;
 }
@@ -127,14 +133,16 @@ __global__ void __launch_bounds__(TS *TS, free_min_blocks<TS>()) k_tile_free(Til
                 const uint32_t from = part < 2 ? 2 * part : 8 + 2 * part;  // words 0 1 | 2 3 | 12 13 | 14
                 cp_async16(d + 2 * part, q + from);
                 if (part < 3) cp_async16(d + 2 * part + 1, q + from + 1);
-                else d[SW_INDEX].x = __uint_as_float(idx);
+                else
+                    *reinterpret_cast<uint2 *>(d + SW_INDEX) =
+                        make_uint2(idx, (A.rec_seq ? __ldg(A.rec_seq + idx) : idx) + 1u);
             }
         };
         if (count) stage(0, 0);
         cp_async_commit();
 
         const TilePixel t = open_tile<TS>(A, F, tile, false);
-        Nearest n{t.dep, 0u};
+        Nearest n{t.dep, 0u, 0u};
         uint32_t col = t.col;
         const float fpx = (float)t.px(), fpy = (float)t.py();
         // no fragment beyond this depth changes a pixel of the block: the largest stored depth, or
@@ -188,7 +196,7 @@ __global__ void __launch_bounds__(TS *TS, free_min_blocks<TS>()) k_tile_free(Til
                 }
             }
         }
-        if (n.rec) col = pending_color<TEX, EYE>(A, n.rec - 1u, EYE && A.eye_records != nullptr, fpx, fpy);
+        if (n.seq) col = pending_color<TEX, EYE>(A, n.rec, EYE && A.eye_records != nullptr, fpx, fpy);
         close_tile(A, F, t, col, n.dep, t.st);
     }
     if (A.fragments) {

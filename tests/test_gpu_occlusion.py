@@ -183,3 +183,40 @@ def test_hidden_pairs_in_a_batch(gpu, tile_size):
     batch.destroy()
     for c in ctxs:
         c.destroy()
+
+
+@pytest.mark.parametrize("rule", ["no_depth", "no_depth_then_depth", "always", "always_no_write", "equal_ties"])
+def test_last_fragment_wins_without_a_depth_order(gpu, oracle, rule):
+    """Frames decided by submission order alone (no depth test, or one that always passes), and
+    coplanar layers decided by it: records are made in any order, the frame is the oracle's."""
+    from mytinygl_gb300.scene import render
+
+    for w, h in SIZES:
+        rng = np.random.default_rng([w, h, 77])
+        s = Scene(f"{rule}_{w}x{h}", w, h)
+        s.glViewport(0, 0, w, h)
+        s.glClear(G.GL_COLOR_BUFFER_BIT | G.GL_DEPTH_BUFFER_BIT | G.GL_STENCIL_BUFFER_BIT)
+        for a in (G.GL_VERTEX_ARRAY, G.GL_COLOR_ARRAY):
+            s.glEnableClientState(a)
+        if not rule.startswith("no_depth"):
+            s.glEnable(G.GL_DEPTH_TEST)
+        s.glDepthFunc({"equal_ties": G.GL_LEQUAL}.get(rule, G.GL_ALWAYS if "always" in rule else G.GL_LESS))
+        if rule == "always_no_write":
+            s.glDepthMask(0)
+        _layer(s, rng, 300, -1.2, 1.2, 1.5, slope=0.0 if rule == "equal_ties" else 0.4)
+        _quads(s, rng, [0.3, 0.3])
+        _layer(s, rng, 300, 0.3, 0.3, 1.5, slope=0.0)
+        if rule == "no_depth_then_depth":
+            s.glEnable(G.GL_DEPTH_TEST)
+            _layer(s, rng, 50, -0.9, 0.9, 1.5)
+        harness.assert_parity(harness.compare(render(oracle, s), render(gpu, s)), color_tol=1, name=s.name)
+
+
+@pytest.mark.parametrize("ntri", [1, 31, 16384, 16385, 40000])
+def test_straddling_triangles_at_the_clip_launch_boundary(gpu, oracle, ntri):
+    """Passes up to 16384 triangles clip in the set-up launch, larger ones in their own."""
+    from mytinygl_gb300 import workloads as W
+    from mytinygl_gb300.scene import render
+
+    s = W.textured_scene(96, 64, ntri=ntri, seed=ntri, tex_size=16, spread=1.2)
+    harness.assert_parity(harness.compare(render(oracle, s), render(gpu, s)), color_tol=1, name=s.name)
