@@ -184,8 +184,9 @@ int run_clears_only(mtgl_dev *d)
 }
 
 // Capacities of a pass's records and pairs: the largest totals the context has seen, or for its
-// first passes an estimate: 9/8 records per filled triangle, 25/8 for polygon modes drawn as
-// points or lines; four pairs per record, and at least 2^18 (a few megabytes) unless the frame
+// first passes an estimate: a record per filled triangle, three for polygon modes drawn as
+// points or lines, as many again in small passes for what clipping splits (sprites across the
+// screen's edge made up to 1.6 times their triangles) and an eighth in large ones; four pairs per record, and at least 2^18 (a few megabytes) unless the frame
 // cannot have that many. Totals beyond them cost one more run of the pass (mtgl_dev_settle).
 // A pass of more than 2^22 primitives, whose records may be gigabytes of which few are
 // needed, takes exact sizes instead: its two waits are nothing beside it.
@@ -198,8 +199,9 @@ PipeConfig capacities(const mtgl_dev *d, const Tables &t)
         const mtgl_raster_state &rs = P.rasters[pd.d.raster].rs;
         const bool fill = pd.d.mode < GL_TRIANGLES ||
                           (rs.polygon_mode_front == GL_FILL && rs.polygon_mode_back == GL_FILL);
-        recs += (uint64_t)pd.d.tri_count * (fill ? 1u : 3u) + pd.d.tri_count / 8;  // clipping splits some
+        recs += (uint64_t)pd.d.tri_count * (fill ? 1u : 3u);
     }
+    recs += std::max<uint64_t>(P.tris / 8, std::min<uint64_t>(P.tris, 1u << 16));  // clipping splits some
     recs = std::max<uint64_t>(recs, d->x.rec_seen);
     uint64_t pairs = std::max<uint64_t>(std::max<uint64_t>(4 * recs, d->x.pair_seen), 1u << 18);
     pairs = std::min<uint64_t>(pairs, recs * std::max<uint32_t>(t.ntiles, 1u));
