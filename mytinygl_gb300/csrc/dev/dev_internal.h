@@ -156,11 +156,21 @@ struct Exec {
 
 // One frame of a pass: a context's framebuffer and pending pass, whose staged client data
 // lies at data_off in the staging area being built.
+// host: where the tile kernel also writes the frame (page-locked; device addresses, or null).
+struct HostFrame {
+    uint32_t *color = nullptr;
+    float *depth = nullptr;
+    uint8_t *stencil = nullptr;
+};
 struct FrameSrc {
     mtgl_dev *dev;
     const Pass *pass;
     int64_t data_off;
+    HostFrame host;
 };
+// The device address of [p, p + bytes) when both ends lie in page-locked host memory mapped
+// into the device's address space and p is 4-byte aligned, else null.
+void *mapped_host(void *p, size_t bytes);
 
 // The tables of a pass inside the staging area (offsets are the same in the host copy and
 // in the device copy).

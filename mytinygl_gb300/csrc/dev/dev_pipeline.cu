@@ -17,6 +17,20 @@ int fail_cuda(const char *what, cudaError_t e)
     return MTGL_ERR_CUDA;
 }
 
+void *mapped_host(void *p, size_t bytes)
+{
+    cudaPointerAttributes a, z;
+    if (!p || !bytes || ((uintptr_t)p & 3u) != 0) return nullptr;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || a.type != cudaMemoryTypeHost || !a.devicePointer ||
+        cudaPointerGetAttributes(&z, static_cast<char *>(p) + bytes - 1) != cudaSuccess ||
+        z.type != cudaMemoryTypeHost ||
+        z.devicePointer != static_cast<void *>(static_cast<char *>(a.devicePointer) + bytes - 1)) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return a.devicePointer;
+}
+
 // ------------------------------------------------------------------ host staging
 
 // ------------------------------------------------------------------ run marks
@@ -419,6 +433,9 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
         F.color = d->color;
         F.depth = d->depth;
         F.stencil = d->stencil;
+        F.host_color = frames[f].host.color;
+        F.host_depth = frames[f].host.depth;
+        F.host_stencil = frames[f].host.stencil;
         F.dims.width = d->width;
         F.dims.height = d->height;
         F.dims.tiles_x = (d->width + ts - 1) / ts;

@@ -212,13 +212,13 @@ PipeConfig capacities(const mtgl_dev *d, const Tables &t)
     return c;
 }
 
-int flush_pass(mtgl_dev *d)
+int flush_pass(mtgl_dev *d, const HostFrame &host = HostFrame())
 {
     int st = mtgl_dev_enter(d);
     if (st) return st;
     Pass &P = d->pass;
     if (P.draws.empty()) return run_clears_only(d);
-    FrameSrc fs{d, &P, 0};
+    FrameSrc fs{d, &P, 0, host};
     Tables t;
     if ((st = build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, true, t))) return st;
     const PipeConfig c = capacities(d, t);
@@ -732,13 +732,21 @@ int mtgl_dev_in_batch(const mtgl_dev *d) { return d && (d->batch || !d->readers.
 int mtgl_dev_read(mtgl_dev *d, uint32_t *color, float *depth, uint8_t *stencil)
 {
     if (!d) return MTGL_ERR_INVALID;
-    int st = mtgl_dev_finish(d);
-    if (st) return st;
+    CK(cudaSetDevice(d->device));
     const size_t n = (size_t)d->width * (size_t)d->height;
+    // The pass that is still queued writes page-locked destinations from its tile launch.
+    HostFrame host;
+    if (!d->pass.draws.empty()) {
+        host.color = (uint32_t *)mapped_host(color, n * 4);
+        host.depth = (float *)mapped_host(depth, n * 4);
+        host.stencil = (uint8_t *)mapped_host(stencil, n);
+    }
+    int st = flush_pass(d, host);
+    if (st || (st = mtgl_dev_settle(d))) return st;
     cudaStream_t s = d->x.stream;
-    if (color) CK(cudaMemcpyAsync(color, d->color, n * 4, cudaMemcpyDeviceToHost, s));
-    if (depth) CK(cudaMemcpyAsync(depth, d->depth, n * 4, cudaMemcpyDeviceToHost, s));
-    if (stencil) CK(cudaMemcpyAsync(stencil, d->stencil, n, cudaMemcpyDeviceToHost, s));
+    if (color && !host.color) CK(cudaMemcpyAsync(color, d->color, n * 4, cudaMemcpyDeviceToHost, s));
+    if (depth && !host.depth) CK(cudaMemcpyAsync(depth, d->depth, n * 4, cudaMemcpyDeviceToHost, s));
+    if (stencil && !host.stencil) CK(cudaMemcpyAsync(stencil, d->stencil, n, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     return MTGL_OK;
 }
@@ -940,7 +948,7 @@ int flush_pass_noalloc(mtgl_dev *d)
     cv.cap = kNoAllocScratchBytes;
     const size_t used0 = d->stage.used;
     const size_t marks0 = d->x.ev_pending.size();
-    FrameSrc fs{d, &P, 0};
+    FrameSrc fs{d, &P, 0, HostFrame()};
     Tables t;
     d->stage.fixed = true;  // tables go into the staging areas the context already holds
     st = build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, false, t);

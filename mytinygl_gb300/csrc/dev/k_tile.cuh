@@ -106,7 +106,7 @@ __device__ __forceinline__ TilePixel open_tile(const TileArgs &A, const DevFrame
     const ClearOp *clears = A.clears + F.clear_base;
     const int nclears = (int)F.nclears;
     const int bx0 = tx * TS, by0 = ty * TS, bx1 = min(bx0 + TS, W), by1 = min(by0 + TS, H);
-    bool load_c = true, load_d = true, load_s = stencil;
+    bool load_c = true, load_d = true, load_s = stencil || F.host_stencil;
     uint32_t cleared = 0;
     for (int i = 0; i < nclears; i++) {
         const ClearOp &c = clears[i];
@@ -146,6 +146,15 @@ __device__ __forceinline__ void close_tile(const TileArgs &A, const DevFrame &F,
     F.color[pix] = col;
     F.depth[pix] = dep;
     if (t.store_stencil) F.stencil[pix] = (uint8_t)st;
+    if (F.host_color) F.host_color[pix] = col;
+    if (F.host_depth) F.host_depth[pix] = dep;
+    if (F.host_stencil) F.host_stencil[pix] = (uint8_t)st;
+}
+
+// A tile without records or clears has nothing to do, unless its frame is read back.
+__device__ __forceinline__ bool idle_tile(const DevFrame &F, uint32_t count)
+{
+    return count == 0 && F.nclears == 0 && !F.host_color && !F.host_depth && !F.host_stencil;
 }
 
 // ------------------------------------------------------------------ coverage of a block
@@ -561,7 +570,7 @@ __global__ void __launch_bounds__(TS *TS, tile_min_blocks<TS>()) k_tile(TileArgs
         const uint32_t tile = A.order ? A.order[it] : it;
         const uint32_t count = A.tile_count[tile], start = A.tile_start[tile];
         const DevFrame &F = A.frames[A.tile_frame ? A.tile_frame[tile] : 0u];
-        if (count == 0 && F.nclears == 0) continue;
+        if (idle_tile(F, count)) continue;
         if (!debug_check(A.debug, (uint64_t)start + count <= A.entries_cap, DBG_TILE_ENTRY)) continue;
         if (it != blockIdx.x) __syncthreads();  // the previous tile's records are done with
 

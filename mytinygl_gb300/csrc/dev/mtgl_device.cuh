@@ -254,6 +254,11 @@ struct DevFrame {
     uint32_t *color;
     float *depth;
     uint8_t *stencil;
+    // page-locked host buffers the tile kernel also writes (device addresses; null: none): the
+    // frame's read-back goes over the link while later tiles render
+    uint32_t *host_color;
+    float *host_depth;
+    uint8_t *host_stencil;
     FrameDims dims;
     uint32_t tile_base;
     uint32_t clear_base, nclears;
