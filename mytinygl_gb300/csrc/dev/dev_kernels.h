@@ -43,7 +43,8 @@ struct GeomArgs {
     int32_t sms;
     uint32_t *debug;                  // status word of the debug bounds checks
     // order-free set-up
-    uint32_t *rec_total;              // records made (device; zeroed by the vertex launch)
+    uint32_t *rec_total;              // records made, then the word of the pair total (device; both
+                                      // zeroed by the vertex launch)
     uint32_t *rec_seq;                // per record: its place in the submission order
     uint32_t *zero;                   // words the vertex launch clears, beside list_counts and rec_total
     uint32_t zero_words;              // (0: none of them)
@@ -82,7 +83,7 @@ struct BinArgs {
     uint32_t nframes;
     int32_t tile_shift;         // tile edge = 1 << tile_shift
     uint32_t ntiles;            // tiles of all frames
-    uint32_t units, wpg;        // bin_units(nrec): work units of the record kernels, and units per 32 records
+    uint32_t units;             // bin_units(nrec): work units of the record kernels
     uint32_t *rec_tiles;        // per unit its pair count, then the exclusive scan (in place)
     uint32_t *keys, *vals;      // pair buffers (capacity >= pairs)
     uint32_t *keys_alt, *vals_alt;
@@ -104,11 +105,11 @@ struct BinArgs {
 };
 
 // The count launch also takes the occlusion bounds first (where tile_near is given).
-// Ordered passes: pairs per unit, scanned, and the pair total. Order-free passes: pairs per tile
-// in tile_count, their scan in tile_start, and the total; the expand launch then writes each
-// tile's list at tile_start and leaves the list's end there.
+// Ordered passes: pairs per unit, scanned, and the pair total. Order-free passes: the pairs (tile
+// in keys, record in vals_alt, rank in keys_alt), pairs per tile in tile_count and their scan in
+// tile_start, and the total (*total_dev zero at launch); the expand launch then writes the lists.
 int launch_bin_count(const BinArgs &a, cudaStream_t s);
-uint32_t bin_units(uint32_t nrec, int sms, uint32_t *wpg);  // at most nrec + 31
+uint32_t bin_units(uint32_t nrec, int sms);  // at most nrec + 31
 int launch_bin_expand(const BinArgs &a, cudaStream_t s);
 // Stable sort of (tile, record) pairs by tile; result in keys/vals. Uses keys_alt/vals_alt
 // as ping-pong storage.
@@ -152,7 +153,7 @@ struct TileArgs {
     int32_t defer;               // every record is a filled triangle with deferrable colour (k_tile.cuh)
     uint32_t *debug;             // status word of the debug bounds checks
     uint32_t entries_cap;        // entries tile_vals holds (debug bounds checks)
-    int32_t order_free;          // the pass renders order-free: tile_start holds each list's end
+    int32_t order_free;          // the pass renders order-free (k_tile_free.cu)
 };
 
 // K4: per tile the clears, then its triangles through the full fragment pipeline

@@ -500,7 +500,8 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     uint32_t *radix_hist = nullptr;
     if ((rc = sc.take(S_VERTS, 3 * (size_t)slots, &verts))) return rc;
     if (eye && (rc = sc.take(S_EYES, slots, &eyes))) return rc;
-    // order-free set-up (capacity mode): no counts, no scan, no emit list
+    // order-free passes (capacity mode): no set-up counts, no scan of them, no emit list, no sort;
+    // with exact sizes the pass runs in order, which gives the same frame
     const bool free_setup = t.order_free && !c.exact && c.rec_cap && slots;
     const bool inline_clip = free_setup && tris <= kInlineClipTris;
     uint32_t *rec_seq = nullptr;
@@ -532,12 +533,12 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         scan_n = std::max<uint32_t>(scan_n, (uint32_t)radix_hist_words(c.pair_cap));
         if ((rc = sc.take(S_RECORDS, (size_t)c.rec_cap * kRecWords, &records))) return rc;
         if (eye && (rc = sc.take(S_EYE_RECORDS, (size_t)c.rec_cap * kEyeWords, &eye_records))) return rc;
+        if ((rc = sc.take(S_KEYS, c.pair_cap, &keys))) return rc;
         if ((rc = sc.take(S_VALS, c.pair_cap, &vals))) return rc;
-        if (!t.order_free) {
-            if ((rc = sc.take(S_REC_TILES, bin_units(c.rec_cap, x.sms, nullptr), &rec_tiles))) return rc;
-            if ((rc = sc.take(S_KEYS, c.pair_cap, &keys))) return rc;
-            if ((rc = sc.take(S_KEYS_ALT, c.pair_cap, &keys_alt))) return rc;
-            if ((rc = sc.take(S_VALS_ALT, c.pair_cap, &vals_alt))) return rc;
+        if ((rc = sc.take(S_KEYS_ALT, c.pair_cap, &keys_alt))) return rc;
+        if ((rc = sc.take(S_VALS_ALT, c.pair_cap, &vals_alt))) return rc;
+        if (!free_setup) {
+            if ((rc = sc.take(S_REC_TILES, bin_units(c.rec_cap, x.sms), &rec_tiles))) return rc;
             if ((rc = sc.take(S_RADIX_HIST, radix_hist_words(c.pair_cap), &radix_hist))) return rc;
         }
     }
@@ -595,7 +596,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         rec_cap = o.nrec = x.h_totals[0];
         if ((rc = sc.take(S_RECORDS, (size_t)rec_cap * kRecWords, &records))) return rc;
         if (eye && (rc = sc.take(S_EYE_RECORDS, (size_t)rec_cap * kEyeWords, &eye_records))) return rc;
-        if (!t.order_free && (rc = sc.take(S_REC_TILES, bin_units(rec_cap, x.sms, nullptr), &rec_tiles))) return rc;
+        if ((rc = sc.take(S_REC_TILES, bin_units(rec_cap, x.sms), &rec_tiles))) return rc;
         if (rec_cap > scan_n) {
             scan_n = rec_cap;
             if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(scan_n), &scan_temp))) return rc;
@@ -611,7 +612,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     if (!free_setup)
         CK(cudaMemsetAsync(tile_count, 0, (tile_near ? 2 : 1) * ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     // (an order-free pass's scan writes every tile's start)
-    if (!t.order_free || !rec_cap) CK(cudaMemsetAsync(tile_start, 0, ((size_t)ntiles + 1) * sizeof(uint32_t), s));
+    if (!free_setup) CK(cudaMemsetAsync(tile_start, 0, ((size_t)ntiles + 1) * sizeof(uint32_t), s));
     BinArgs ba;
     memset(&ba, 0, sizeof(ba));
     ba.records = records;
@@ -630,38 +631,40 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ba.sort_total_dev = x.d_totals + 3;
     ba.totals_host = c.exact ? nullptr : x.h_totals;
     ba.debug = x.d_totals + kDebugStatusWord;
-    ba.order_free = t.order_free ? 1 : 0;
+    ba.order_free = free_setup ? 1 : 0;
     ba.scan_temp = free_setup ? tile_count + scan_at : scan_temp;
     ba.scan_zeroed = free_setup ? 1 : 0;
     ba.sms = x.sms;
     uint32_t pair_cap = c.pair_cap;
-    ba.units = bin_units(rec_cap, x.sms, &ba.wpg);
-    if (rec_cap) {
-        launches += launch_bin_count(ba, s);
-        CK(cudaGetLastError());
-        if (c.exact) {
-            CK(cudaMemcpyAsync(x.h_totals + 1, x.d_totals + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            pair_cap = o.npairs = x.h_totals[1];
-            if ((rc = sc.take(S_VALS, pair_cap, &vals))) return rc;
-            if (!t.order_free) {
-                const size_t hist = radix_hist_words(pair_cap);
-                if ((rc = sc.take(S_KEYS, pair_cap, &keys)) || (rc = sc.take(S_KEYS_ALT, pair_cap, &keys_alt)) ||
-                    (rc = sc.take(S_VALS_ALT, pair_cap, &vals_alt)) || (rc = sc.take(S_RADIX_HIST, hist, &radix_hist)))
-                    return rc;
-                const uint32_t need = std::max<uint32_t>(std::max<uint32_t>((uint32_t)hist, rec_cap), scan_n);
-                if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(need), &scan_temp))) return rc;
-                ba.scan_temp = scan_temp;
-            }
-        }
+    ba.units = bin_units(rec_cap, x.sms);
+    auto give_pairs = [&]() {
         ba.keys = keys;
         ba.vals = vals;
         ba.keys_alt = keys_alt;
         ba.vals_alt = vals_alt;
         ba.radix_hist = radix_hist;
         ba.npairs = pair_cap;
+    };
+    if (rec_cap) {
+        if (!c.exact) give_pairs();  // an order-free count launch writes the pairs
+        launches += launch_bin_count(ba, s);
+        CK(cudaGetLastError());
+        if (c.exact) {
+            CK(cudaMemcpyAsync(x.h_totals + 1, x.d_totals + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            pair_cap = o.npairs = x.h_totals[1];
+            const size_t hist = radix_hist_words(pair_cap);
+            if ((rc = sc.take(S_KEYS, pair_cap, &keys)) || (rc = sc.take(S_VALS, pair_cap, &vals)) ||
+                (rc = sc.take(S_KEYS_ALT, pair_cap, &keys_alt)) || (rc = sc.take(S_VALS_ALT, pair_cap, &vals_alt)) ||
+                (rc = sc.take(S_RADIX_HIST, hist, &radix_hist)))
+                return rc;
+            const uint32_t need = std::max<uint32_t>(std::max<uint32_t>((uint32_t)hist, rec_cap), scan_n);
+            if ((rc = sc.take(S_SCAN_TEMP, scan_temp_words(need), &scan_temp))) return rc;
+            ba.scan_temp = scan_temp;
+        }
+        give_pairs();
         launches += launch_bin_expand(ba, s);
-        if (!t.order_free) {
+        if (!free_setup) {
             launches += launch_bin_sort(ba, s);
             launches += launch_tile_ranges(ba, s);
         }
@@ -694,7 +697,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ta.any_stencil = t.any_stencil ? 1 : 0;
     ta.defer = t.defer ? 1 : 0;
     ta.fragments = x.d_frags;
-    ta.order_free = t.order_free && rec_cap ? 1 : 0;
+    ta.order_free = free_setup ? 1 : 0;
     ta.ctas = c.ctas;
     if (order) {
         launches += launch_tile_order(tile_count, ntiles, order_aux, order, x.sms, s);

@@ -178,7 +178,7 @@ int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, u
 // records, each lane sets one up into shared memory (BoxRec), and the warp then runs over the
 // candidates of all 32 in order, 32 at a time, each lane finding its candidate's record in the
 // prefix sums of the tile counts: every lane has a candidate whatever the boxes are. Passes of
-// few records (full-screen quads, sprites) split a group's candidates over A.wpg warps in
+// few records (full-screen quads, sprites) split a group's candidates over several warps in
 // contiguous parts. Both keep submission order: a part's pairs follow the earlier parts'.
 
 constexpr int kRecWarps = 4;  // warps per CTA of the record kernels
@@ -385,72 +385,118 @@ __device__ __forceinline__ void take_bound(const BinArgs &A, const BoxRec &t, in
 }
 
 // The passes over the candidates: occlusion bounds; pairs per unit and the pair writes (ordered
-// passes, sorted by tile afterwards); and, for order-free passes (k_tile_free.cu), pairs per
-// tile and the record indices straight into the tiles' lists, in whatever order they come.
-enum RecPass { PASS_OCCLUDE, PASS_COUNT, PASS_EXPAND, PASS_COUNT_FREE, PASS_EXPAND_FREE };
+// passes, sorted by tile afterwards); and, for order-free passes (k_tile_free.cu), the pairs in
+// one go, in whatever order they come: each takes its rank in its tile's list as it is
+// counted, and k_bin_place moves it there once the tiles' starts are scanned.
+enum RecPass { PASS_OCCLUDE, PASS_COUNT, PASS_EXPAND, PASS_PAIRS };
+
+// PASS_PAIRS: kept pairs collect in shared memory and leave 64 at a time, so that the one
+// counter all warps share and the wait for a rank are paid per 64 pairs, by full warps (of a
+// deep frame's candidates one in fifty is kept).
+constexpr uint32_t kQueueFlush = 64, kQueue = kQueueFlush + 32;
+
+__device__ __forceinline__ void flush_pairs(const BinArgs &A, const uint2 *queue, uint32_t n)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t pos = 0;
+    if (lane == 0) pos = atomicAdd(A.total_dev, n);
+    uint2 q[kQueueFlush / 32];
+    uint32_t rank[kQueueFlush / 32];
+#pragma unroll
+    for (uint32_t k = 0; k < kQueueFlush / 32; k++)
+        if (k * 32 + lane < n) {
+            q[k] = queue[k * 32 + lane];
+            rank[k] = atomicAdd(A.tile_count + q[k].x, 1u);
+        }
+    pos = __shfl_sync(0xffffffffu, pos, 0) + lane;
+#pragma unroll
+    for (uint32_t k = 0; k < kQueueFlush / 32; k++, pos += 32)
+        if (k * 32 + lane < n && pos < A.npairs) {
+            A.keys[pos] = q[k].x;
+            A.vals_alt[pos] = q[k].y;
+            A.keys_alt[pos] = rank[k];
+        }
+}
 
 template <RecPass PASS>
 __global__ void __launch_bounds__(kRecWarps * 32) k_bin_records(BinArgs A)
 {
     __shared__ BoxRec s_box[kRecWarps][32];
+    __shared__ uint32_t s_end[kRecWarps][32];  // inclusive sums of the candidate counts
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
     const uint32_t n = records_in(A);
-    BoxRec *box = s_box[warp];
-    if (PASS == PASS_COUNT_FREE && A.tile_frame)
+    __shared__ uint2 s_queue[PASS == PASS_PAIRS ? kRecWarps : 1][PASS == PASS_PAIRS ? kQueue : 1];  // tile, record
+    uint32_t queued = 0;
+    const BoxRec *box = s_box[warp];
+    const uint32_t *ends = s_end[warp];
+    if (PASS == PASS_PAIRS && A.tile_frame)
         for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.ntiles; t += gridDim.x * blockDim.x)
             A.tile_frame[t] = frame_of_tile(A, t);
+    // the host's units are for the record capacity: fewer records take more warps each
+    uint32_t wpg = 1;
+    while (wpg < 32u && ((n + 31u) / 32u) * wpg * 2u <= A.units) wpg *= 2;
     for (uint32_t u = blockIdx.x * kRecWarps + warp; u < A.units; u += gridDim.x * kRecWarps) {
         // unit u: part u % wpg of the candidates of records [r0, r0 + 32)
-        const uint32_t r0 = u / A.wpg * 32u, part = u % A.wpg;
+        const uint32_t r0 = u / wpg * 32u, part = u % wpg;
         uint32_t kept = 0;
         if (r0 < n) {
             BoxRec b;
             const int cnt = r0 + lane < n ? box_of<PASS == PASS_OCCLUDE>(A, r0 + lane, b) : 0;
-            uint32_t incl = warp_incl_scan((uint32_t)cnt);
+            const uint32_t incl = warp_incl_scan((uint32_t)cnt);
             const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-            if (cnt) box[lane] = b;
+            if (cnt) s_box[warp][lane] = b;
+            s_end[warp][lane] = incl;
             __syncwarp();
-            const uint32_t per = ((total + A.wpg - 1) / A.wpg + 31u) & ~31u;
+            const uint32_t per = ((total + wpg - 1) / wpg + 31u) & ~31u;
             const uint32_t lo = min(part * per, total), hi = min(lo + per, total);
-            uint32_t at = PASS == PASS_EXPAND ? A.rec_tiles[u] : 0u;
+            const uint32_t at = PASS == PASS_EXPAND ? A.rec_tiles[u] : 0u;
+            // the lane's current record and its candidates [first, end): a box of many tiles
+            // serves many steps before the next search
+            uint32_t j = 0, first = 0, end = 0;
             for (uint32_t c0 = lo; c0 < hi; c0 += 32) {
                 const uint32_t c = c0 + lane;
-                // the record: the first lane whose inclusive sum exceeds c
-                uint32_t j = 0;
-#pragma unroll
-                for (uint32_t step = 16; step; step >>= 1)
-                    if (__shfl_sync(0xffffffffu, incl, j + step - 1) <= c) j += step;
-                const uint32_t before = __shfl_sync(0xffffffffu, incl - (uint32_t)cnt, j & 31u);
                 bool get = false;
-                int col = 0, row = 0;
+                uint32_t tile = 0;
                 if (c < hi) {
+                    if (c >= end) {  // the record: the first whose inclusive sum exceeds c
+                        j = 0;
+#pragma unroll
+                        for (uint32_t step = 16; step; step >>= 1)
+                            if (ends[j + step - 1] <= c) j += step;
+                        first = j ? ends[j - 1] : 0u;
+                        end = ends[j];
+                    }
                     const BoxRec &t = box[j];
-                    box_tile(t, (int)(c - before), col, row);
-                    if (PASS == PASS_OCCLUDE) take_bound(A, t, col, row);
-                    else get = tile_gets_pair(A, t, col, row);
+                    int col, row;
+                    box_tile(t, (int)(c - first), col, row);
+                    if (PASS == PASS_OCCLUDE) {
+                        take_bound(A, t, col, row);
+                    } else {
+                        get = tile_gets_pair(A, t, col, row);
+                        tile = t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
+                        get = debug_check(A.debug, tile < A.ntiles, DBG_BIN_TILE) && get;
+                    }
                 }
                 if (PASS == PASS_OCCLUDE) continue;
-                if (PASS == PASS_COUNT_FREE || PASS == PASS_EXPAND_FREE) {
-                    if (!get) continue;
-                    const BoxRec &t = box[j];
-                    const uint32_t tile = t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
-                    if (!debug_check(A.debug, tile < A.ntiles, DBG_BIN_TILE)) continue;
-                    if (PASS == PASS_COUNT_FREE) {
-                        atomicAdd(A.tile_count + tile, 1u);
-                    } else {
-                        const uint32_t pos = atomicAdd(A.tile_start + tile, 1u);
-                        if (pos < A.npairs) A.vals[pos] = r0 + j;
-                    }
-                    continue;
-                }
                 const uint32_t m = __ballot_sync(0xffffffffu, get);
                 if (PASS == PASS_EXPAND && get) {
                     const uint32_t pos = at + kept + (uint32_t)__popc(m & below);
                     if (pos < A.npairs) {
-                        const BoxRec &t = box[j];
-                        const uint32_t tile = t.tile0 + (uint32_t)row * t.tiles_x + (uint32_t)col;
                         A.keys[pos] = tile;
                         A.vals[pos] = r0 + j;
+                    }
+                }
+                if (PASS == PASS_PAIRS && m) {
+                    if (get) s_queue[warp][queued + (uint32_t)__popc(m & below)] = make_uint2(tile, r0 + j);
+                    queued += (uint32_t)__popc(m);
+                    __syncwarp();
+                    if (queued >= kQueueFlush) {
+                        flush_pairs(A, s_queue[warp], kQueueFlush);
+                        queued -= kQueueFlush;
+                        const uint2 rest = s_queue[warp][kQueueFlush + lane];  // fewer than 32
+                        __syncwarp();
+                        if (lane < queued) s_queue[warp][lane] = rest;
+                        __syncwarp();
                     }
                 }
                 kept += (uint32_t)__popc(m);
@@ -459,6 +505,16 @@ __global__ void __launch_bounds__(kRecWarps * 32) k_bin_records(BinArgs A)
         }
         if (PASS == PASS_COUNT && lane == 0) A.rec_tiles[u] = kept;  // units past the records: none
     }
+    if (PASS == PASS_PAIRS && queued) flush_pairs(A, s_queue[warp], queued);
+}
+
+// Order-free passes: each pair's record to its place in its tile's list.
+__global__ void __launch_bounds__(256) k_bin_place(BinArgs A)
+{
+    const uint32_t n = *A.total_dev;
+    if (n > A.npairs) return;  // the tile launch leaves the frames alone then
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        A.vals[__ldg(A.tile_start + A.keys[i]) + A.keys_alt[i]] = A.vals_alt[i];
 }
 
 // grids cover the work or the GPU (16 CTAs per SM), whichever is smaller; kernels loop over the rest
@@ -500,14 +556,13 @@ int launch_tile_ranges(const BinArgs &a, cudaStream_t s)
     return a.npairs ? 2 : 1;
 }
 
-// Warps per group of 32 records: the group count alone fills the GPU (64 warps per SM) from
+// Work units for up to nrec records: the groups of 32 alone fill the GPU (64 warps per SM) from
 // about 300,000 records up; fewer groups split their candidates, up to 32 ways.
-uint32_t bin_units(uint32_t nrec, int sms, uint32_t *wpg)
+uint32_t bin_units(uint32_t nrec, int sms)
 {
     const uint32_t groups = (nrec + 31u) / 32u, warps = (uint32_t)(sms > 0 ? sms : 1) * 64u;
     uint32_t k = 1;
     while (k < 32 && (uint64_t)groups * k < warps) k *= 2;
-    if (wpg) *wpg = k;
     return groups * k;
 }
 
@@ -529,15 +584,17 @@ int launch_bin_count(const BinArgs &a, cudaStream_t s)
     if (!a.order_free) return occlude + launch_records<PASS_COUNT>(a, s) +
                               launch_scan(a.rec_tiles, a.rec_tiles, a.units, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev,
                                           a.totals_host);
-    return occlude + launch_records<PASS_COUNT_FREE>(a, s) +
-           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev, a.totals_host,
-                       a.scan_zeroed != 0);
+    return occlude + launch_records<PASS_PAIRS>(a, s) +
+           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.sort_total_dev, a.debug, s, a.nrec_dev,
+                       a.totals_host, a.scan_zeroed != 0);
 }
 
 int launch_bin_expand(const BinArgs &a, cudaStream_t s)
 {
     if (!a.nrec) return 0;
-    return a.order_free ? launch_records<PASS_EXPAND_FREE>(a, s) : launch_records<PASS_EXPAND>(a, s);
+    if (!a.order_free) return launch_records<PASS_EXPAND>(a, s);
+    k_bin_place<<<stride_grid(std::min<uint32_t>(a.npairs, 1u << 20), 256, a.sms), 256, 0, s>>>(a);
+    return 1;
 }
 
 // ------------------------------------------------------------------ persistent work order

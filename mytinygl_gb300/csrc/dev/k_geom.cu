@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(128) k_vertex(GeomArgs A)
     // the later stages' counters, cleared here instead of by memsets of their own
     for (uint32_t i = g; i < A.zero_words; i += gridDim.x * blockDim.x) A.zero[i] = 0u;
     if (A.zero_words && g < 2) A.list_counts[g] = 0u;
-    if (A.zero_words && g == 2) *A.rec_total = 0u;
+    if (A.zero_words && g >= 2 && g < 4) A.rec_total[g - 2] = 0u;  // and the pair total behind it
     const bool live = g < A.total_slots;
     int d = 0;
     uint32_t k = 0, vsi = 0;

@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(TS *TS, free_min_blocks<TS>()) k_tile_free(Til
     uint32_t frags = 0;
     for (uint32_t it = blockIdx.x; it < A.ntiles; it += gridDim.x) {
         const uint32_t tile = A.order ? A.order[it] : it;
-        const uint32_t count = A.tile_count[tile], start = A.tile_start[tile] - count;  // tile_start: the list's end
+        const uint32_t count = A.tile_count[tile], start = A.tile_start[tile];
         const DevFrame &F = A.frames[A.tile_frame ? A.tile_frame[tile] : 0u];
         if (idle_tile(F, count)) continue;
         if (!debug_check(A.debug, (uint64_t)start + count <= A.entries_cap, DBG_TILE_ENTRY)) continue;
