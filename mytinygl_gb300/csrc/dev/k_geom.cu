@@ -294,15 +294,21 @@ __device__ __forceinline__ int clip_start(uint32_t ma, uint32_t mb, uint32_t mc)
     return ((ma | mb | mc) >> p) & 1u ? p : kClipEmpty;
 }
 
-// The Sutherland-Hodgman pass of plane p over a triangle, in registers, for the common case
-// of a triangle crossing one plane. Writes the pass's output polygon (3 or 4 vertices, in the
-// pass's order) and returns its size; returns 0 when the general clipper must run instead:
-// an intersection the pass drops (|den| <= 1e-10), or an output vertex not inside a later
-// plane (a later pass would change the polygon; a pass whose vertices are all inside copies
-// them unchanged, in order).
+// The first of the planes after p that not all vertices are inside (in: the planes they are all
+// inside), where the next pass must run; 6 if there is none.
+__device__ __forceinline__ int next_pass(uint32_t in, int p)
+{
+    const uint32_t later = kAllInside & ~in & ~((2u << p) - 1u);
+    return later ? __ffs(later) - 1 : 6;
+}
+
+// The Sutherland-Hodgman pass of plane p over a triangle, in registers. Writes the pass's output
+// polygon (3 or 4 vertices, in the pass's order), the planes that all of them are inside
+// (`in`) and returns its size; returns 0 when the pass drops an intersection (|den| <= 1e-10)
+// and clip_rest must run it instead.
 template <class V>
 __device__ __forceinline__ int clip_one_plane(const V &v0, const V &v1, const V &v2, int p, V &o0, V &o1, V &o2,
-                                              V &o3)
+                                              V &o3, uint32_t &in)
 {
     const float d0 = plane_dist(v0.clip, p), d1 = plane_dist(v1.clip, p), d2 = plane_dist(v2.clip, p);
     const bool i0 = d0 >= 0.0f, i1 = d1 >= 0.0f, i2 = d2 >= 0.0f;
@@ -347,10 +353,9 @@ __device__ __forceinline__ int clip_one_plane(const V &v0, const V &v1, const V 
         return 0;
     }
     if (!ok) return 0;
-    uint32_t in = inside_mask(o0.clip) & inside_mask(o1.clip) & inside_mask(o2.clip);
+    in = inside_mask(o0.clip) & inside_mask(o1.clip) & inside_mask(o2.clip);
     if (n == 4) in &= inside_mask(o3.clip);
-    const uint32_t later = kAllInside & ~((2u << p) - 1u);  // the planes after p
-    return (in & later) == later ? n : 0;
+    return n;
 }
 
 // The clip list is processed grouped by these classes, so that a warp's lanes take the same
@@ -364,40 +369,36 @@ __device__ __forceinline__ uint32_t clip_class(uint32_t ma, uint32_t mb, uint32_
     return later + 8u * (uint32_t)p + m;
 }
 
-// clip_triangle (clipping.h:106-126): Sutherland-Hodgman passes from plane `first` on (the
-// earlier ones copy the triangle unchanged, see clip_start); result in bufA[0..n)
+// clip_triangle's (clipping.h:106-126) Sutherland-Hodgman passes over the n vertices of bufA from
+// plane p on, result in bufA. A pass over vertices that are all inside its plane copies them
+// unchanged, in order, so those passes are left out: the buffers are indexed by run-time values,
+// live in local memory, and copying them is what the passes cost.
 template <class V>
-__device__ __noinline__ int clip_triangle(V *bufA, V *bufB, int first)
+__device__ __noinline__ int clip_rest(V *bufA, V *bufB, int n, int p)
 {
-    int n = 3;
     V *in = bufA, *out = bufB;
-    for (int p = first; p < 6; p++) {
+    while (p < 6) {
         int m = 0;
-        const V *prev = &in[n - 1];
-        float pd = plane_dist(prev->clip, p);
+        uint32_t all = kAllInside;
+        auto put = [&](const V &v) {
+            out[m++] = v;
+            all &= inside_mask(v.clip);
+        };
+        V prev = in[n - 1];
+        float pd = plane_dist(prev.clip, p);
         for (int i = 0; i < n; i++) {
-            const V *cur = &in[i];
-            float cd = plane_dist(cur->clip, p);
-            if (pd >= 0) {
-                if (cd >= 0) {
-                    if (m < kClipMax) out[m++] = *cur;
-                } else {
-                    float den = pd - cd;
-                    if (fabsf(den) > 1e-10f && m < kClipMax) {
-                        out[m] = cv_lerp(*prev, *cur, pd / den);
-                        snap_plane(out[m], p);
-                        m++;
-                    }
-                }
-            } else if (cd >= 0) {
-                float den = pd - cd;
+            const V cur = in[i];
+            const float cd = plane_dist(cur.clip, p);
+            const bool pi = pd >= 0, ci = cd >= 0;
+            if (pi != ci) {
+                const float den = pd - cd;
                 if (fabsf(den) > 1e-10f && m < kClipMax) {
-                    out[m] = cv_lerp(*prev, *cur, pd / den);
-                    snap_plane(out[m], p);
-                    m++;
+                    V x = cv_lerp(prev, cur, pd / den);
+                    snap_plane(x, p);
+                    put(x);
                 }
-                if (m < kClipMax) out[m++] = *cur;
             }
+            if (ci && m < kClipMax) put(cur);
             prev = cur;
             pd = cd;
         }
@@ -406,11 +407,30 @@ __device__ __noinline__ int clip_triangle(V *bufA, V *bufB, int first)
         in = out;
         out = tmp;
         if (n == 0) return 0;
+        p = next_pass(all, p);
     }
-    // after six passes the result is in `in`; move it to bufA if needed
     if (in != bufA)
         for (int i = 0; i < n; i++) bufA[i] = in[i];
     return n;
+}
+
+// clip_triangle of a triangle straddling its first plane `start` (clip_start); result in buf.
+template <class V>
+__device__ __forceinline__ int clip_polygon(const V &v0, const V &v1, const V &v2, int start, V *buf, V *other)
+{
+    uint32_t in;
+    int n = clip_one_plane(v0, v1, v2, start, buf[0], buf[1], buf[2], buf[3], in);
+    int p = 6;
+    if (n) {
+        p = next_pass(in, start);
+    } else {
+        buf[0] = v0;
+        buf[1] = v1;
+        buf[2] = v2;
+        n = 3;
+        p = start;
+    }
+    return p < 6 ? clip_rest(buf, other, n, p) : n;
 }
 
 template <class V>
@@ -1156,14 +1176,8 @@ __device__ __forceinline__ uint32_t clip_fan(const DevRaster &R, uint32_t raster
     V bufA[kClipMax];
     int nv = 0;
     if (start < kClipNone) {
-        nv = clip_one_plane(v0, v1, v2, start, bufA[0], bufA[1], bufA[2], bufA[3]);
-        if (!nv) {
-            V bufB[kClipMax];
-            bufA[0] = v0;
-            bufA[1] = v1;
-            bufA[2] = v2;
-            nv = clip_triangle(bufA, bufB, start);
-        }
+        V bufB[kClipMax];
+        nv = clip_polygon(v0, v1, v2, start, bufA, bufB);
     }
     if (nv >= 3) {
         for (int j = 0; j < nv; j++) persp_divide(bufA[j]);
@@ -1183,14 +1197,8 @@ __device__ __forceinline__ uint32_t clip_fan_count(const DevRaster &R, const Fra
     ClipPos bufA[kClipMax];
     int nv = 0;
     if (start < kClipNone) {
-        nv = clip_one_plane(v0, v1, v2, start, bufA[0], bufA[1], bufA[2], bufA[3]);
-        if (!nv) {
-            ClipPos bufB[kClipMax];
-            bufA[0] = v0;
-            bufA[1] = v1;
-            bufA[2] = v2;
-            nv = clip_triangle(bufA, bufB, start);
-        }
+        ClipPos bufB[kClipMax];
+        nv = clip_polygon(v0, v1, v2, start, bufA, bufB);
     }
     uint32_t produced = 0;
     if (nv >= 3) {
@@ -1322,7 +1330,6 @@ __device__ __forceinline__ void clip_emit(const GeomArgs &A, bool listed, uint32
     V buf[kClipMax];
     int nv = 0;
     Prim<EYE> P;
-    uint32_t n = 0;
     if (listed) {
         P = prim_of<EYE>(A, t);
         uint32_t e0, e1, e2;
@@ -1333,29 +1340,32 @@ __device__ __forceinline__ void clip_emit(const GeomArgs &A, bool listed, uint32
         load_cv(A, element_slot(*P.D, e2), v2);
         const int start = clip_start(inside_mask(v0.clip), inside_mask(v1.clip), inside_mask(v2.clip));
         if (start < kClipNone) {
-            nv = clip_one_plane(v0, v1, v2, start, buf[0], buf[1], buf[2], buf[3]);
-            if (!nv) {
-                V other[kClipMax];
-                buf[0] = v0;
-                buf[1] = v1;
-                buf[2] = v2;
-                nv = clip_triangle(buf, other, start);
-            }
-        }
-        for (int j = 0; j < nv; j++) persp_divide(buf[j]);
-        for (int j = 1; j + 1 < nv; j++) {
-            TriBox tb;
-            n += tri_box(P.R->rs, P.dims, buf[0].clip, buf[j].clip, buf[j + 1].clip, tb) == kTriFill ? 1u : 0u;
+            V other[kClipMax];
+            nv = clip_polygon(v0, v1, v2, start, buf, other);
         }
     }
-    const uint32_t base = take_slots(A, n);
-    if (!n) return;
-    const RecOut o = slots_of(A, EYE, base);
-    uint32_t made = 0;
-    for (int j = 1; j + 1 < nv; j++) {
-        const uint32_t one = setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, buf[0], buf[j], buf[j + 1], o, made);
-        if (one) put_seq(A, base + made, t, (uint32_t)j - 1u);
-        made += one;
+    V first;
+    uint32_t fills = 0;  // bit j: the fan triangle (0, j, j + 1) makes a record
+    if (nv >= 3) {
+        first = buf[0];
+        V b = buf[1];
+        persp_divide(first);
+        persp_divide(b);
+        buf[1] = b;
+        for (int j = 1; j + 1 < nv; j++) {
+            V c = buf[j + 1];
+            persp_divide(c);
+            buf[j + 1] = c;
+            TriBox tb;
+            if (tri_box(P.R->rs, P.dims, first.clip, b.clip, c.clip, tb) == kTriFill) fills |= 1u << j;
+            b = c;
+        }
+    }
+    uint32_t at = take_slots(A, (uint32_t)__popc(fills));
+    for (; fills; fills &= fills - 1u, at++) {
+        const int j = __ffs(fills) - 1;
+        if (setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, first, buf[j], buf[j + 1], slots_of(A, EYE, at), 0))
+            put_seq(A, at, t, (uint32_t)j - 1u);
     }
 }
 
@@ -1442,7 +1452,12 @@ __global__ void __launch_bounds__(128) k_setup_free(GeomArgs A)
     }
 }
 
-// the listed triangles (grid capped as k_clip's)
+// The listed triangles (grid capped as k_clip's). Bound by local memory: the buffers' traffic and,
+// in small passes, its latency (a quarter of the issue slots used at 16 warps per SM). Leaving out
+// the passes that copy took the 256-frame batch's 1.4 million straddling triangles from 478 to
+// 372 us, and the 1080p frame of 100,000 triangles from 32 to 25 us. Eight blocks an SM (368 us)
+// hold against 11 (375 us) and 16 (448 us, 64 registers): more buffers than the caches hold. One-plane
+// polygons in registers with the rest apart: 700 us (three triangles' code, most of it idle).
 template <bool EYE>
 __global__ void __launch_bounds__(64) k_clip_free(GeomArgs A)
 {
