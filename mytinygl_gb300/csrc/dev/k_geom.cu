@@ -302,60 +302,47 @@ __device__ __forceinline__ int next_pass(uint32_t in, int p)
     return later ? __ffs(later) - 1 : 6;
 }
 
-// The Sutherland-Hodgman pass of plane p over a triangle, in registers. Writes the pass's output
-// polygon (3 or 4 vertices, in the pass's order), the planes that all of them are inside
-// (`in`) and returns its size; returns 0 when the pass drops an intersection (|den| <= 1e-10)
-// and clip_rest must run it instead.
+// The Sutherland-Hodgman pass of plane p over a triangle with one or two vertices inside it.
+// Writes the pass's output polygon (3 or 4 vertices, in the pass's order) to buf, the planes that
+// all of them are inside to `in`, and returns its size; returns 0 when the pass drops an
+// intersection (|den| <= 1e-10) and clip_rest must run it instead. The three rotations of each
+// case are one code: with a the vertex alone on its side, c -> a -> n, the edges c -> a and
+// a -> n cross, and the rotation only says which vertex the pass writes first.
 template <class V>
-__device__ __forceinline__ int clip_one_plane(const V &v0, const V &v1, const V &v2, int p, V &o0, V &o1, V &o2,
-                                              V &o3, uint32_t &in)
+__device__ __forceinline__ int clip_one_plane(const V &v0, const V &v1, const V &v2, int p, V *buf, uint32_t &in)
 {
     const float d0 = plane_dist(v0.clip, p), d1 = plane_dist(v1.clip, p), d2 = plane_dist(v2.clip, p);
     const bool i0 = d0 >= 0.0f, i1 = d1 >= 0.0f, i2 = d2 >= 0.0f;
-    // the intersection the pass puts on edge a -> b
-    auto cross = [p](const V &a, const V &b, float da, float db, V &out) -> bool {
-        const float den = da - db;
-        if (!(fabsf(den) > 1e-10f)) return false;
-        out = cv_lerp(a, b, da / den);
-        snap_plane(out, p);
-        return true;
-    };
-    bool ok;
-    int n;
-    if (i0 && !i1 && !i2) {         // edges 2->0, 0->1 cross: X20 v0 X01
-        ok = cross(v2, v0, d2, d0, o0) && cross(v0, v1, d0, d1, o2);
-        o1 = v0;
-        n = 3;
-    } else if (!i0 && i1 && !i2) {  // X01 v1 X12
-        ok = cross(v0, v1, d0, d1, o0) && cross(v1, v2, d1, d2, o2);
-        o1 = v1;
-        n = 3;
-    } else if (!i0 && !i1 && i2) {  // X20 X12 v2
-        ok = cross(v2, v0, d2, d0, o0) && cross(v1, v2, d1, d2, o1);
-        o2 = v2;
-        n = 3;
-    } else if (i0 && i1 && !i2) {   // X20 v0 v1 X12
-        ok = cross(v2, v0, d2, d0, o0) && cross(v1, v2, d1, d2, o3);
-        o1 = v0;
-        o2 = v1;
-        n = 4;
-    } else if (!i0 && i1 && i2) {   // X20 X01 v1 v2
-        ok = cross(v2, v0, d2, d0, o0) && cross(v0, v1, d0, d1, o1);
-        o2 = v1;
-        o3 = v2;
-        n = 4;
-    } else if (i0 && !i1 && i2) {   // v0 X01 X12 v2
-        ok = cross(v0, v1, d0, d1, o1) && cross(v1, v2, d1, d2, o2);
-        o0 = v0;
-        o3 = v2;
-        n = 4;
+    const bool two = (int)i0 + (int)i1 + (int)i2 == 2;
+    const int alone = i0 != two ? 0 : (i1 != two ? 1 : 2);
+    const V a = alone == 0 ? v0 : (alone == 1 ? v1 : v2);
+    const V n = alone == 0 ? v1 : (alone == 1 ? v2 : v0);
+    const V c = alone == 0 ? v2 : (alone == 1 ? v0 : v1);
+    const float da = alone == 0 ? d0 : (alone == 1 ? d1 : d2);
+    const float dn = alone == 0 ? d1 : (alone == 1 ? d2 : d0);
+    const float dc = alone == 0 ? d2 : (alone == 1 ? d0 : d1);
+    const float den_ca = dc - da, den_an = da - dn;
+    if (!(fabsf(den_ca) > 1e-10f) || !(fabsf(den_an) > 1e-10f)) return 0;
+    V ca = cv_lerp(c, a, dc / den_ca), an = cv_lerp(a, n, da / den_an);
+    snap_plane(ca, p);
+    snap_plane(an, p);
+    in = inside_mask(ca.clip) & inside_mask(an.clip);
+    // around the polygon: ca a an (a inside), or an n c ca (a outside)
+    const int size = two ? 4 : 3, first = two ? (alone == 2 ? 0 : 3 - alone) : (alone == 2 ? 2 : 0);
+    auto put = [&](int k, const V &v) { buf[k - first + (k < first ? size : 0)] = v; };
+    if (two) {
+        put(0, an);
+        put(1, n);
+        put(2, c);
+        put(3, ca);
+        in &= inside_mask(n.clip) & inside_mask(c.clip);
     } else {
-        return 0;
+        put(0, ca);
+        put(1, a);
+        put(2, an);
+        in &= inside_mask(a.clip);
     }
-    if (!ok) return 0;
-    in = inside_mask(o0.clip) & inside_mask(o1.clip) & inside_mask(o2.clip);
-    if (n == 4) in &= inside_mask(o3.clip);
-    return n;
+    return size;
 }
 
 // The clip list is processed grouped by these classes, so that a warp's lanes take the same
@@ -419,7 +406,7 @@ template <class V>
 __device__ __forceinline__ int clip_polygon(const V &v0, const V &v1, const V &v2, int start, V *buf, V *other)
 {
     uint32_t in;
-    int n = clip_one_plane(v0, v1, v2, start, buf[0], buf[1], buf[2], buf[3], in);
+    int n = clip_one_plane(v0, v1, v2, start, buf, in);
     int p = 6;
     if (n) {
         p = next_pass(in, start);
@@ -1321,63 +1308,73 @@ __device__ __forceinline__ uint32_t take_slots(const GeomArgs &A, uint32_t n)
     return __shfl_sync(0xffffffffu, base, 0) + incl - n;
 }
 
-// Clips, divides and fans the straddling triangle t (listed false: no triangle), with its
-// records' slots taken by the whole warp at once; every lane calls.
+// Clips, divides and fans the triangle t (listed false: no triangle), with its records' slots
+// taken by the whole warp at once; every lane calls.
 template <bool EYE>
 __device__ __forceinline__ void clip_emit(const GeomArgs &A, bool listed, uint32_t t)
 {
     using V = CVx<EYE>;
-    V buf[kClipMax];
-    int nv = 0;
+    V buf[kClipMax];  // a clipped triangle's polygon
+    V v0, v1, v2;     // the triangle, then the fan triangle at hand
     Prim<EYE> P;
+    uint32_t fills = 0;  // bit j: the fan triangle (0, j, j + 1) makes a record
     if (listed) {
         P = prim_of<EYE>(A, t);
         uint32_t e0, e1, e2;
         element_triple(P.D->mode, P.k, e0, e1, e2);
-        V v0, v1, v2;
         load_cv(A, element_slot(*P.D, e0), v0);
         load_cv(A, element_slot(*P.D, e1), v1);
         load_cv(A, element_slot(*P.D, e2), v2);
         const int start = clip_start(inside_mask(v0.clip), inside_mask(v1.clip), inside_mask(v2.clip));
+        int nv = start == kClipNone ? 3 : 0;
         if (start < kClipNone) {
             V other[kClipMax];
             nv = clip_polygon(v0, v1, v2, start, buf, other);
+            v0 = buf[0];
+            v1 = buf[1];
+            v2 = buf[2];
         }
-    }
-    V first;
-    uint32_t fills = 0;  // bit j: the fan triangle (0, j, j + 1) makes a record
-    if (nv >= 3) {
-        first = buf[0];
-        V b = buf[1];
-        persp_divide(first);
-        persp_divide(b);
-        buf[1] = b;
-        for (int j = 1; j + 1 < nv; j++) {
-            V c = buf[j + 1];
-            persp_divide(c);
-            buf[j + 1] = c;
+        if (nv >= 3) {
             TriBox tb;
-            if (tri_box(P.R->rs, P.dims, first.clip, b.clip, c.clip, tb) == kTriFill) fills |= 1u << j;
-            b = c;
+            persp_divide(v0);
+            persp_divide(v1);
+            persp_divide(v2);
+            if (tri_box(P.R->rs, P.dims, v0.clip, v1.clip, v2.clip, tb) == kTriFill) fills = 2u;
+            float4 b = v2.clip;
+            if (nv > 3) buf[2] = v2;
+            for (int j = 2; j + 1 < nv; j++) {
+                V c = buf[j + 1];
+                persp_divide(c);
+                buf[j + 1] = c;
+                if (tri_box(P.R->rs, P.dims, v0.clip, b, c.clip, tb) == kTriFill) fills |= 1u << j;
+                b = c.clip;
+            }
         }
     }
     uint32_t at = take_slots(A, (uint32_t)__popc(fills));
     for (; fills; fills &= fills - 1u, at++) {
         const int j = __ffs(fills) - 1;
-        if (setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, first, buf[j], buf[j + 1], slots_of(A, EYE, at), 0))
+        if (j > 1) {
+            v1 = buf[j];
+            v2 = buf[j + 1];
+        }
+        if (setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, v0, v1, v2, slots_of(A, EYE, at), 0))
             put_seq(A, at, t, (uint32_t)j - 1u);
     }
 }
 
 // One thread per triangle decides (positions alone); the block's triangles that make a record
-// are then packed to its first threads, which write them; straddling ones are packed the same
-// way and clipped in place (INLINE_CLIP: passes of few triangles, where two more launches cost
-// more than idle lanes) or listed for k_clip_free.
+// are then packed to its first threads, which write them; straddling ones are listed for
+// k_clip_free. Passes of few triangles (INLINE_CLIP) clip in place, where two more launches cost
+// more than idle lanes: both kinds go through clip_emit, the kernel's only copy of the record's
+// set-up. A cold kernel of one block waits for its own instructions more than for anything
+// else: with a second copy, and each rotation of the clip written out, 12 triangles took
+// 18.8 us, so 12.9 us.
 template <bool EYE, bool INLINE_CLIP>
 __global__ void __launch_bounds__(128) k_setup_free(GeomArgs A)
 {
     constexpr uint32_t kB = 128, kWarps = kB / 32;
-    __shared__ uint32_t s_list[2][kB];               // records, straddling triangles
+    __shared__ uint32_t s_list[kB];                  // the triangles that make records
     __shared__ uint32_t s_n[2][kWarps], s_base[2];   // per warp, then where the block's entries go
     const uint32_t t = blockIdx.x * kB + threadIdx.x;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, below = (1u << lane) - 1u;
@@ -1414,14 +1411,21 @@ __global__ void __launch_bounds__(128) k_setup_free(GeomArgs A)
             if (w < warp) before[l] += s_n[l][w];
             n[l] += s_n[l][w];
         }
-    if (make) s_list[0][before[0] + (uint32_t)__popc(makes & below)] = t;
-    if (INLINE_CLIP && straddles) s_list[1][before[1] + (uint32_t)__popc(want & below)] = t;
+    if (make) s_list[before[0] + (uint32_t)__popc(makes & below)] = t;
+    if (INLINE_CLIP) {
+        // behind the others, so that few warps have both
+        if (straddles) s_list[n[0] + before[1] + (uint32_t)__popc(want & below)] = t;
+        __syncthreads();
+        const uint32_t both = n[0] + n[1];
+        if (warp * 32 < both) clip_emit<EYE>(A, threadIdx.x < both, threadIdx.x < both ? s_list[threadIdx.x] : 0u);
+        return;
+    }
     if (threadIdx.x == 0) s_base[0] = n[0] ? atomicAdd(A.rec_total, n[0]) : 0u;
-    if (!INLINE_CLIP && threadIdx.x == 32) s_base[1] = n[1] ? atomicAdd(A.list_counts, n[1]) : 0u;
+    if (threadIdx.x == 32) s_base[1] = n[1] ? atomicAdd(A.list_counts, n[1]) : 0u;
     __syncthreads();
     if (threadIdx.x < n[0]) {
         using V = CVx<EYE>;
-        const uint32_t u = s_list[0][threadIdx.x], at = s_base[0] + threadIdx.x;
+        const uint32_t u = s_list[threadIdx.x], at = s_base[0] + threadIdx.x;
         const Prim<EYE> P = prim_of<EYE>(A, u);
         uint32_t e0, e1, e2;
         element_triple(P.D->mode, P.k, e0, e1, e2);
@@ -1434,9 +1438,7 @@ __global__ void __launch_bounds__(128) k_setup_free(GeomArgs A)
         persp_divide(v2);
         if (setup_fan_tri(*P.R, P.D->raster, P.frame, P.dims, v0, v1, v2, slots_of(A, EYE, at), 0)) put_seq(A, at, u, 0);
     }
-    if (INLINE_CLIP) {
-        if (warp * 32 < n[1]) clip_emit<EYE>(A, threadIdx.x < n[1], threadIdx.x < n[1] ? s_list[1][threadIdx.x] : 0u);
-    } else if (want) {
+    if (want) {
         // the clip list, grouped later by class (k_clip_sort)
         const uint32_t bucket = cls * kClipSlots + (blockIdx.x & (kClipSlots - 1));
         const uint32_t peers = __match_any_sync(0xffffffffu, straddles ? bucket : 0xFFFFFFFFu);
@@ -1455,7 +1457,8 @@ __global__ void __launch_bounds__(128) k_setup_free(GeomArgs A)
 // The listed triangles (grid capped as k_clip's). Bound by local memory: the buffers' traffic and,
 // in small passes, its latency (a quarter of the issue slots used at 16 warps per SM). Leaving out
 // the passes that copy took the 256-frame batch's 1.4 million straddling triangles from 478 to
-// 372 us, and the 1080p frame of 100,000 triangles from 32 to 25 us. Eight blocks an SM (368 us)
+// 372 us, and the 1080p frame of 100,000 triangles from 32 to 25 us; one code for the rotations of the
+// one-plane clip, so fewer paths in a warp, to 348 and 22 us. Eight blocks an SM (368 us)
 // hold against 11 (375 us) and 16 (448 us, 64 registers): more buffers than the caches hold. One-plane
 // polygons in registers with the rest apart: 700 us (three triangles' code, most of it idle).
 template <bool EYE>
