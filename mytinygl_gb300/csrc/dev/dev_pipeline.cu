@@ -427,6 +427,9 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
             hrs[rsb + i] = R;
         }
         order_free = order_free && (p.draws.empty() || (triangles && frame_rule));
+        bool whole = true;
+        for (const ClearOp &c : p.clears)
+            whole = whole && c.x0 <= 0 && c.y0 <= 0 && c.x1 >= d->width && c.y1 >= d->height;
         if (!p.clears.empty()) memcpy(hcl + clb, p.clears.data(), p.clears.size() * sizeof(ClearOp));
         DevFrame F;
         memset(&F, 0, sizeof(F));
@@ -442,7 +445,15 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
         F.dims.tiles_y = (d->height + ts - 1) / ts;
         F.tile_base = tile_base;
         F.clear_base = clb;
-        F.nclears = (uint32_t)p.clears.size();
+        F.nclears = whole ? 0u : (uint32_t)p.clears.size();
+        if (whole)
+            for (const ClearOp &c : p.clears) {
+                F.cleared |= c.mask;
+                if (c.mask & GL_COLOR_BUFFER_BIT) F.clear_color = c.color;
+                if (c.mask & GL_DEPTH_BUFFER_BIT) F.clear_depth = c.depth;
+                if (c.mask & GL_STENCIL_BUFFER_BIT) F.clear_stencil = c.stencil & 0xFFu;
+            }
+        F.tiles_x_inv = UINT32_MAX / (uint32_t)F.dims.tiles_x;
         F.occlude = occlude ? 1u : 0u;
         t.occlude = t.occlude || occlude;
         hfr[f] = F;

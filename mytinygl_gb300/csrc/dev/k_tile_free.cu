@@ -110,13 +110,14 @@ __global__ void __launch_bounds__(TS *TS, free_min_blocks<TS>()) k_tile_free(Til
     constexpr int kThreads = TS * TS;
     __shared__ float4 s_rec[2][kStage * kStageWords];
 
-    if (A.guard && (A.guard[0] > A.records_cap || A.guard[1] > A.pairs_cap)) return;
+    const bool over = over_capacity(A);  // waited for with the first tile's words
     const int lane = threadIdx.x & 31;
     uint32_t frags = 0;
     for (uint32_t it = blockIdx.x; it < A.ntiles; it += gridDim.x) {
         const uint32_t tile = A.order ? A.order[it] : it;
         const uint32_t count = A.tile_count[tile], start = A.tile_start[tile];
         const DevFrame &F = A.frames[A.tile_frame ? A.tile_frame[tile] : 0u];
+        if (over) return;
         if (idle_tile(F, count)) continue;
         if (!debug_check(A.debug, (uint64_t)start + count <= A.entries_cap, DBG_TILE_ENTRY)) continue;
         if (it != blockIdx.x) __syncthreads();  // the previous tile's records are done with

@@ -263,7 +263,19 @@ struct DevFrame {
     uint32_t tile_base;
     uint32_t clear_base, nclears;
     uint32_t occlude;  // binning may drop pairs hidden behind a triangle covering their tile (k_bin.cu)
+    // clears of the whole framebuffer, when the frame has no others (nclears is 0 then): the
+    // buffers and the last values
+    uint32_t cleared, clear_color;
+    float clear_depth;
+    uint32_t clear_stencil;
+    uint32_t tiles_x_inv;  // (2^32 - 1) / tiles_x: see tile_row
 };
+// local / tiles_x: the product with tiles_x_inv is at most one too small for local < 2^31
+__device__ __forceinline__ uint32_t tile_row(const DevFrame &F, uint32_t local)
+{
+    const uint32_t n = (uint32_t)F.dims.tiles_x, q = __umulhi(local, F.tiles_x_inv);
+    return local - q * n >= n ? q + 1 : q;
+}
 
 // ------------------------------------------------------------------ scalar helpers
 

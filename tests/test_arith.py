@@ -466,3 +466,16 @@ def test_warp_transpose():
         for i in range(32):
             for j in range(32):
                 assert t[i] >> j & 1 == v[j] >> i & 1
+
+
+def test_tile_row_by_reciprocal():
+    """The tile kernel's row of a tile: the high product with (2^32 - 1) / n, one more when the rest
+    holds another n, for every width in tiles a frame can have."""
+    rng = np.random.default_rng(11)
+    for n in list(range(1, 70)) + [127, 128, 129, 512, 513, 1023, 1024, 1025, 2047, 2048]:
+        rows = rng.integers(0, 2048, 200, dtype=np.uint64)
+        near = (rows[:, None] * n + np.array([0, 1, n - 1], np.uint64)).ravel()
+        local = np.concatenate([near, rng.integers(0, 2048 * n, 500, dtype=np.uint64), [2**31 - 1]]).astype(np.uint64)
+        q = (local * np.uint64(0xFFFFFFFF // n)) >> np.uint64(32)
+        q = np.where(local - q * n >= n, q + 1, q)
+        assert np.array_equal(q, local // n), n
