@@ -109,6 +109,7 @@ __global__ void __launch_bounds__(TS *TS, free_min_blocks<TS>()) k_tile_free(Til
 {
     constexpr int kThreads = TS * TS;
     __shared__ float4 s_rec[2][kStage * kStageWords];
+    __shared__ HostTile<TS> s_out;
 
     const bool over = over_capacity(A);  // waited for with the first tile's words
     const int lane = threadIdx.x & 31;
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(TS *TS, free_min_blocks<TS>()) k_tile_free(Til
             }
         }
         if (n.seq) col = pending_color<TEX, EYE>(A, n.rec, EYE && A.eye_records != nullptr, fpx, fpy);
-        close_tile(A, F, t, col, n.dep, t.st);
+        close_tile<TS>(A, F, t, col, n.dep, t.st, &s_out);
     }
     if (A.fragments) {
         const uint32_t fw = __reduce_add_sync(0xffffffffu, frags);
