@@ -400,12 +400,12 @@ int mtgl_dev_batch_readback(mtgl_batch *b, mtgl_dev *target, uint32_t *host_colo
     if (st) return st;
     // A frame of this run goes to mapped page-locked memory from the tile launch itself, while
     // later tiles render: 256 uneven frames (116 MB) 5.43 -> 5.05 ms, 48 served ones 5.33 -> 4.27
-    // ms. Frames under 2^15 pixels keep the read-back kernel's 16-byte stores: 128 of 64-160
-    // pixels a side measured the same either way (565 and 564 us).
+    // ms, 128 frames of 64-160 pixels a side 558 -> 540 us. Frames under 2^12 pixels, a few tiles
+    // whose stores are short, keep the read-back kernel's 16-byte ones, many frames a launch.
     bool in_tiles = false;
     const size_t pixels = (size_t)target->width * (size_t)target->height;
     for (FrameSrc &f : b->frames)
-        if (f.dev == target && b->cfg.readback_kernel && !f.host.color && pixels >= (1u << 15)) {
+        if (f.dev == target && b->cfg.readback_kernel && !f.host.color && pixels >= (1u << 12)) {
             f.host.color = (uint32_t *)mapped_host(host_color, pixels * 4);
             in_tiles = f.host.color != nullptr;
             break;
