@@ -610,6 +610,12 @@ __device__ __forceinline__ bool clamp_box(const mtgl_raster_state &rs, const Fra
     return x0 <= x1 && y0 <= y1;
 }
 
+// R_FLAGS: the raster state's enables and depth function, which the tile kernel tests by.
+__device__ __forceinline__ uint32_t draw_bits(const DevRaster &R)
+{
+    return ((R.fs.ctl & 0xFFFu) << kRecCtlShift) | (((R.rs.depth_func - GL_NEVER) & 7u) << kRecDepthFuncShift);
+}
+
 __device__ __forceinline__ void rec_header(float4 *r4, int64_t x0, int64_t y0, int64_t x1, int64_t y1,
                                            uint32_t raster_id, uint32_t frame, uint32_t flags)
 {
@@ -625,15 +631,16 @@ __device__ __forceinline__ void rec_header(float4 *r4, int64_t x0, int64_t y0, i
 
 // One point square of final colour c and depth `depth` (the caller applied texture, alpha
 // test and fog). Returns the records produced (0 or 1).
-__device__ __forceinline__ uint32_t point_rec(const mtgl_raster_state &rs, uint32_t raster_id, uint32_t frame,
+__device__ __forceinline__ uint32_t point_rec(const DevRaster &R, uint32_t raster_id, uint32_t frame,
                                               const FrameDims &dims, int64_t x0, int64_t y0, int64_t x1, int64_t y1,
                                               float depth, float4 c, float *rec)
 {
+    const mtgl_raster_state &rs = R.rs;
     if (!clamp_box(rs, dims, x0, y0, x1, y1)) return 0;
     if (rec) {
         float4 *r4 = reinterpret_cast<float4 *>(rec);
         rec_header(r4, x0, y0, x1, y1, raster_id, frame,
-                   ((uint32_t)REC_POINT << kRecTypeShift) | (raises_depth(rs) ? kFlagRaisesDepth : 0u));
+                   ((uint32_t)REC_POINT << kRecTypeShift) | (raises_depth(rs) ? kFlagRaisesDepth : 0u) | draw_bits(R));
         rec[R_Z0] = depth;
         r4[5] = c;
     }
@@ -651,7 +658,7 @@ __device__ __forceinline__ uint32_t screen_point(const DevRaster &R, uint32_t ra
     const float depth = map_depth(R, z);
     if (rs.alpha_test && !cmp_pass(rs.alpha_func, c.w, rs.alpha_ref)) return 0;
     if (rs.fog) c = lerp_rgb(ld4(rs.fog_color), c, fog_factor(rs, -ez));
-    return point_rec(rs, raster_id, frame, dims, x, y, x, y, depth, c, rec);
+    return point_rec(R, raster_id, frame, dims, x, y, x, y, depth, c, rec);
 }
 
 // flush_points' per-vertex part (raster.c:1020-1164): clip-volume test, divide, screen
@@ -680,7 +687,7 @@ __device__ __forceinline__ uint32_t vertex_point(const DevRaster &R, uint32_t ra
     int32_t ps = x86_f2i(rs.point_size + 0.5f);
     if (ps < 1) ps = 1;
     const int64_t xs = (int64_t)cx - ps / 2, ys = (int64_t)cy - ps / 2;
-    return point_rec(rs, raster_id, frame, dims, xs, ys, xs + ps - 1, ys + ps - 1, depth, c, rec);
+    return point_rec(R, raster_id, frame, dims, xs, ys, xs + ps - 1, ys + ps - 1, depth, c, rec);
 }
 
 // draw_line_full's setup (raster.c:107-241): endpoints, width and the interpolants; the tile
@@ -708,7 +715,7 @@ __device__ __forceinline__ uint32_t line_rec(const DevRaster &R, uint32_t raster
     if (rec) {
         float4 *r4 = reinterpret_cast<float4 *>(rec);
         rec_header(r4, bx0, by0, bx1, by1, raster_id, frame,
-                   ((uint32_t)REC_LINE << kRecTypeShift) | (raises_depth(rs) ? kFlagRaisesDepth : 0u));
+                   ((uint32_t)REC_LINE << kRecTypeShift) | (raises_depth(rs) ? kFlagRaisesDepth : 0u) | draw_bits(R));
         r4[0] = make_float4(__int_as_float(x0), __int_as_float(y0), __int_as_float(x1), __int_as_float(y1));
         r4[1].x = __int_as_float(lw);
         rec[R_Z0] = z0;
@@ -955,8 +962,7 @@ __device__ __forceinline__ uint32_t setup_fan_tri(const DevRaster &R, uint32_t r
     // edge_function(a, b, p) = (px - ax) * (by - ay) - (py - ay) * (bx - ax): the per-edge
     // differences are the same floats whether formed per pixel or once here
     const uint32_t flags = (back ? 1u : 0u) | (zc << 1) | (raises_depth(rs) ? kFlagRaisesDepth : 0u) |
-                           ((R.fs.ctl & 0xFFFu) << kRecCtlShift) |
-                           (((rs.depth_func - GL_NEVER) & 7u) << kRecDepthFuncShift);
+                           draw_bits(R);
     r4[12] = make_float4(__uint_as_float(flags), fy2 - fy1, fx2 - fx1, fy0 - fy2);
     r4[13] = make_float4(fx0 - fx2, fy1 - fy0, fx1 - fx0, __uint_as_float(frame));
     r4[14] = (zc == ZC_LESS || zc == ZC_LEQUAL) && R.default_depth_range

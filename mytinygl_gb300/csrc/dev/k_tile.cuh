@@ -408,19 +408,20 @@ struct PixelOut {
     uint32_t flags;  // bit 0: a fragment; bit 1: depth written
 };
 
-// write_line_pixel (raster.c:86-104) and the pixel loop of draw_points (raster.c:1140-1160):
-// depth test, blend with the stored colour, depth write, masked colour write.
-__device__ __forceinline__ PixelOut point_ops(const mtgl_raster_state &rs, float depth, float4 c, uint32_t col,
+// write_line_pixel (raster.c:86-104) and the pixel loop of draw_points (raster.c:1140-1160) past
+// the depth test: blend with the stored colour, depth write, masked colour write. ctl: the
+// record's enables.
+__device__ __forceinline__ PixelOut point_ops(const FragState &S, uint32_t ctl, float depth, float4 c, uint32_t col,
                                               float dep)
 {
     PixelOut o{col, dep, 1u};
-    if (rs.depth_test && !cmp_pass(rs.depth_func, depth, dep)) return o;
-    if (rs.blend) c = blend(rs, c, unpack_rgba(col));
-    if (rs.depth_test && rs.depth_mask) {
+    if (ctl & FC_BLEND) c = blend(__ldg(&S.blend_src), __ldg(&S.blend_dst), c, unpack_rgba(col));
+    if (ctl & FC_DEPTH_WRITE) {
         o.dep = depth;
         o.flags |= 2u;
     }
-    o.col = masked_write(rs, col, c);
+    if (ctl & FC_MASK_ALL) o.col = pack_rgba(c.x, c.y, c.z, c.w);
+    else if (!(ctl & FC_MASK_NONE)) o.col = masked_write(__ldg(&S.color_mask), col, c);
     return o;
 }
 
@@ -475,39 +476,63 @@ static __device__ __noinline__ uint32_t line_mask(const float4 &q0, int lw, int 
     return line_mask_of<int64_t, uint64_t>(x0, y0, x1, y1, lw, wx0, wy0);
 }
 
+// Steps to a line's pixel and in all: along x for an x-major line, else along y.
+template <class I>
+__device__ __forceinline__ void line_step(I x0, I y0, I x1, I y1, int px, int py, int32_t &k, int32_t &total)
+{
+    const I dx = x1 - x0, dy = y1 - y0;
+    const I adx = dx < 0 ? -dx : dx, ady = dy < 0 ? -dy : dy;
+    k = (int32_t)(adx > ady ? (dx < 0 ? x0 - px : px - x0) : (ady > 0 ? (dy < 0 ? y0 - py : py - y0) : 0));
+    total = (int32_t)(adx > ady ? adx : ady);
+}
+
 // One pixel a point or line record covers: with the step's t, its colour, depth, texel and fog.
+// Where many short lines meet (a mesh's pole) a pixel takes hundreds of them one after another, and
+// the latency of this function bounds the launch: the enables and the depth function come with the
+// record, the depth test is first (nothing before it has an effect), and the steps are 32-bit (a
+// wireframe sphere with its points, whole passes: 417 -> 388 us).
 static __device__ __noinline__ PixelOut shade_prim(const TileArgs &A, const float4 *q, int px, int py, uint32_t col,
                                                    float dep)
 {
-    PixelOut none{col, dep, 0u};
-    const float4 q0 = q[0], q3 = q[3], c0 = q[5], q11 = q[11];
-    const DevRaster &R = A.rasters[min(__float_as_uint(q11.w), A.nrasters - 1)];
-    const mtgl_raster_state &rs = R.rs;
-    if (((__float_as_uint(q[12].x) >> kRecTypeShift) & 3u) == REC_POINT) return point_ops(rs, q3.x, c0, col, dep);
-
-    const int64_t x0 = __float_as_int(q0.x), y0 = __float_as_int(q0.y);
-    const int64_t dx = __float_as_int(q0.z) - x0, dy = __float_as_int(q0.w) - y0;
-    const int64_t adx = dx < 0 ? -dx : dx, ady = dy < 0 ? -dy : dy;
-    const int64_t k = adx > ady ? (dx < 0 ? x0 - px : px - x0) : (ady > 0 ? (dy < 0 ? y0 - py : py - y0) : 0);
-    const int32_t total = (int32_t)(adx > ady ? adx : ady);
-    const float t = (float)(int32_t)k / (float)(total == 0 ? 1 : total);
+    const PixelOut none{col, dep, 0u};
+    const float4 q0 = q[0], q3 = q[3];
+    const uint32_t flags = __float_as_uint(q[12].x), ctl = flags >> kRecCtlShift;
+    const uint32_t func = GL_NEVER + ((flags >> kRecDepthFuncShift) & 7u);
+    const DevRaster &R = A.rasters[min(__float_as_uint(q[11].w), A.nrasters - 1)];
+    const FragState &S = R.fs;
+    if (((flags >> kRecTypeShift) & 3u) == REC_POINT) {
+        if ((ctl & FC_DEPTH) && !cmp_pass(func, q3.x, dep)) return none;
+        return point_ops(S, ctl, q3.x, q[5], col, dep);
+    }
+    const int x0 = __float_as_int(q0.x), y0 = __float_as_int(q0.y), x1 = __float_as_int(q0.z), y1 = __float_as_int(q0.w);
+    auto small = [](int v) { return v > -(1 << 29) && v < (1 << 29); };
+    int32_t k, total;
+    if (small(x0) && small(y0) && small(x1) && small(y1)) line_step<int32_t>(x0, y0, x1, y1, px, py, k, total);
+    else line_step<int64_t>(x0, y0, x1, y1, px, py, k, total);
+    const float t = (float)k / (float)(total == 0 ? 1 : total);
     const float z = q3.x + t * (q3.y - q3.x);
-    const float depth = map_depth(R, z);
-    float4 c = lerp_col(c0, q[6], t);
-    if (R.tex) {
+    const float u01 = (z + 1.0f) * 0.5f;
+    const float depth = (ctl & FC_DEFAULT_RANGE) ? u01 : map_depth_range(u01, R.rs.depth_near, R.rs.depth_far);
+    if ((ctl & FC_DEPTH) && !cmp_pass(func, depth, dep)) return none;
+    float4 c = lerp_col(q[5], q[6], t);
+    // the reference never leaves its loop when the alpha test fails (raster.c:175, 183 skip the
+    // Bresenham step); here the pixel is dropped
+    if (ctl & FC_TEXTURE) {
         const float4 q8 = q[8];
         const float u = q8.x + t * (q8.z - q8.x);
         const float v = q8.y + t * (q8.w - q8.y);
-        const float4 tc = sample_lod(R.fs, u, v, 0.0f);
-        // the reference never leaves its loop when this test fails (raster.c:175, 183 skip the
-        // Bresenham step); here the pixel is dropped
-        if (rs.alpha_test && !cmp_pass(rs.alpha_func, tc.w, rs.alpha_ref)) return none;
+        const float4 tc = sample_lod(S, u, v, 0.0f);
+        if ((ctl & FC_ALPHA) && !cmp_pass(__ldg(&S.alpha_func), tc.w, __ldg(&S.alpha_ref))) return none;
         c = make_float4(c.x * tc.x, c.y * tc.y, c.z * tc.z, c.w * tc.w);
-    } else if (rs.alpha_test && !cmp_pass(rs.alpha_func, c.w, rs.alpha_ref)) {
+    } else if ((ctl & FC_ALPHA) && !cmp_pass(__ldg(&S.alpha_func), c.w, __ldg(&S.alpha_ref))) {
         return none;
     }
-    if (rs.fog) c = lerp_rgb(ld4(rs.fog_color), c, fog_factor(rs, -(q11.x + t * (q11.y - q11.x))));
-    return point_ops(rs, depth, c, col, dep);
+    if (ctl & FC_FOG) {
+        const float4 q11 = q[11];
+        c = lerp_rgb(__ldg(reinterpret_cast<const float4 *>(S.fog_color)), c,
+                     fog_factor(S.fog_mode, S.fog_density, S.fog_start, S.fog_end, -(q11.x + t * (q11.y - q11.x))));
+    }
+    return point_ops(S, ctl, depth, c, col, dep);
 }
 
 // ------------------------------------------------------------------ triangles
