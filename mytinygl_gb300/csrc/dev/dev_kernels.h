@@ -91,7 +91,7 @@ struct BinArgs {
     uint32_t *tile_near;        // per tile: the occlusion bound (near_key; zero at launch); null when no
                                 // frame of the pass has one
     uint32_t *tile_start;       // exclusive scan of tile_count
-    uint32_t *tile_frame;       // per tile: the frame owning it (written by the range pass; may be null)
+    uint32_t *tile_frame;       // per tile: the frame owning it, written with the tiles' ranges (null: one frame)
     uint32_t *radix_hist;       // radix histograms
     uint32_t *scan_temp;
     uint32_t *total_dev;        // where the pair scan writes its total: the pairs generated
@@ -133,7 +133,7 @@ struct TileArgs {
     const uint32_t *tile_vals;   // record indices sorted by tile, submission order within a tile
     const uint32_t *tile_start;  // per tile
     const uint32_t *tile_count;
-    const uint32_t *tile_frame;  // per tile: its frame (null: found by a search of the frame table)
+    const uint32_t *tile_frame;  // per tile: its frame (null: the pass has one)
     const DevRaster *rasters;
     uint32_t nrasters;
     const ClearOp *clears;       // all frames' clears; a frame holds its range

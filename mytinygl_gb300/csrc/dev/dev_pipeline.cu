@@ -682,6 +682,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     } else {
         CK(cudaMemsetAsync(x.d_totals + 1, 0, sizeof(uint32_t), s));
         if (!c.exact) CK(cudaMemcpyAsync(x.h_totals, x.d_totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        if (tile_frame) launches += launch_tile_ranges(ba, s);  // frames that only clear: their tiles' frames
     }
     x.prof_mark();
 
@@ -696,7 +697,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ta.entries_cap = rec_cap ? pair_cap : 0u;
     ta.tile_start = tile_start;
     ta.tile_count = tile_count;
-    ta.tile_frame = rec_cap ? tile_frame : nullptr;  // written by the range pass, which runs with records
+    ta.tile_frame = tile_frame;  // written by the range pass, which runs with records
     ta.rasters = ga.rasters;
     ta.nrasters = std::max<uint32_t>(1, t.nrasters);
     ta.clears = reinterpret_cast<const ClearOp *>(ds + t.off_clears);

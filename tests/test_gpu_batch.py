@@ -14,6 +14,7 @@ import pytest
 
 import feature_scenes as F
 import harness
+from mytinygl_gb300 import gl as G
 from mytinygl_gb300 import workloads as W
 from mytinygl_gb300.scene import render
 
@@ -224,6 +225,67 @@ def test_readback_kernel_destinations(gpu):
     assert launches[1] == launches[0] + 1
     for c in ctxs:
         c.destroy()
+
+
+@pytest.mark.parametrize("tile", [8, 16, 32])
+@pytest.mark.parametrize("n", [2, 3, 5])
+def test_frames_that_only_clear(gpu, oracle, tile, n):
+    """A batch in which no frame draws a primitive: every frame takes its clears (of the whole
+    framebuffer, of a part, of one buffer), and is read back, below and above the size from
+    which the tile launch writes read-backs, into page-locked and pageable memory and not at all."""
+    torch = pytest.importorskip("torch")
+    sizes = [(70, 33), (64, 64), (16, 12), (129, 96), (257, 17)][:n]
+    every = G.GL_COLOR_BUFFER_BIT | G.GL_DEPTH_BUFFER_BIT | G.GL_STENCIL_BUFFER_BIT
+
+    def first(c, w, h):
+        c.glViewport(0, 0, w, h)
+        c.glClear(every)
+        c.glBegin(G.GL_TRIANGLES)
+        for x, y in ((-0.9, -0.8), (0.9, -0.7), (0.1, 0.9)):
+            c.glColor3f(0.5 + 0.4 * x, 0.5 - 0.4 * y, 0.25)
+            c.glVertex3f(x, y, 0.3 * x)
+        c.glEnd()
+        c.glFinish()
+
+    def clears(c, i, w, h):
+        c.glClearColor(0.1 + 0.15 * i, 0.8 - 0.1 * i, 0.4, 1.0)
+        c.glClearDepth(0.9 - 0.1 * i)
+        c.glClearStencil(i + 1)
+        if i % 3 == 1:
+            c.glEnable(G.GL_SCISSOR_TEST)
+            c.glScissor(w // 5, h // 4, w // 2, h // 2)
+        c.glClear(G.GL_COLOR_BUFFER_BIT if i % 3 == 2 else every)
+        c.glBegin(G.GL_TRIANGLES)  # no whole triangle
+        c.glVertex2f(0.0, 0.0)
+        c.glEnd()
+
+    want = []
+    for i, (w, h) in enumerate(sizes):
+        c = oracle.context(w, h)
+        first(c, w, h)
+        clears(c, i, w, h)
+        want.append(c.read() + (c.glGetError(),))
+        c.destroy()
+    for reads in ("none", "page-locked", "pageable"):
+        ctxs = [gpu.context(w, h) for w, h in sizes]
+        hosts = None
+        if reads != "none":
+            hosts = [torch.full((h, w), 77, dtype=torch.int32, pin_memory=reads == "page-locked").numpy().view(np.uint32)
+                     for w, h in sizes]
+        for i, (c, (w, h)) in enumerate(zip(ctxs, sizes)):
+            c.make_current()
+            first(c, w, h)
+            clears(c, i, w, h)
+        b = gpu.batch(tile_size=tile)
+        b.render(ctxs, colors=hosts)
+        b.wait()
+        for i, c in enumerate(ctxs):
+            c.make_current()
+            assert hosts is None or np.array_equal(hosts[i], want[i][0]), f"{reads}: read-back of frame {i}"
+            assert_identical([c.read() + (c.glGetError(),)], [want[i]], [f"{reads}: frame {i}"])
+        b.destroy()
+        for c in ctxs:
+            c.destroy()
 
 
 @pytest.mark.slow
