@@ -41,7 +41,7 @@ uint32_t round_capacity(uint64_t v)
     while (p < v) p <<= 1;
     const uint64_t q = std::max<uint64_t>(256, p / 8);
     const uint64_t r = (v + q - 1) / q * q;
-    return (uint32_t)std::min<uint64_t>(r, 0xFFFFFF00ull);
+    return (uint32_t)std::min<uint64_t>(r, kMaxEntries);
 }
 
 }  // namespace

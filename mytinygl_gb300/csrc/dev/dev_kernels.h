@@ -68,9 +68,14 @@ constexpr uint32_t kInlineClipTris = 16384;  // passes up to this many triangles
 // 8-byte aligned; debug is the
 // status word its bounded waits report to (may be null).
 size_t scan_temp_words(uint32_t n);
-// With `host` (two page-locked words) the launch also writes *rec_total and the total there.
+// Sums stay at 2^32 - 1 instead of wrapping. With `host` (two page-locked words) the launch also
+// writes rec_total[0] and [1], the pass's record and pair totals, there.
 int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
                 cudaStream_t s, const uint32_t *rec_total = nullptr, uint32_t *host = nullptr, bool temp_zeroed = false);
+
+// The most records or pairs a pass may make: a larger total is refused (MTGL_ERR_OVERFLOW). Below
+// 2^32 by more than the kernels' strides, so that their 32-bit loops end.
+constexpr uint32_t kMaxEntries = 0xF0000000u;
 
 // Element counts of the binning stage live on the device (written by the scans), so the
 // stage runs without the host knowing them. `nrec` / `npairs` on the host are capacities:

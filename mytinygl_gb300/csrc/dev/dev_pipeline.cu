@@ -17,6 +17,12 @@ int fail_cuda(const char *what, cudaError_t e)
     return MTGL_ERR_CUDA;
 }
 
+static int fail_entries(const char *what)
+{
+    snprintf(g_err, sizeof(g_err), "pass too large (more than %u %s)", kMaxEntries, what);
+    return MTGL_ERR_OVERFLOW;
+}
+
 void *mapped_host(void *p, size_t bytes)
 {
     cudaPointerAttributes a, z;
@@ -605,6 +611,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         CK(cudaMemcpyAsync(x.h_totals, x.d_totals, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         rec_cap = o.nrec = x.h_totals[0];
+        if (rec_cap > kMaxEntries) return fail_entries("records");
         if ((rc = sc.take(S_RECORDS, (size_t)rec_cap * kRecWords, &records))) return rc;
         if (eye && (rc = sc.take(S_EYE_RECORDS, (size_t)rec_cap * kEyeWords, &eye_records))) return rc;
         if ((rc = sc.take(S_REC_TILES, bin_units(rec_cap, x.sms), &rec_tiles))) return rc;
@@ -664,6 +671,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
             CK(cudaMemcpyAsync(x.h_totals + 1, x.d_totals + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
             CK(cudaStreamSynchronize(s));
             pair_cap = o.npairs = x.h_totals[1];
+            if (pair_cap > kMaxEntries) return fail_entries("tile pairs");
             const size_t hist = radix_hist_words(pair_cap);
             if ((rc = sc.take(S_KEYS, pair_cap, &keys)) || (rc = sc.take(S_VALS, pair_cap, &vals)) ||
                 (rc = sc.take(S_KEYS_ALT, pair_cap, &keys_alt)) || (rc = sc.take(S_VALS_ALT, pair_cap, &vals_alt)) ||

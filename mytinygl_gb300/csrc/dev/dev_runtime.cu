@@ -208,7 +208,7 @@ PipeConfig capacities(const mtgl_dev *d, const Tables &t)
     PipeConfig c;
     c.exact = false;
     c.rec_cap = (uint32_t)std::min<uint64_t>(recs, 0x7FFFFF00ull);
-    c.pair_cap = (uint32_t)std::min<uint64_t>(pairs, 0xFFFFFF00ull);
+    c.pair_cap = (uint32_t)std::min<uint64_t>(pairs, kMaxEntries);
     return c;
 }
 
@@ -223,7 +223,13 @@ int flush_pass(mtgl_dev *d, const HostFrame &host = HostFrame())
     if ((st = build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, true, t))) return st;
     const PipeConfig c = capacities(d, t);
     PipeOut o;
-    if ((st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o))) return st;
+    if ((st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o))) {
+        if (st == MTGL_ERR_OVERFLOW) {  // no size renders it: the frame goes without
+            P.reset();
+            d->stage.used = 0;
+        }
+        return st;
+    }
     if ((st = d->stage.mark_uploaded(d->x.stream))) return st;
     if (c.exact) {
         d->stats.setup_triangles += o.nrec;
@@ -273,6 +279,7 @@ int mtgl_dev_settle(mtgl_dev *d)
         PipeConfig c;
         PipeOut o;
         int rc = run_pipeline(d->x, d->x.pool, d->stage, d->ran_t, c, &o);
+        if (rc == MTGL_ERR_OVERFLOW) d->stage.used = 0;
         if (rc || (rc = d->stage.mark_uploaded(d->x.stream)) || (rc = d->stage.wait())) return rc;
         nrec = o.nrec;
         npairs = o.npairs;

@@ -32,22 +32,46 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
     return v;
 }
 
+// Sums that stay at the largest value instead of wrapping, so that a total past 32 bits is seen as
+// one that fits nowhere. (Saturating addition of unsigned numbers is associative: the sum, or
+// the limit.)
+__device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b)
+{
+    const uint32_t s = a + b;
+    return s < a ? 0xFFFFFFFFu : s;
+}
+// saturating scan over the warp: returns the exclusive sum, the inclusive one in *incl
+__device__ __forceinline__ uint32_t warp_sat_scan(uint32_t v, uint32_t *incl)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t n = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = sat_add(v, n);
+    }
+    *incl = v;
+    const uint32_t before = __shfl_up_sync(0xffffffffu, v, 1);
+    return lane ? before : 0u;
+}
+
 // exclusive block scan of one value per thread; returns the block total in *total
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *total)
 {
     __shared__ uint32_t warp_sums[kScanThreads / 32 + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = warp_incl_scan(v);
+    uint32_t incl;
+    const uint32_t before = warp_sat_scan(v, &incl);
     if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = lane < kScanThreads / 32 ? warp_sums[lane] : 0u;
-        uint32_t wi = warp_incl_scan(w);
-        if (lane < kScanThreads / 32) warp_sums[lane] = wi - w;
+        uint32_t wi;
+        const uint32_t wb = warp_sat_scan(lane < kScanThreads / 32 ? warp_sums[lane] : 0u, &wi);
+        __syncwarp();
+        if (lane < kScanThreads / 32) warp_sums[lane] = wb;
         if (lane == kScanThreads / 32 - 1) warp_sums[kScanThreads / 32] = wi;
     }
     __syncthreads();
-    uint32_t r = warp_sums[warp] + incl - v;
+    const uint32_t r = sat_add(warp_sums[warp], before);
     *total = warp_sums[kScanThreads / 32];
     __syncthreads();
     return r;
@@ -89,7 +113,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
     }
     uint32_t sum = 0;
 #pragma unroll
-    for (int i = 0; i < kScanItems; i++) sum += v[i];
+    for (int i = 0; i < kScanItems; i++) sum = sat_add(sum, v[i]);
     uint32_t agg;
     uint32_t run = block_excl_scan(sum, &agg);
     if (threadIdx.x < 32) {
@@ -114,29 +138,33 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
                 // the nearest tile with its inclusive prefix ends the walk; the nearer ones add sums
                 const uint32_t prefixed = __ballot_sync(0xffffffffu, (st >> 32) == 2);
                 const uint32_t upto = prefixed ? (uint32_t)__ffs(prefixed) - 1u : 31u;
-                prefix += __reduce_add_sync(0xffffffffu, lane <= upto ? (uint32_t)st : 0u);
+                // (in halves, whose 32 sums fit)
+                const uint32_t add = lane <= upto ? (uint32_t)st : 0u;
+                const uint32_t lo = __reduce_add_sync(0xffffffffu, add & 0xFFFFu);
+                const uint32_t hi = __reduce_add_sync(0xffffffffu, add >> 16) + (lo >> 16);
+                prefix = sat_add(prefix, hi > 0xFFFFu ? 0xFFFFFFFFu : (hi << 16) | (lo & 0xFFFFu));
                 if (prefixed) break;
             }
-            if (lane == 0) st_status(status + tile, kScanPrefix | (prefix + agg));
+            if (lane == 0) st_status(status + tile, kScanPrefix | sat_add(prefix, agg));
         }
         if (lane == 0) {
             s_prefix = prefix;
             if (tile + 1 == gridDim.x) {
-                *total_dev = prefix + agg;
+                *total_dev = sat_add(prefix, agg);
                 if (host) {  // page-locked: the pass's record and pair totals, without a copy behind it
-                    host[0] = *rec_total;
-                    host[1] = prefix + agg;
+                    host[0] = rec_total[0];
+                    host[1] = rec_total[1];  // an ordered pass's is this scan's
                 }
             }
         }
     }
     __syncthreads();
-    run += s_prefix;
+    run = sat_add(run, s_prefix);
     uint32_t o[kScanItems];
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         o[i] = run;
-        run += v[i];
+        run = sat_add(run, v[i]);
     }
     if (base + kScanItems <= n) {
         *reinterpret_cast<uint4 *>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -399,7 +427,13 @@ __device__ __forceinline__ void flush_pairs(const BinArgs &A, const uint2 *queue
 {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t pos = 0;
-    if (lane == 0) pos = atomicAdd(A.total_dev, n);
+    if (lane == 0) {
+        // Past the capacity the exact total serves nothing, and would wrap: an addition that finds
+        // it exceeded is taken back, so that it stays exceeded and below the capacity (at most
+        // kMaxEntries) and 64 for every resident warp, far from 2^32.
+        pos = atomicAdd(A.total_dev, n);
+        if (pos > A.npairs) atomicSub(A.total_dev, n);
+    }
     uint2 q[kQueueFlush / 32];
     uint32_t rank[kQueueFlush / 32];
 #pragma unroll
@@ -513,8 +547,10 @@ __global__ void __launch_bounds__(256) k_bin_place(BinArgs A)
 {
     const uint32_t n = *A.total_dev;
     if (n > A.npairs) return;  // the tile launch leaves the frames alone then
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        A.vals[__ldg(A.tile_start + A.keys[i]) + A.keys_alt[i]] = A.vals_alt[i];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t at = __ldg(A.tile_start + A.keys[i]) + A.keys_alt[i];
+        if (at < A.npairs) A.vals[at] = A.vals_alt[i];
+    }
 }
 
 // grids cover the work or the GPU (16 CTAs per SM), whichever is smaller; kernels loop over the rest

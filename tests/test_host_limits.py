@@ -1,0 +1,141 @@
+"""What the host does with a pass that fits nowhere or whose memory cannot be had (CPU only: the
+library's host code over stand-ins for the CUDA runtime and the kernel launches)."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import fake_gpu
+from mytinygl_gb300 import gl as G
+
+MTGL_OK, MTGL_ERR_OVERFLOW = 0, 7
+
+
+@pytest.fixture(scope="module")
+def fake():
+    return fake_gpu.load()
+
+
+@pytest.fixture
+def gpu(fake):
+    """(context, controls): a context whose passes make 5 records and 9 pairs."""
+    lib, ctl = fake
+    ctl.fake_alloc_limit(0)
+    ctl.fake_totals(5, 9)
+    ctl.fake_log_clear()
+    ctx = lib.context(64, 48)
+    yield ctx, ctl
+    ctl.fake_alloc_limit(0)
+    ctl.fake_totals(5, 9)
+    ctx.destroy()
+
+
+def draw(ctx, triangles=1, blend=False):
+    (ctx.glEnable if blend else ctx.glDisable)(G.GL_BLEND)
+    ctx.glClear(G.GL_COLOR_BUFFER_BIT)
+    ctx.glBegin(G.GL_TRIANGLES)
+    for k in range(3 * triangles):
+        ctx.glVertex2f(0.1 * (k % 7), 0.1 * (k % 5))
+    ctx.glEnd()
+
+
+def finish(ctx):
+    return ctx.glib.lib.mtgl_finish(ctx.handle)
+
+
+def log(ctl):
+    out = ctl.fake_log().decode().split()
+    ctl.fake_log_clear()
+    return out
+
+
+@pytest.mark.parametrize("blend", [False, True], ids=["order-free", "ordered"])
+def test_totals_past_32_bits_are_refused(gpu, blend):
+    """A total that reached the limit of the saturating sums: the capacity run leaves the frame alone,
+    the exact one is refused, and the context goes on with its next pass."""
+    ctx, ctl = gpu
+    for totals in ((5, 0xFFFFFFFF), (0xFFFFFFFF, 0xFFFFFFFF)):
+        draw(ctx, blend=blend)
+        ctl.fake_totals(*totals)
+        assert finish(ctx) == MTGL_ERR_OVERFLOW
+        assert "tile" not in log(ctl)
+        ctl.fake_totals(5, 9)
+        draw(ctx, blend=blend)
+        assert finish(ctx) == MTGL_OK and log(ctl)[-1] == "tile"
+
+
+def test_a_batch_past_32_bits_is_refused(fake, gpu):
+    ctx, ctl = gpu
+    b = fake[0].batch(use_graph=0)
+    draw(ctx)
+    ctl.fake_totals(5, 0xFFFFFFFF)
+    b.render([ctx])
+    assert fake[0].lib.mtgl_dev_batch_wait(b.handle) == MTGL_ERR_OVERFLOW
+    assert "tile" not in log(ctl)
+    ctl.fake_totals(5, 9)
+    draw(ctx)
+    b.render([ctx])
+    b.wait()
+    assert log(ctl)[-1] == "tile"
+    b.destroy()
+
+
+# ---- the sums that decide it, restated
+
+MASK = 0xFFFFFFFF
+
+
+def sat_add(a, b):
+    s = (a + b) & MASK
+    return MASK if s < a else s
+
+
+def test_saturating_sums():
+    """k_scan's sums: any grouping of saturating additions gives min(sum, 2^32 - 1), and the look-back's
+    sum of 32 words in 16-bit halves does too; below the limit every sum is the plain one."""
+    rng = np.random.default_rng(5)
+    for case in range(300):
+        hi = [10, 1 << 20, 1 << 27, 1 << 32][case % 4]
+        v = [int(x) for x in rng.integers(0, hi, 64)]
+        want = min(sum(v), MASK)
+        left = 0
+        for x in v:
+            left = sat_add(left, x)
+        tree = list(v)
+        while len(tree) > 1:
+            tree = [sat_add(tree[i], tree[i + 1]) for i in range(0, len(tree), 2)]
+        assert left == tree[0] == want
+        total = 0
+        for g in (v[:32], v[32:]):  # two windows of the look-back
+            lo = sum(x & 0xFFFF for x in g)
+            h = sum(x >> 16 for x in g) + (lo >> 16)
+            assert lo <= MASK and h <= MASK
+            total = sat_add(total, MASK if h > 0xFFFF else (h << 16) | (lo & 0xFFFF))
+        assert total == want
+
+
+def test_the_pair_total_stays_past_its_capacity():
+    """flush_pairs' total under any interleaving: warps add 1 to 64 pairs and take an addition back
+    that found the capacity exceeded. Past the capacity it stays past it and never comes near 2^32;
+    within it, it is the plain sum. (16 warps stand for the GPU's: the bound is the capacity plus 64
+    for each.)"""
+    rng = np.random.default_rng(6)
+    for cap, adds in ((100, 5), (100, 4000), (0xF0000000, 4000), (0, 50)):
+        start = max(0, cap - 20_000)  # what earlier warps added, none of it taken back
+        total, plain, most = start, start, 0
+        undo = []  # warps between their addition and its removal
+        left = adds
+        while left or undo:
+            if left and len(undo) < 16 and rng.random() < 0.6:
+                n = int(rng.integers(1, 65))
+                left -= 1
+                pos, total, plain = total, (total + n) & MASK, plain + n
+                if pos > cap:
+                    undo.append(n)
+            elif undo:
+                total = (total - undo.pop(int(rng.integers(len(undo))))) & MASK
+            most = max(most, total)
+            assert (total > cap) == (plain > cap)
+        assert most <= cap + 64 * 17
+        if plain <= cap:
+            assert total == plain
