@@ -59,7 +59,8 @@ int mtgl_set_option(GLState *ctx, int option, int value);
  * comes from one static 64 MiB device array that every GPU loading the library holds.
  * Returns 0, or MTGL_ERR_OVERFLOW when the pass needs more scratch than that or more
  * staging than ctx already holds; the pass then stays queued and renders at the next
- * mtgl_finish. All calls share the array, so calls whose GPU work overlapped would race:
+ * mtgl_finish. A pass that glFlush submitted before is completed first if need be, in the
+ * same array (or refused in the same way). All calls share the array, so calls whose GPU work overlapped would race:
  * every context renders on its own stream, so that holds even for two contexts flushed
  * one after the other from one thread. The library therefore orders them: each call's
  * GPU work waits for the previous call's on the same device (one event per device,

@@ -267,24 +267,30 @@ extern "C" int dev_current_device(void)
     return cudaGetDevice(&d) == cudaSuccess ? d : -1;
 }
 
-int mtgl_dev_settle(mtgl_dev *d)
+// The last flushed pass, checked against its totals; where its capacities did not hold it runs
+// again with scratch from `sc`. Refused for want of room in `sc` it stays as it is.
+static int settle_from(mtgl_dev *d, ScratchSource &sc)
 {
     if (!d->unsettled) return MTGL_OK;
-    d->unsettled = false;  // a failure below leaves nothing to retry
+    const bool pool = &sc == &d->x.pool;
+    d->unsettled = !pool;  // a failure below leaves nothing to retry
     const int st = d->stage.wait();
     if (st) return st;
     uint32_t nrec = d->x.h_totals[0], npairs = d->x.h_totals[1];
     if (nrec > d->ran_c.rec_cap || npairs > d->ran_c.pair_cap) {
         // the tile launch left the framebuffer untouched: run the staged tables again
+        const uint32_t totals[2] = {nrec, npairs};
         PipeConfig c;
         PipeOut o;
-        int rc = run_pipeline(d->x, d->x.pool, d->stage, d->ran_t, c, &o);
-        if (rc == MTGL_ERR_OVERFLOW) d->stage.used = 0;
+        int rc = run_pipeline(d->x, sc, d->stage, d->ran_t, c, &o);
+        if (rc) memcpy(d->x.h_totals, totals, sizeof(totals));  // the run's own may fit
+        if (rc == MTGL_ERR_OVERFLOW && pool) d->stage.used = 0;
         if (rc || (rc = d->stage.mark_uploaded(d->x.stream)) || (rc = d->stage.wait())) return rc;
         nrec = o.nrec;
         npairs = o.npairs;
         d->stats.kernel_launches += (uint64_t)o.launches;
     }
+    d->unsettled = false;
     d->x.rec_seen = std::max(d->x.rec_seen, nrec);
     d->x.pair_seen = std::max(d->x.pair_seen, npairs);
     d->stats.setup_triangles += nrec;
@@ -292,6 +298,8 @@ int mtgl_dev_settle(mtgl_dev *d)
     d->stage.used = 0;
     return MTGL_OK;
 }
+
+int mtgl_dev_settle(mtgl_dev *d) { return settle_from(d, d->x.pool); }
 
 int mtgl_dev_enter(mtgl_dev *d)
 {
@@ -850,7 +858,8 @@ int mtgl_dev_debug_bounds(void)
 //
 // Limits: a pass whose scratch does not fit is refused with MTGL_ERR_OVERFLOW before
 // anything is drawn, and stays queued (mtgl_finish or mtgl_dev_flush can still render
-// it). The pass's tables must fit the staging areas the context already holds. Every
+// it); so is one that glFlush submitted before and that turned out larger than its
+// capacities. The pass's tables must fit the staging areas the context already holds. Every
 // call, from every context on the device, shares the one array and overwrites what the
 // previous call left. Two calls whose GPU work overlapped would race on it (each context
 // has its own stream, so even two calls made one after the other from one thread would),
@@ -943,16 +952,41 @@ void drop_profile_marks(Exec &x, size_t keep)
 
 int flush_pass_noalloc(mtgl_dev *d)
 {
-    int st = mtgl_dev_enter(d);
-    if (st) return st;
+    int st;
+    std::unique_lock<std::mutex> lock(g_noalloc_mu, std::defer_lock);
+    NoAllocDevice *nd = nullptr;
+    Carve cv;
+    auto hold_array = [&]() -> int {
+        if (!lock.owns_lock()) lock.lock();
+        const int rc = noalloc_setup(d->device, &nd);
+        if (rc) return rc;
+        cv = Carve();
+        cv.base = nd->scratch;
+        cv.cap = kNoAllocScratchBytes;
+        // the previous call's kernels (any context, any stream) are done with the array first
+        if (nd->pending) CK(cudaStreamWaitEvent(d->x.stream, nd->done, 0));
+        return MTGL_OK;
+    };
+    // whatever was enqueued on the array, the next call waits for it
+    auto used_array = [&]() -> int {
+        CK(cudaEventRecord(nd->done, d->x.stream));
+        nd->pending = true;
+        return MTGL_OK;
+    };
+    if (d->unsettled) {  // an earlier flush's pass that has to run again takes the array too
+        const size_t marks = d->x.ev_pending.size();
+        if ((st = hold_array())) return st;
+        const int rc = settle_from(d, cv);
+        if ((st = used_array())) return st;
+        if (rc) {
+            drop_profile_marks(d->x, marks);
+            return rc;
+        }
+    }
+    if ((st = mtgl_dev_enter(d))) return st;
     Pass &P = d->pass;
     if (P.draws.empty()) return run_clears_only(d);  // clears launch kernels only
-    std::lock_guard<std::mutex> lock(g_noalloc_mu);
-    NoAllocDevice *nd = nullptr;
-    if ((st = noalloc_setup(d->device, &nd))) return st;
-    Carve cv;
-    cv.base = nd->scratch;
-    cv.cap = kNoAllocScratchBytes;
+    if ((st = hold_array())) return st;
     const size_t used0 = d->stage.used;
     const size_t marks0 = d->x.ev_pending.size();
     FrameSrc fs{d, &P, 0, HostFrame()};
@@ -966,15 +1000,11 @@ int flush_pass_noalloc(mtgl_dev *d)
                      "mtgl_flush_noalloc: the pass's tables exceed the context's staging areas; the pass stays queued");
         return st;
     }
-    // the previous call's kernels (any context, any stream) are done with the array first
-    if (nd->pending) CK(cudaStreamWaitEvent(d->x.stream, nd->done, 0));
     PipeConfig c;  // exact sizing
     PipeOut o;
-    st = run_pipeline(d->x, cv, d->stage, t, c, &o);
-    // whatever this call enqueued, the next call waits for it
-    CK(cudaEventRecord(nd->done, d->x.stream));
-    nd->pending = true;
-    if (st) {
+    const int rc = run_pipeline(d->x, cv, d->stage, t, c, &o);
+    if ((st = used_array())) return st;
+    if ((st = rc)) {
         d->stage.used = used0;  // drop the tables; the pass stays queued
         drop_profile_marks(d->x, marks0);
         return st;

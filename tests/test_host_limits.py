@@ -80,6 +80,50 @@ def test_a_batch_past_32_bits_is_refused(fake, gpu):
     b.destroy()
 
 
+@pytest.mark.parametrize("then", ["nothing", "clear", "draw"])
+def test_noalloc_flush_completes_a_flushed_pass_without_allocating(gpu, then):
+    """glFlush submits a pass that exceeds its capacities; mtgl_flush_noalloc runs it again, and
+    what is queued, from the static array."""
+    ctx, ctl = gpu
+    for _ in range(2):
+        draw(ctx)
+        assert finish(ctx) == MTGL_OK
+    draw(ctx)
+    ctl.fake_totals(5000, 6000)
+    ctx.glFlush()
+    assert log(ctl)[-1] == "over"
+    before = ctl.fake_allocs()
+    ctl.fake_totals(6, 10)
+    if then == "clear":
+        ctx.glClear(G.GL_COLOR_BUFFER_BIT)
+    assert ctx.glib.lib.mtgl_flush_noalloc(ctx.handle) == MTGL_OK
+    assert log(ctl) == "vertex count emit bin sort tile".split() + ["clear"] * (then == "clear")
+    if then == "draw":
+        draw(ctx)  # (the draw completes a flushed pass itself)
+        before = ctl.fake_allocs()
+        assert ctx.glib.lib.mtgl_flush_noalloc(ctx.handle) == MTGL_OK
+        assert log(ctl)[-1] == "tile"
+    assert ctl.fake_allocs() == before
+    assert finish(ctx) == MTGL_OK and ctx.glGetError() == 0
+
+
+def test_noalloc_flush_refuses_a_flushed_pass_that_does_not_fit(gpu):
+    """The flushed pass needs more than the static array: refused, nothing allocated, as often as
+    asked, and the next ordinary call renders it."""
+    ctx, ctl = gpu
+    draw(ctx)
+    ctl.fake_totals(400_000, 6000)  # 96 MB of records
+    ctx.glFlush()
+    log(ctl)
+    before = ctl.fake_allocs()
+    for _ in range(2):
+        assert ctx.glib.lib.mtgl_flush_noalloc(ctx.handle) == MTGL_ERR_OVERFLOW
+        assert "tile" not in log(ctl) and ctl.fake_allocs() == before
+    assert finish(ctx) == MTGL_OK
+    assert log(ctl)[-1] == "tile"
+    assert ctx.stats()["setup_triangles"] == 400_000
+
+
 # ---- the sums that decide it, restated
 
 MASK = 0xFFFFFFFF
