@@ -123,6 +123,7 @@ struct PoolScratch final : ScratchSource {
     void *p[kScratchSlots] = {};
     size_t cap[kScratchSlots] = {};
     uint64_t allocs = 0;  // device allocations made by growth
+    bool shortage = false;  // an allocation found no memory
     int get(int slot, size_t bytes, void **out) override;
     void release();
 };

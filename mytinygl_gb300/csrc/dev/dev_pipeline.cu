@@ -14,6 +14,7 @@ thread_local char g_err[512] = "";
 int fail_cuda(const char *what, cudaError_t e)
 {
     snprintf(g_err, sizeof(g_err), "%s: %s", what, cudaGetErrorString(e));
+    cudaGetLastError();  // reported here: not left for a later check to find
     return MTGL_ERR_CUDA;
 }
 
@@ -215,7 +216,12 @@ int PoolScratch::get(int slot, size_t bytes, void **out)
         if (p[slot]) CK(cudaFreeAsync(p[slot], stream));
         p[slot] = nullptr;
         cap[slot] = 0;
-        CK(cudaMallocAsync(&p[slot], ncap, stream));
+        const cudaError_t e = cudaMallocAsync(&p[slot], ncap, stream);
+        if (e != cudaSuccess) {
+            p[slot] = nullptr;
+            shortage = e == cudaErrorMemoryAllocation;
+            return fail_cuda("cudaMallocAsync", e);
+        }
         allocs++;
         cap[slot] = ncap;
     }

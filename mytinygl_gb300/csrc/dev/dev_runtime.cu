@@ -189,7 +189,8 @@ int run_clears_only(mtgl_dev *d)
 // screen's edge made up to 1.6 times their triangles) and an eighth in large ones; four pairs per record, and at least 2^18 (a few megabytes) unless the frame
 // cannot have that many. Totals beyond them cost one more run of the pass (mtgl_dev_settle).
 // A pass of more than 2^22 primitives, whose records may be gigabytes of which few are
-// needed, takes exact sizes instead: its two waits are nothing beside it.
+// needed, takes exact sizes instead: its two waits are nothing beside it. So does one whose
+// estimate finds no memory (flush_pass).
 PipeConfig capacities(const mtgl_dev *d, const Tables &t)
 {
     const Pass &P = d->pass;
@@ -218,12 +219,21 @@ int flush_pass(mtgl_dev *d, const HostFrame &host = HostFrame())
     if (st) return st;
     Pass &P = d->pass;
     if (P.draws.empty()) return run_clears_only(d);
+    const size_t used0 = d->stage.used;
     FrameSrc fs{d, &P, 0, host};
     Tables t;
     if ((st = build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, true, t))) return st;
-    const PipeConfig c = capacities(d, t);
+    PipeConfig c = capacities(d, t);
     PipeOut o;
-    if ((st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o))) {
+    d->x.pool.shortage = false;
+    st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o);
+    if (st && d->x.pool.shortage) {  // the estimate found no memory: exact sizes, in a pool without its buffers, may
+        c = PipeConfig();
+        d->x.pool.release();
+        st = run_pipeline(d->x, d->x.pool, d->stage, t, c, &o);
+    }
+    if (st) {
+        d->stage.used = used0;  // drop the tables; the pass stays queued
         if (st == MTGL_ERR_OVERFLOW) {  // no size renders it: the frame goes without
             P.reset();
             d->stage.used = 0;
@@ -268,12 +278,11 @@ extern "C" int dev_current_device(void)
 }
 
 // The last flushed pass, checked against its totals; where its capacities did not hold it runs
-// again with scratch from `sc`. Refused for want of room in `sc` it stays as it is.
+// again with scratch from `sc`. When that fails the pass stays as it is, for the next call to try
+// again, unless no amount of memory renders it.
 static int settle_from(mtgl_dev *d, ScratchSource &sc)
 {
     if (!d->unsettled) return MTGL_OK;
-    const bool pool = &sc == &d->x.pool;
-    d->unsettled = !pool;  // a failure below leaves nothing to retry
     const int st = d->stage.wait();
     if (st) return st;
     uint32_t nrec = d->x.h_totals[0], npairs = d->x.h_totals[1];
@@ -282,9 +291,18 @@ static int settle_from(mtgl_dev *d, ScratchSource &sc)
         const uint32_t totals[2] = {nrec, npairs};
         PipeConfig c;
         PipeOut o;
+        d->x.pool.shortage = false;
         int rc = run_pipeline(d->x, sc, d->stage, d->ran_t, c, &o);
+        if (rc && d->x.pool.shortage) {  // the first run's buffers may be in the way
+            d->x.pool.release();
+            rc = run_pipeline(d->x, sc, d->stage, d->ran_t, c, &o);
+        }
+        if (rc == MTGL_ERR_OVERFLOW && &sc == &d->x.pool) {
+            d->unsettled = false;
+            d->stage.used = 0;
+            return rc;
+        }
         if (rc) memcpy(d->x.h_totals, totals, sizeof(totals));  // the run's own may fit
-        if (rc == MTGL_ERR_OVERFLOW && pool) d->stage.used = 0;
         if (rc || (rc = d->stage.mark_uploaded(d->x.stream)) || (rc = d->stage.wait())) return rc;
         nrec = o.nrec;
         npairs = o.npairs;
@@ -757,7 +775,15 @@ int mtgl_dev_read(mtgl_dev *d, uint32_t *color, float *depth, uint8_t *stencil)
         host.stencil = (uint8_t *)mapped_host(stencil, n);
     }
     int st = flush_pass(d, host);
-    if (st || (st = mtgl_dev_settle(d))) return st;
+    if (st || (st = mtgl_dev_settle(d))) {
+        if (d->unsettled) {  // its next run must not write the caller's memory any more
+            DevFrame *f = reinterpret_cast<DevFrame *>(d->stage.p + d->ran_t.off_frames);
+            f->host_color = nullptr;
+            f->host_depth = nullptr;
+            f->host_stencil = nullptr;
+        }
+        return st;
+    }
     cudaStream_t s = d->x.stream;
     if (color && !host.color) CK(cudaMemcpyAsync(color, d->color, n * 4, cudaMemcpyDeviceToHost, s));
     if (depth && !host.depth) CK(cudaMemcpyAsync(depth, d->depth, n * 4, cudaMemcpyDeviceToHost, s));

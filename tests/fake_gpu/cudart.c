@@ -8,9 +8,11 @@
 static size_t g_limit; /* bytes (0: none) */
 static long g_allocs;  /* device and page-locked allocations made */
 static cudaError_t g_last;
+static int g_locked;   /* all host memory is page-locked */
 static char g_token[16];
 
 void fake_alloc_limit(size_t bytes) { g_limit = bytes; }
+void fake_page_locked(int on) { g_locked = on; }
 long fake_allocs(void) { return g_allocs; }
 
 static cudaError_t fail(cudaError_t e)
@@ -59,8 +61,11 @@ cudaError_t cudaMemsetAsync(void *d, int v, size_t n, cudaStream_t s) { (void)s;
 cudaError_t cudaGetSymbolAddress(void **p, const void *symbol) { *p = (void *)symbol; return cudaSuccess; }
 cudaError_t cudaPointerGetAttributes(struct cudaPointerAttributes *a, const void *p)
 {
-    (void)p;
     memset(a, 0, sizeof(*a)); /* ordinary host memory */
+    if (g_locked) {
+        a->type = cudaMemoryTypeHost;
+        a->devicePointer = a->hostPointer = (void *)p;
+    }
     return cudaSuccess;
 }
 

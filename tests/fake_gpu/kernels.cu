@@ -1,6 +1,6 @@
 // kernels.cu — stand-ins for the kernel launches: no pixel is computed. Each names itself in a log,
 // the counting ones give the totals a test asks for, and the tile launch notes whether its guard
-// let it write.
+// let it write, and whether it writes the frame to the host too.
 #include <string>
 
 #include "dev_internal.h"
@@ -67,7 +67,8 @@ int launch_tile_ranges(const BinArgs &, cudaStream_t) { return 1; }
 int launch_tile_order(const uint32_t *, uint32_t, uint32_t *, uint32_t *, int, cudaStream_t) { return 2; }
 int launch_tile(const TileArgs &a, cudaStream_t)
 {
-    return say(a.guard && (a.guard[0] > a.records_cap || a.guard[1] > a.pairs_cap) ? "over" : "tile");
+    if (a.guard && (a.guard[0] > a.records_cap || a.guard[1] > a.pairs_cap)) return say("over");
+    return say(a.frames[0].host_color ? "tile+read" : "tile");
 }
 int tile_occupancy(const TileArgs &) { return 4; }
 void launch_clear(const ClearOp *, int, FrameDims, uint32_t *, float *, uint8_t *, cudaStream_t) { say("clear"); }

@@ -25,6 +25,7 @@ def gpu(fake):
     ctl.fake_log_clear()
     ctx = lib.context(64, 48)
     yield ctx, ctl
+    ctl.fake_page_locked(0)
     ctl.fake_alloc_limit(0)
     ctl.fake_totals(5, 9)
     ctx.destroy()
@@ -122,6 +123,72 @@ def test_noalloc_flush_refuses_a_flushed_pass_that_does_not_fit(gpu):
     assert finish(ctx) == MTGL_OK
     assert log(ctl)[-1] == "tile"
     assert ctx.stats()["setup_triangles"] == 400_000
+
+
+def draw_many(ctx, n):
+    """n triangles over three vertices."""
+    pos = np.array([[-0.5, -0.5], [0.5, -0.5], [0.0, 0.5]], np.float32)
+    ctx.glClear(G.GL_COLOR_BUFFER_BIT)
+    ctx.glEnableClientState(G.GL_VERTEX_ARRAY)
+    ctx.glVertexPointer(2, G.GL_FLOAT, 0, pos)
+    ctx.glDrawElements(G.GL_TRIANGLES, 3 * n, G.GL_UNSIGNED_INT, np.tile(np.arange(3, dtype=np.uint32), n))
+
+
+def test_an_estimate_without_memory_takes_exact_sizes(gpu):
+    """100,000 triangles of which 5 make records: the estimate asks for 27 MB of records, the pass
+    needs 2 MB."""
+    ctx, ctl = gpu
+    draw_many(ctx, 100_000)
+    ctl.fake_alloc_limit(8 << 20)
+    ctx.glFlush()
+    assert ctx.glGetError() == 0
+    assert log(ctl) == "vertex count emit bin sort tile".split()
+    assert finish(ctx) == MTGL_OK
+
+
+def test_a_pass_without_memory_stays_queued(gpu):
+    ctx, ctl = gpu
+    draw_many(ctx, 1000)
+    ctl.fake_alloc_limit(64)
+    assert finish(ctx) != MTGL_OK and finish(ctx) != MTGL_OK
+    assert "tile" not in log(ctl)
+    ctl.fake_alloc_limit(0)
+    assert finish(ctx) == MTGL_OK and log(ctl)[-1] == "tile"
+    assert ctx.stats()["passes"] == 1
+
+
+def test_a_second_run_without_memory_is_tried_again(gpu):
+    """The pass exceeded its capacities and the exact sizes find no memory: every call that needs the
+    frame says so, and the first that finds memory renders it."""
+    ctx, ctl = gpu
+    draw(ctx)
+    ctl.fake_totals(400_000, 6000)
+    ctx.glFlush()
+    assert log(ctl)[-1] == "over"
+    ctl.fake_alloc_limit(8 << 20)
+    assert finish(ctx) != MTGL_OK and finish(ctx) != MTGL_OK
+    assert "tile" not in log(ctl)
+    ctl.fake_alloc_limit(0)
+    assert finish(ctx) == MTGL_OK and log(ctl)[-1] == "tile"
+    assert ctx.stats()["setup_triangles"] == 400_000
+
+
+def test_a_failed_read_is_not_written_later(gpu):
+    """A read into page-locked memory fails for want of memory: the pass renders later without
+    writing that memory."""
+    ctx, ctl = gpu
+    host = np.zeros(64 * 48, np.uint32)
+    read = ctx.glib.lib.mtgl_read_framebuffer
+    at = ctypes.c_void_p(host.ctypes.data)
+    ctl.fake_page_locked(1)
+    draw(ctx)
+    assert read(ctx.handle, at, None, None) == MTGL_OK and log(ctl)[-1] == "tile+read"
+    draw(ctx)
+    ctl.fake_totals(400_000, 6000)
+    ctl.fake_alloc_limit(8 << 20)
+    assert read(ctx.handle, at, None, None) != MTGL_OK and "over" in log(ctl)
+    ctl.fake_alloc_limit(0)
+    assert finish(ctx) == MTGL_OK and log(ctl)[-1] == "tile"
 
 
 # ---- the sums that decide it, restated
