@@ -71,7 +71,7 @@ size_t scan_temp_words(uint32_t n);
 // Sums stay at 2^32 - 1 instead of wrapping. With `host` (two page-locked words) the launch also
 // writes rec_total[0] and [1], the pass's record and pair totals, there.
 int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
-                cudaStream_t s, const uint32_t *rec_total = nullptr, uint32_t *host = nullptr, bool temp_zeroed = false);
+                cudaStream_t s, const uint32_t *rec_total = nullptr, uint32_t *host = nullptr);
 
 // The most records or pairs a pass may make: a larger total is refused (MTGL_ERR_OVERFLOW). Below
 // 2^32 by more than the kernels' strides, so that their 32-bit loops end.
@@ -98,11 +98,10 @@ struct BinArgs {
     uint32_t *tile_start;       // exclusive scan of tile_count
     uint32_t *tile_frame;       // per tile: the frame owning it, written with the tiles' ranges (null: one frame)
     uint32_t *radix_hist;       // radix histograms
-    uint32_t *scan_temp;
+    uint32_t *scan_temp;        // (zero at launch in order-free passes)
     uint32_t *total_dev;        // where the pair scan writes its total: the pairs generated
     uint32_t *totals_host;      // page-locked words that get the record and pair totals (may be null)
     uint32_t *sort_total_dev;   // a word the sort's histogram scans may overwrite
-    int32_t scan_zeroed;        // scan_temp is zero already
     int32_t order_free;         // tile lists need no order (k_tile_free.cu)
     uint32_t npairs;            // pair capacity of keys/vals (writes beyond are dropped)
     int32_t sms;                // SMs of the device (grid sizes)

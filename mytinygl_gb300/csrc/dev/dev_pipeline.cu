@@ -657,7 +657,6 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
     ba.debug = x.d_totals + kDebugStatusWord;
     ba.order_free = free_setup ? 1 : 0;
     ba.scan_temp = free_setup ? tile_count + scan_at : scan_temp;
-    ba.scan_zeroed = free_setup ? 1 : 0;
     ba.sms = x.sms;
     uint32_t pair_cap = c.pair_cap;
     ba.units = bin_units(rec_cap, x.sms);

@@ -34,47 +34,65 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v)
 
 // Sums that stay at the largest value instead of wrapping, so that a total past 32 bits is seen as
 // one that fits nowhere. (Saturating addition of unsigned numbers is associative: the sum, or
-// the limit.)
-__device__ __forceinline__ uint32_t sat_add(uint32_t a, uint32_t b)
+// the limit.) Scans whose total decides nothing (SAT false) add plainly.
+template <bool SAT>
+__device__ __forceinline__ uint32_t add_to(uint32_t a, uint32_t b)
 {
     const uint32_t s = a + b;
-    return s < a ? 0xFFFFFFFFu : s;
+    return SAT && s < a ? 0xFFFFFFFFu : s;
 }
-// saturating scan over the warp: returns the exclusive sum, the inclusive one in *incl
-__device__ __forceinline__ uint32_t warp_sat_scan(uint32_t v, uint32_t *incl)
+// scan over the warp: returns the exclusive sum, the inclusive one in *incl
+template <bool SAT>
+__device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *incl)
 {
     const int lane = threadIdx.x & 31;
+    uint32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t n = __shfl_up_sync(0xffffffffu, v, o);
-        if (lane >= o) v = sat_add(v, n);
+        const uint32_t n = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x = add_to<SAT>(x, n);
     }
-    *incl = v;
-    const uint32_t before = __shfl_up_sync(0xffffffffu, v, 1);
+    *incl = x;
+    if (!SAT) return x - v;
+    const uint32_t before = __shfl_up_sync(0xffffffffu, x, 1);
     return lane ? before : 0u;
 }
 
 // exclusive block scan of one value per thread; returns the block total in *total
+template <bool SAT>
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t *total)
 {
     __shared__ uint32_t warp_sums[kScanThreads / 32 + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t incl;
-    const uint32_t before = warp_sat_scan(v, &incl);
+    const uint32_t before = warp_excl_scan<SAT>(v, &incl);
     if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
     if (warp == 0) {
         uint32_t wi;
-        const uint32_t wb = warp_sat_scan(lane < kScanThreads / 32 ? warp_sums[lane] : 0u, &wi);
+        const uint32_t wb = warp_excl_scan<SAT>(lane < kScanThreads / 32 ? warp_sums[lane] : 0u, &wi);
         __syncwarp();
         if (lane < kScanThreads / 32) warp_sums[lane] = wb;
         if (lane == kScanThreads / 32 - 1) warp_sums[kScanThreads / 32] = wi;
     }
     __syncthreads();
-    const uint32_t r = sat_add(warp_sums[warp], before);
+    const uint32_t r = add_to<SAT>(warp_sums[warp], before);
     *total = warp_sums[kScanThreads / 32];
     __syncthreads();
     return r;
+}
+
+// A radix sort's work: pairs on the device, their capacity, digits of a pass.
+struct SortCount {
+    const uint32_t *pairs;
+    uint32_t cap, digits;
+};
+constexpr int kRadixThreads = 256;
+constexpr int kRadixItems = 8;  // per thread
+constexpr int kRadixTile = kRadixThreads * kRadixItems;
+__host__ __device__ __forceinline__ uint32_t radix_blocks(uint32_t pairs)
+{
+    return pairs / kRadixTile + (pairs % kRadixTile ? 1u : 0u);
 }
 
 // Single-pass exclusive scan with decoupled look-back (Merrill and Garland, "Single-pass
@@ -93,14 +111,20 @@ constexpr uint64_t kScanSum = 1ull << 32, kScanPrefix = 2ull << 32;
 __device__ __forceinline__ uint64_t ld_status(const uint64_t *p) { return *(const volatile uint64_t *)p; }
 __device__ __forceinline__ void st_status(uint64_t *p, uint64_t v) { *(volatile uint64_t *)p = v; }
 
+// With `sort` the values are a digit histogram's, a column per tile of the pairs there are (n: of as
+// many as fit), and the blocks past them leave at once.
+template <bool SAT>
 __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint32_t *out, uint32_t n,
                                                       uint64_t *status, uint32_t *ticket, uint32_t *total_dev,
-                                                      uint32_t *debug, const uint32_t *rec_total, uint32_t *host)
+                                                      uint32_t *debug, const uint32_t *rec_total, uint32_t *host,
+                                                      SortCount sort)
 {
     __shared__ uint32_t s_tile, s_prefix;
     if (threadIdx.x == 0) s_tile = gridDim.x == 1 ? 0u : atomicAdd(ticket, 1u);
+    if (sort.pairs) n = radix_blocks(min(__ldg(sort.pairs), sort.cap)) * sort.digits;
     __syncthreads();
     const uint32_t tile = s_tile;
+    if (sort.pairs && (uint64_t)tile * kScanTile >= n) return;
     const uint32_t base = tile * (uint32_t)kScanTile + threadIdx.x * kScanItems;
     // each thread's 8 values as two 16-byte words (base is a multiple of 8 words)
     uint32_t v[kScanItems];
@@ -113,9 +137,9 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
     }
     uint32_t sum = 0;
 #pragma unroll
-    for (int i = 0; i < kScanItems; i++) sum = sat_add(sum, v[i]);
+    for (int i = 0; i < kScanItems; i++) sum = add_to<SAT>(sum, v[i]);
     uint32_t agg;
-    uint32_t run = block_excl_scan(sum, &agg);
+    uint32_t run = block_excl_scan<SAT>(sum, &agg);
     if (threadIdx.x < 32) {
         // warp 0 looks back 32 tiles at a time: lane k reads the status of tile (window - k)
         const uint32_t lane = threadIdx.x;
@@ -138,19 +162,23 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
                 // the nearest tile with its inclusive prefix ends the walk; the nearer ones add sums
                 const uint32_t prefixed = __ballot_sync(0xffffffffu, (st >> 32) == 2);
                 const uint32_t upto = prefixed ? (uint32_t)__ffs(prefixed) - 1u : 31u;
-                // (in halves, whose 32 sums fit)
-                const uint32_t add = lane <= upto ? (uint32_t)st : 0u;
-                const uint32_t lo = __reduce_add_sync(0xffffffffu, add & 0xFFFFu);
-                const uint32_t hi = __reduce_add_sync(0xffffffffu, add >> 16) + (lo >> 16);
-                prefix = sat_add(prefix, hi > 0xFFFFu ? 0xFFFFFFFFu : (hi << 16) | (lo & 0xFFFFu));
+                uint32_t add = lane <= upto ? (uint32_t)st : 0u;
+                if (SAT) {  // in halves, whose 32 sums fit
+                    const uint32_t lo = __reduce_add_sync(0xffffffffu, add & 0xFFFFu);
+                    const uint32_t hi = __reduce_add_sync(0xffffffffu, add >> 16) + (lo >> 16);
+                    add = hi > 0xFFFFu ? 0xFFFFFFFFu : (hi << 16) | (lo & 0xFFFFu);
+                } else {
+                    add = __reduce_add_sync(0xffffffffu, add);
+                }
+                prefix = add_to<SAT>(prefix, add);
                 if (prefixed) break;
             }
-            if (lane == 0) st_status(status + tile, kScanPrefix | sat_add(prefix, agg));
+            if (lane == 0) st_status(status + tile, kScanPrefix | add_to<SAT>(prefix, agg));
         }
         if (lane == 0) {
             s_prefix = prefix;
             if (tile + 1 == gridDim.x) {
-                *total_dev = sat_add(prefix, agg);
+                *total_dev = add_to<SAT>(prefix, agg);
                 if (host) {  // page-locked: the pass's record and pair totals, without a copy behind it
                     host[0] = rec_total[0];
                     host[1] = rec_total[1];  // an ordered pass's is this scan's
@@ -159,12 +187,12 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(const uint32_t *in, uint3
         }
     }
     __syncthreads();
-    run = sat_add(run, s_prefix);
+    run = add_to<SAT>(run, s_prefix);
     uint32_t o[kScanItems];
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         o[i] = run;
-        run = sat_add(run, v[i]);
+        run = add_to<SAT>(run, v[i]);
     }
     if (base + kScanItems <= n) {
         *reinterpret_cast<uint4 *>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
@@ -182,8 +210,9 @@ size_t scan_temp_words(uint32_t n)
     return 2 * (((size_t)n + kScanTile - 1) / kScanTile) + 64;
 }
 
-int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
-                cudaStream_t s, const uint32_t *rec_total, uint32_t *host, bool temp_zeroed)
+template <bool SAT>
+static int start_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
+                      cudaStream_t s, const uint32_t *rec_total, uint32_t *host, SortCount sort, bool temp_zeroed = false)
 {
     if (n == 0) {
         cudaMemsetAsync(total_dev, 0, sizeof(uint32_t), s);
@@ -195,8 +224,14 @@ int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, u
     uint64_t *status = reinterpret_cast<uint64_t *>(temp);
     uint32_t *ticket = temp + 2 * (size_t)nb;
     if (nb > 1 && !temp_zeroed) cudaMemsetAsync(temp, 0, (2 * (size_t)nb + 1) * sizeof(uint32_t), s);
-    k_scan<<<nb, kScanThreads, 0, s>>>(in, out, n, status, ticket, total_dev, debug, rec_total, host);
+    k_scan<SAT><<<nb, kScanThreads, 0, s>>>(in, out, n, status, ticket, total_dev, debug, rec_total, host, sort);
     return 1;
+}
+
+int launch_scan(const uint32_t *in, uint32_t *out, uint32_t n, uint32_t *temp, uint32_t *total_dev, uint32_t *debug,
+                cudaStream_t s, const uint32_t *rec_total, uint32_t *host)
+{
+    return start_scan<true>(in, out, n, temp, total_dev, debug, s, rec_total, host, SortCount{nullptr, 0u, 0u});
 }
 
 // ------------------------------------------------------------------ record -> tiles
@@ -427,13 +462,7 @@ __device__ __forceinline__ void flush_pairs(const BinArgs &A, const uint2 *queue
 {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t pos = 0;
-    if (lane == 0) {
-        // Past the capacity the exact total serves nothing, and would wrap: an addition that finds
-        // it exceeded is taken back, so that it stays exceeded and below the capacity (at most
-        // kMaxEntries) and 64 for every resident warp, far from 2^32.
-        pos = atomicAdd(A.total_dev, n);
-        if (pos > A.npairs) atomicSub(A.total_dev, n);
-    }
+    if (lane == 0) pos = atomicAdd(A.total_dev, n);
     uint2 q[kQueueFlush / 32];
     uint32_t rank[kQueueFlush / 32];
 #pragma unroll
@@ -442,6 +471,10 @@ __device__ __forceinline__ void flush_pairs(const BinArgs &A, const uint2 *queue
             q[k] = queue[k * 32 + lane];
             rank[k] = atomicAdd(A.tile_count + q[k].x, 1u);
         }
+    // Past the capacity the exact total serves nothing, and would wrap: an addition that finds it
+    // exceeded is taken back, so that it stays exceeded and below the capacity (at most kMaxEntries)
+    // and 64 for every resident warp, far from 2^32. (Looked at here, with the ranks on their way.)
+    if (lane == 0 && pos > A.npairs) atomicSub(A.total_dev, n);
     pos = __shfl_sync(0xffffffffu, pos, 0) + lane;
 #pragma unroll
     for (uint32_t k = 0; k < kQueueFlush / 32; k++, pos += 32)
@@ -621,8 +654,8 @@ int launch_bin_count(const BinArgs &a, cudaStream_t s)
                               launch_scan(a.rec_tiles, a.rec_tiles, a.units, a.scan_temp, a.total_dev, a.debug, s, a.nrec_dev,
                                           a.totals_host);
     return occlude + launch_records<PASS_PAIRS>(a, s) +
-           launch_scan(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.sort_total_dev, a.debug, s, a.nrec_dev,
-                       a.totals_host, a.scan_zeroed != 0);
+           start_scan<false>(a.tile_count, a.tile_start, a.ntiles, a.scan_temp, a.sort_total_dev, a.debug, s, a.nrec_dev,
+                             a.totals_host, SortCount{nullptr, 0u, 0u}, true);
 }
 
 int launch_bin_expand(const BinArgs &a, cudaStream_t s)
@@ -692,35 +725,38 @@ int launch_tile_order(const uint32_t *tile_count, uint32_t ntiles, uint32_t *aux
 
 // ------------------------------------------------------------------ stable radix sort by tile
 
-constexpr int kRadixThreads = 256;
+// The grids and the scratch are for the capacity, the work for the pairs there are: blocks step
+// through the tiles of kRadixTile pairs, and a pass's histogram has a column per tile in use. (A
+// context's capacity is its largest pass's: 40 blended quads after a pass of two million in the
+// same context, whole passes: 371 us with a histogram of the capacity, 267 so, 255 in a context
+// of their own.)
 constexpr int kRadixWarps = kRadixThreads / 32;
-constexpr int kRadixItems = 8;  // per thread
-constexpr int kRadixTile = kRadixThreads * kRadixItems;
 constexpr int kRadixDigits = 512;  // up to 9-bit digits; a sort uses ceil(bits / 9) balanced passes
 
 size_t radix_hist_words(uint32_t npairs)
 {
-    const size_t nb = (npairs + kRadixTile - 1) / kRadixTile;
-    return nb * kRadixDigits + 64;
+    return (size_t)radix_blocks(npairs) * kRadixDigits + 64;
 }
 
 __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t *keys, uint32_t cap,
                                                              const uint32_t *n_dev, int shift, uint32_t mask,
-                                                             uint32_t *hist, uint32_t nblocks)
+                                                             uint32_t *hist)
 {
-    const uint32_t n = min(*n_dev, cap);
+    const uint32_t n = min(*n_dev, cap), nblocks = radix_blocks(n);
     const int ndig = (int)mask + 1;
     __shared__ uint32_t h[kRadixDigits];
-    for (int i = threadIdx.x; i < ndig; i += kRadixThreads) h[i] = 0;
-    __syncthreads();
-    const uint32_t base = blockIdx.x * (uint32_t)kRadixTile;
+    for (uint32_t b = blockIdx.x; b < nblocks; b += gridDim.x) {
+        for (int i = threadIdx.x; i < ndig; i += kRadixThreads) h[i] = 0;
+        __syncthreads();
+        const uint32_t base = b * (uint32_t)kRadixTile;
 #pragma unroll
-    for (int k = 0; k < kRadixItems; k++) {
-        const uint32_t i = base + k * kRadixThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & mask], 1u);
+        for (int k = 0; k < kRadixItems; k++) {
+            const uint32_t i = base + k * kRadixThreads + threadIdx.x;
+            if (i < n) atomicAdd(&h[(keys[i] >> shift) & mask], 1u);
+        }
+        __syncthreads();
+        for (int d = threadIdx.x; d < ndig; d += kRadixThreads) hist[(size_t)d * nblocks + b] = h[d];
     }
-    __syncthreads();
-    for (int d = threadIdx.x; d < ndig; d += kRadixThreads) hist[(size_t)d * nblocks + blockIdx.x] = h[d];
 }
 
 // Stable scatter: warp w owns items [w*256, w*256+256) of the block, taken 32 at a time in
@@ -731,95 +767,98 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t *ke
 __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t *keys, const uint32_t *vals,
                                                                 uint32_t cap, const uint32_t *n_dev, int shift,
                                                                 uint32_t mask,
-                                                                const uint32_t *hist_scan, uint32_t nblocks,
+                                                                const uint32_t *hist_scan,
                                                                 uint32_t *keys_out, uint32_t *vals_out)
 {
     __shared__ uint32_t wcount[kRadixWarps][kRadixDigits];  // per warp and digit: count, then block-local start
     __shared__ uint32_t dstart[kRadixDigits];                // block-local start of each digit's run
     __shared__ uint32_t gdelta[kRadixDigits];                // global start minus block-local start
     __shared__ uint32_t skey[kRadixTile], sval[kRadixTile];
-    const uint32_t n = min(*n_dev, cap);
+    __shared__ uint32_t wsum[kRadixWarps];
+    const uint32_t n = min(*n_dev, cap), nblocks = radix_blocks(n);
     const int ndig = (int)mask + 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < kRadixWarps * kRadixDigits; i += kRadixThreads) (&wcount[0][0])[i] = 0;
-    __syncthreads();
-    const uint32_t bbase = blockIdx.x * (uint32_t)kRadixTile;
-    const uint32_t wbase = bbase + warp * 32 * kRadixItems;
     const uint32_t lt = (1u << lane) - 1u;
-    uint32_t key[kRadixItems], val[kRadixItems], rank[kRadixItems];
-#pragma unroll
-    for (int k = 0; k < kRadixItems; k++) {
-        const uint32_t i = wbase + k * 32 + lane;
-        const bool valid = i < n;
-        key[k] = valid ? keys[i] : 0u;
-        val[k] = valid ? vals[i] : 0u;
-        const uint32_t d = valid ? ((key[k] >> shift) & mask) : 0xFFFFFFFFu;
-        const uint32_t peers = __match_any_sync(0xffffffffu, d);
-        const int leader = __ffs(peers) - 1;
-        const uint32_t pre = valid ? wcount[warp][d] : 0u;
-        __syncwarp();
-        if (valid && lane == leader) wcount[warp][d] = pre + __popc(peers);
-        __syncwarp();
-        rank[k] = pre + __popc(peers & lt);
-    }
-    __syncthreads();
-    // per digit: the block's count, then each warp's start within the digit's run
-    for (int d = threadIdx.x; d < kRadixDigits; d += kRadixThreads) {
-        uint32_t run = 0;
-#pragma unroll
-        for (int w = 0; w < kRadixWarps; w++) {
-            const uint32_t c = d < ndig ? wcount[w][d] : 0u;
-            wcount[w][d] = run;
-            run += c;
-        }
-        dstart[d] = run;  // the count for now
-    }
-    __syncthreads();
-    // exclusive scan of the digit counts (512 entries, 2 per thread) into block-local starts
-    {
-        const int d0 = 2 * threadIdx.x;
-        const uint32_t c0 = dstart[d0], c1 = dstart[d0 + 1];
-        uint32_t incl = c0 + c1, x = incl;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        __shared__ uint32_t wsum[kRadixWarps];
-        if (lane == 31) wsum[warp] = x;
+    for (uint32_t b = blockIdx.x; b < nblocks; b += gridDim.x) {
+        if (b != blockIdx.x) __syncthreads();  // the previous tile's pairs have left
+        for (int i = threadIdx.x; i < kRadixWarps * kRadixDigits; i += kRadixThreads) (&wcount[0][0])[i] = 0;
         __syncthreads();
-        uint32_t before = 0;
-        for (int w = 0; w < warp; w++) before += wsum[w];
-        const uint32_t excl = before + x - incl;
-        __syncthreads();
-        dstart[d0] = excl;
-        dstart[d0 + 1] = excl + c0;
-        if (d0 < ndig) gdelta[d0] = hist_scan[(size_t)d0 * nblocks + blockIdx.x] - excl;
-        if (d0 + 1 < ndig) gdelta[d0 + 1] = hist_scan[(size_t)(d0 + 1) * nblocks + blockIdx.x] - (excl + c0);
-    }
-    __syncthreads();
-    // items into shared memory in digit order (stable: warp order, then item order)
+        const uint32_t bbase = b * (uint32_t)kRadixTile;
+        const uint32_t wbase = bbase + warp * 32 * kRadixItems;
+        uint32_t key[kRadixItems], val[kRadixItems], rank[kRadixItems];
 #pragma unroll
-    for (int k = 0; k < kRadixItems; k++) {
-        const uint32_t i = wbase + k * 32 + lane;
-        if (i < n) {
-            const uint32_t d = (key[k] >> shift) & mask;
-            const uint32_t at = dstart[d] + wcount[warp][d] + rank[k];
-            skey[at] = key[k];
-            sval[at] = val[k];
+        for (int k = 0; k < kRadixItems; k++) {
+            const uint32_t i = wbase + k * 32 + lane;
+            const bool valid = i < n;
+            key[k] = valid ? keys[i] : 0u;
+            val[k] = valid ? vals[i] : 0u;
+            const uint32_t d = valid ? ((key[k] >> shift) & mask) : 0xFFFFFFFFu;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const int leader = __ffs(peers) - 1;
+            const uint32_t pre = valid ? wcount[warp][d] : 0u;
+            __syncwarp();
+            if (valid && lane == leader) wcount[warp][d] = pre + __popc(peers);
+            __syncwarp();
+            rank[k] = pre + __popc(peers & lt);
         }
-    }
-    __syncthreads();
-    // consecutive slots of one digit go to consecutive global positions
-    const uint32_t valid_n = n > bbase ? min((uint32_t)kRadixTile, n - bbase) : 0u;
+        __syncthreads();
+        // per digit: the block's count, then each warp's start within the digit's run
+        for (int d = threadIdx.x; d < kRadixDigits; d += kRadixThreads) {
+            uint32_t run = 0;
 #pragma unroll
-    for (int k = 0; k < kRadixItems; k++) {
-        const uint32_t at = k * kRadixThreads + threadIdx.x;
-        if (at < valid_n) {
-            const uint32_t kk = skey[at];
-            const uint32_t pos = gdelta[(kk >> shift) & mask] + at;
-            keys_out[pos] = kk;
-            vals_out[pos] = sval[at];
+            for (int w = 0; w < kRadixWarps; w++) {
+                const uint32_t c = d < ndig ? wcount[w][d] : 0u;
+                wcount[w][d] = run;
+                run += c;
+            }
+            dstart[d] = run;  // the count for now
+        }
+        __syncthreads();
+        // exclusive scan of the digit counts (512 entries, 2 per thread) into block-local starts
+        {
+            const int d0 = 2 * threadIdx.x;
+            const uint32_t c0 = dstart[d0], c1 = dstart[d0 + 1];
+            uint32_t incl = c0 + c1, x = incl;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) wsum[warp] = x;
+            __syncthreads();
+            uint32_t before = 0;
+            for (int w = 0; w < warp; w++) before += wsum[w];
+            const uint32_t excl = before + x - incl;
+            __syncthreads();
+            dstart[d0] = excl;
+            dstart[d0 + 1] = excl + c0;
+            if (d0 < ndig) gdelta[d0] = hist_scan[(size_t)d0 * nblocks + b] - excl;
+            if (d0 + 1 < ndig) gdelta[d0 + 1] = hist_scan[(size_t)(d0 + 1) * nblocks + b] - (excl + c0);
+        }
+        __syncthreads();
+        // items into shared memory in digit order (stable: warp order, then item order)
+#pragma unroll
+        for (int k = 0; k < kRadixItems; k++) {
+            const uint32_t i = wbase + k * 32 + lane;
+            if (i < n) {
+                const uint32_t d = (key[k] >> shift) & mask;
+                const uint32_t at = dstart[d] + wcount[warp][d] + rank[k];
+                skey[at] = key[k];
+                sval[at] = val[k];
+            }
+        }
+        __syncthreads();
+        // consecutive slots of one digit go to consecutive global positions
+        const uint32_t valid_n = n > bbase ? min((uint32_t)kRadixTile, n - bbase) : 0u;
+#pragma unroll
+        for (int k = 0; k < kRadixItems; k++) {
+            const uint32_t at = k * kRadixThreads + threadIdx.x;
+            if (at < valid_n) {
+                const uint32_t kk = skey[at];
+                const uint32_t pos = gdelta[(kk >> shift) & mask] + at;
+                keys_out[pos] = kk;
+                vals_out[pos] = sval[at];
+            }
         }
     }
 }
@@ -833,15 +872,15 @@ int launch_bin_sort(BinArgs &a, cudaStream_t s)
     while (bits < 32 && (1u << bits) < a.ntiles) bits++;
     const int passes = (bits + 8) / 9;
     const int width = (bits + passes - 1) / passes;  // balanced digits of at most 9 bits
-    const uint32_t nb = (n + kRadixTile - 1) / kRadixTile;
+    const uint32_t nb = radix_blocks(n), grid = std::min<uint32_t>(nb, 16u * (uint32_t)std::max(1, a.sms));
     for (int shift = 0; shift < bits; shift += width) {
         const int nbits = (bits - shift) < width ? (bits - shift) : width;
         const uint32_t mask = (1u << nbits) - 1u;
-        k_radix_hist<<<nb, kRadixThreads, 0, s>>>(a.keys, n, a.total_dev, shift, mask, a.radix_hist, nb);
-        launches += 2 + launch_scan(a.radix_hist, a.radix_hist, nb * (mask + 1u), a.scan_temp, a.sort_total_dev,
-                                    a.debug, s);
-        k_radix_scatter<<<nb, kRadixThreads, 0, s>>>(a.keys, a.vals, n, a.total_dev, shift, mask, a.radix_hist, nb,
-                                                     a.keys_alt, a.vals_alt);
+        k_radix_hist<<<grid, kRadixThreads, 0, s>>>(a.keys, n, a.total_dev, shift, mask, a.radix_hist);
+        launches += 2 + start_scan<false>(a.radix_hist, a.radix_hist, nb * (mask + 1u), a.scan_temp, a.sort_total_dev, a.debug, s,
+                                          nullptr, nullptr, SortCount{a.total_dev, n, mask + 1u});
+        k_radix_scatter<<<grid, kRadixThreads, 0, s>>>(a.keys, a.vals, n, a.total_dev, shift, mask, a.radix_hist,
+                                                       a.keys_alt, a.vals_alt);
         uint32_t *tk = a.keys, *tv = a.vals;
         a.keys = a.keys_alt;
         a.vals = a.vals_alt;

@@ -130,3 +130,33 @@ def test_a_batch_settles_its_contexts_first():
             c.destroy()
     for i, (a, b) in enumerate(zip(*out)):
         harness.assert_parity(harness.compare(a, b), color_tol=1, name=f"batched after flush {i}")
+
+
+def test_small_ordered_passes_after_a_large_one():
+    """Capacities stay at the largest pass's: passes of no pair, of one, of a few and of many pairs
+    (both sides of a sort tile's 2048) follow it in the same context."""
+    w, h = 333, 257
+    out = []
+    for lib in (harness.oracle(), harness.product()):
+        ctx = lib.context(w, h)
+        ctx.glViewport(0, 0, w, h)
+        ctx.glClear(ALL)
+        quads(ctx, 900, 11, w, h)
+        ctx.glFinish()
+        frames = []
+        for n, scale in ((0, 1.0), (1, 0.01), (1, 1.0), (6, 1.0), (7, 1.0), (60, 0.3)):
+            ctx.glClear(G.GL_COLOR_BUFFER_BIT)
+            ctx.glPushMatrix()
+            ctx.glScalef(scale, scale, 1.0)
+            if n:
+                quads(ctx, n, n, w, h)
+            else:  # outside the view
+                ctx.glTranslatef(5.0, 0.0, 0.0)
+                quads(ctx, 3, 3, w, h)
+            ctx.glPopMatrix()
+            ctx.glFlush()
+            frames.append(ctx.read() + (ctx.glGetError(),))
+        out.append(frames)
+        ctx.destroy()
+    for i, (a, b) in enumerate(zip(*out)):
+        harness.assert_parity(harness.compare(a, b), color_tol=1, name=f"pass {i}")
