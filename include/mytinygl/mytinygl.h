@@ -43,7 +43,10 @@ int mtgl_reset_stats(GLState *ctx);
 /* Per-phase device timing of ctx's passes (vertex / setup / bin / tile). */
 int mtgl_set_profiling(GLState *ctx, int enable);
 int mtgl_get_timings(GLState *ctx, mtgl_timings *out);
-/* cudaStream_t of ctx, for callers that order their own GPU work with the renderer's. */
+/* cudaStream_t of ctx, for callers that order their own GPU work with the renderer's: what
+ * glFlush submitted is in the stream when it returns. (From this call on glFlush waits, on the
+ * host, until ctx's pass is counted; without it a pass that exceeds its learned capacities is
+ * run again when ctx is next used.) */
 void *mtgl_cuda_stream(GLState *ctx);
 /* Back-end option of ctx (MTGL_OPT_* in mtgl_dev.h). */
 int mtgl_set_option(GLState *ctx, int option, int value);

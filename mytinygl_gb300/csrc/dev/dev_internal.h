@@ -202,6 +202,7 @@ struct PipeConfig {
     uint32_t pair_cap = 0;
     int32_t ctas = 0;        // tile CTAs that step through the tiles (0: one CTA per tile)
     bool order = false;      // hand out tiles costliest first
+    cudaEvent_t counted = nullptr;  // capacity mode: recorded when the totals are known (may be null)
 };
 
 struct PipeOut {
@@ -236,6 +237,9 @@ struct mtgl_dev {
     bool unsettled = false;
     mtgl::Tables ran_t;
     mtgl::PipeConfig ran_c;
+    // the caller has this context's stream: a flush waits for its totals, so that a second run too is
+    // in the stream when it returns (created with the stream's first use)
+    cudaEvent_t counted = nullptr;
     // ordering against batches, which run on their own streams: work of this context's
     // stream that a batch must wait for, and a batch this context's stream must wait for
     cudaEvent_t tail = nullptr;

@@ -697,6 +697,7 @@ int run_pipeline(Exec &x, ScratchSource &sc, const HostStage &st, const Tables &
         if (!c.exact) CK(cudaMemcpyAsync(x.h_totals, x.d_totals, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         if (tile_frame) launches += launch_tile_ranges(ba, s);  // frames that only clear: their tiles' frames
     }
+    if (!c.exact && c.counted) CK(cudaEventRecord(c.counted, s));
     x.prof_mark();
 
     TileArgs ta;

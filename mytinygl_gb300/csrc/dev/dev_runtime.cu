@@ -208,6 +208,7 @@ PipeConfig capacities(const mtgl_dev *d, const Tables &t)
     pairs = std::min<uint64_t>(pairs, recs * std::max<uint32_t>(t.ntiles, 1u));
     PipeConfig c;
     c.exact = false;
+    c.counted = d->counted;
     c.rec_cap = (uint32_t)std::min<uint64_t>(recs, 0x7FFFFF00ull);
     c.pair_cap = (uint32_t)std::min<uint64_t>(pairs, kMaxEntries);
     return c;
@@ -256,6 +257,10 @@ int flush_pass(mtgl_dev *d, const HostFrame &host = HostFrame())
     d->stats.vertex_bytes += P.vbytes;
     d->stats.kernel_launches += (uint64_t)o.launches;
     P.reset();
+    if (d->unsettled && c.counted) {
+        CK(cudaEventSynchronize(c.counted));
+        if (d->x.h_totals[0] > c.rec_cap || d->x.h_totals[1] > c.pair_cap) return mtgl_dev_settle(d);
+    }
     return MTGL_OK;
 }
 
@@ -393,6 +398,7 @@ int mtgl_dev_destroy(mtgl_dev *d)
     d->stage.release();
     d->x.destroy();
     cudaEventDestroy(d->tail);
+    if (d->counted) cudaEventDestroy(d->counted);
     if (d->after_batch) mark_drop(d->after_batch);
     delete d;
     return MTGL_OK;
@@ -829,7 +835,17 @@ int mtgl_dev_timings(mtgl_dev *d, mtgl_timings *out)
     return MTGL_OK;
 }
 
-void *mtgl_dev_stream(mtgl_dev *d) { return d ? (void *)d->x.stream : nullptr; }
+void *mtgl_dev_stream(mtgl_dev *d)
+{
+    if (!d) return nullptr;
+    // whatever was flushed is in the stream, and what will be is when its flush returns
+    if (cudaSetDevice(d->device) == cudaSuccess && !d->counted &&
+        cudaEventCreateWithFlags(&d->counted, cudaEventDisableTiming) != cudaSuccess)
+        d->counted = nullptr;
+    cudaGetLastError();
+    mtgl_dev_settle(d);
+    return (void *)d->x.stream;
+}
 
 int mtgl_dev_set_option(mtgl_dev *d, int option, int value)
 {

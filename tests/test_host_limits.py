@@ -191,6 +191,28 @@ def test_a_failed_read_is_not_written_later(gpu):
     assert finish(ctx) == MTGL_OK and log(ctl)[-1] == "tile"
 
 
+def test_a_shared_stream_holds_every_flushed_pass(gpu):
+    """A caller that has the context's stream finds a pass that ran twice in it: when it asks for
+    the stream after the flush, and when it has it before."""
+    ctx, ctl = gpu
+    stream = ctx.glib.lib.mtgl_cuda_stream
+    stream.argtypes, stream.restype = [ctypes.c_void_p], ctypes.c_void_p
+    draw(ctx)
+    ctl.fake_totals(5000, 6000)
+    ctx.glFlush()
+    assert log(ctl)[-1] == "over"
+    assert stream(ctx.handle)
+    assert log(ctl) == "vertex count emit bin sort tile".split()
+    for records in (8000, 9000):
+        draw(ctx)
+        ctl.fake_totals(records, 6000)
+        ctx.glFlush()
+        assert log(ctl) == "vertex setup bin over vertex count emit bin sort tile".split()
+    draw(ctx)
+    ctx.glFlush()
+    assert log(ctl) == "vertex setup bin tile".split()
+
+
 # ---- the sums that decide it, restated
 
 MASK = 0xFFFFFFFF
