@@ -42,15 +42,23 @@ static void play_streams(play_job *j)
  * more than playing 256 frames of resident geometry takes alone (453 us; 952 us with 16 fresh
  * threads). A helper takes the first listed job that wants one, and ends after two idle
  * seconds, at library unload, or (by not existing there) in a forked child. Jobs of several
- * calling threads share the helpers; every caller also plays its own job. */
+ * calling threads share the helpers; every caller also plays its own job. Every helper is
+ * joined, by the next that ends or at unload, so that none is in this code when it goes. */
 #define PLAY_MAX_THREADS 64
 #define PLAY_IDLE_SECONDS 2
 
 static pthread_mutex_t g_mu = PTHREAD_MUTEX_INITIALIZER;
 static pthread_cond_t g_work = PTHREAD_COND_INITIALIZER; /* a job was listed, or the library unloads */
-static pthread_cond_t g_idle = PTHREAD_COND_INITIALIZER; /* a helper left its job, or ended */
+static pthread_cond_t g_idle = PTHREAD_COND_INITIALIZER; /* a helper left its job, or was started */
 static play_job *g_jobs;
-static int32_t g_helpers, g_waiting; /* alive; of those, waiting for work */
+/* A helper's place. FREE -> TAKEN (being started) -> its thread id known; it ends on its own;
+ * with both, it may be joined. */
+enum { SLOT_FREE = 0, SLOT_TAKEN = 1, SLOT_STARTED = 2, SLOT_ENDED = 4 };
+static struct play_slot {
+    pthread_t tid;
+    int state;
+} g_slot[PLAY_MAX_THREADS];
+static int32_t g_helpers, g_waiting; /* helpers not ended; of those, waiting for work */
 static int g_unload;
 
 static play_job *wanting_job(void)
@@ -60,9 +68,25 @@ static play_job *wanting_job(void)
     return NULL;
 }
 
+/* Joins the helpers that have ended (g_mu held; given up meanwhile). They hold no lock any more. */
+static void join_ended(void)
+{
+    pthread_t tid[PLAY_MAX_THREADS];
+    int n = 0;
+    for (int i = 0; i < PLAY_MAX_THREADS; i++)
+        if (g_slot[i].state == (SLOT_TAKEN | SLOT_STARTED | SLOT_ENDED)) {
+            tid[n++] = g_slot[i].tid;
+            g_slot[i].state = SLOT_FREE;
+        }
+    if (!n) return;
+    pthread_mutex_unlock(&g_mu);
+    for (int i = 0; i < n; i++) pthread_join(tid[i], NULL);
+    pthread_mutex_lock(&g_mu);
+}
+
 static void *play_helper(void *arg)
 {
-    (void)arg;
+    struct play_slot *slot = (struct play_slot *)arg;
     pthread_mutex_lock(&g_mu);
     while (!g_unload) {
         play_job *j = wanting_job();
@@ -85,8 +109,9 @@ static void *play_helper(void *arg)
         j->active--;
         pthread_cond_broadcast(&g_idle);
     }
+    if (!g_unload) join_ended();
+    slot->state |= SLOT_ENDED;
     g_helpers--;
-    pthread_cond_broadcast(&g_idle);
     pthread_mutex_unlock(&g_mu);
     return NULL;
 }
@@ -97,6 +122,7 @@ static void fork_child(void)
     pthread_cond_init(&g_work, NULL);
     pthread_cond_init(&g_idle, NULL);
     g_jobs = NULL;
+    for (int i = 0; i < PLAY_MAX_THREADS; i++) g_slot[i].state = SLOT_FREE;
     g_helpers = g_waiting = 0;
 }
 static void fork_prepare(void) { pthread_mutex_lock(&g_mu); }
@@ -109,8 +135,42 @@ __attribute__((destructor)) static void play_unload(void)
     pthread_mutex_lock(&g_mu);
     g_unload = 1;
     pthread_cond_broadcast(&g_work);
-    while (g_helpers > 0) pthread_cond_wait(&g_idle, &g_mu);
+    for (int i = 0; i < PLAY_MAX_THREADS; i++) {
+        while (g_slot[i].state != SLOT_FREE && !(g_slot[i].state & SLOT_STARTED)) pthread_cond_wait(&g_idle, &g_mu);
+        if (g_slot[i].state == SLOT_FREE || pthread_equal(g_slot[i].tid, pthread_self())) continue;
+        const pthread_t tid = g_slot[i].tid;
+        g_slot[i].state = SLOT_FREE;
+        pthread_mutex_unlock(&g_mu);
+        pthread_join(tid, NULL);
+        pthread_mutex_lock(&g_mu);
+    }
     pthread_mutex_unlock(&g_mu);
+}
+
+/* Starts a helper unless there are `want` (g_mu held; given up meanwhile, so that those already
+ * started get on with the job). Returns 0 when none is to be had. */
+static int start_helper(int32_t want)
+{
+    struct play_slot *slot = NULL;
+    if (g_unload || g_helpers >= want || g_helpers >= PLAY_MAX_THREADS) return 0;
+    for (int i = 0; i < PLAY_MAX_THREADS && !slot; i++)
+        if (g_slot[i].state == SLOT_FREE) slot = &g_slot[i];
+    if (!slot) return 0;
+    slot->state = SLOT_TAKEN;
+    g_helpers++;
+    pthread_mutex_unlock(&g_mu);
+    pthread_t tid;
+    const int failed = pthread_create(&tid, NULL, play_helper, slot);
+    pthread_mutex_lock(&g_mu);
+    if (failed) {
+        slot->state = SLOT_FREE;
+        g_helpers--;
+    } else {
+        slot->tid = tid;
+        slot->state |= SLOT_STARTED;
+    }
+    pthread_cond_broadcast(&g_idle);
+    return !failed;
 }
 
 /* Plays the job with up to `helpers` other threads; returns when every stream is played. */
@@ -124,15 +184,7 @@ static void play_shared(play_job *j, int32_t helpers)
     g_jobs = j;
     const int32_t woken = g_waiting < helpers ? g_waiting : helpers;
     for (int32_t k = 0; k < woken; k++) pthread_cond_signal(&g_work);
-    while (g_helpers < helpers && g_helpers < PLAY_MAX_THREADS) {
-        pthread_attr_t at;
-        pthread_t th;
-        pthread_attr_init(&at);
-        pthread_attr_setdetachstate(&at, PTHREAD_CREATE_DETACHED);
-        const int failed = pthread_create(&th, &at, play_helper, NULL);
-        pthread_attr_destroy(&at);
-        if (failed) break;
-        g_helpers++;
+    while (__atomic_load_n(&j->next, __ATOMIC_RELAXED) < j->n && start_helper(helpers)) {
     }
     pthread_mutex_unlock(&g_mu);
     play_streams(j); /* this thread plays too; with no helper it plays every stream in order */
