@@ -389,7 +389,8 @@ int build_tables(Exec &x, HostStage &st, const FrameSrc *frames, uint32_t nframe
         const Pass &p = *frames[f].pass;
         const mtgl_dev *d = frames[f].dev;
         uint8_t *data = ds + frames[f].data_off;
-        bool occlude = !p.draws.empty(), triangles = true;
+        // (binning packs a box's corners into 16 bits each for it)
+        bool occlude = !p.draws.empty() && d->width <= 65536 && d->height <= 65536, triangles = true;
         uint32_t frame_rule = 0;
         for (const PendingDraw &pd : p.draws) {
             DevDraw dd = pd.d;

@@ -26,6 +26,34 @@ void fake_totals(uint32_t records, uint32_t pairs)
 }
 const char *fake_log() { return g_log.c_str(); }
 void fake_log_clear() { g_log.clear(); }
+// whether binning may drop hidden pairs of a w x h frame of one opaque depth-tested triangle
+int fake_occludes(int32_t w, int32_t h)
+{
+    mtgl_dev *d = nullptr;
+    if (mtgl_dev_create(w, h, &d) != MTGL_OK) return -1;
+    DevRaster R;
+    memset(&R, 0, sizeof(R));
+    R.rs.polygon_mode_front = R.rs.polygon_mode_back = GL_FILL;
+    R.rs.depth_func = GL_LESS;
+    R.depth_rejection = 1;
+    R.fs.ctl = FC_DEPTH | FC_DEPTH_WRITE | FC_MASK_ALL;
+    PendingDraw p;
+    memset(&p.d, 0, sizeof(p.d));
+    p.d.mode = GL_TRIANGLES;
+    p.d.tri_count = 1;
+    d->pass.rasters.push_back(R);
+    d->pass.draws.push_back(p);
+    d->pass.tris = 1;
+    FrameSrc fs{d, &d->pass, 0, HostFrame()};
+    Tables t;
+    int r = -1;
+    if (build_tables(d->x, d->stage, &fs, 1, kTileShiftPlain, true, t) == MTGL_OK)
+        r = (int)reinterpret_cast<const DevFrame *>(d->stage.p + t.off_frames)->occlude;
+    if ((t.occlude ? 1 : 0) != r) r = -1;
+    d->pass.reset();
+    mtgl_dev_destroy(d);
+    return r;
+}
 }
 
 namespace mtgl {

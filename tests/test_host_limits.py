@@ -213,6 +213,13 @@ def test_a_shared_stream_holds_every_flushed_pass(gpu):
     assert log(ctl) == "vertex setup bin tile".split()
 
 
+@pytest.mark.parametrize("size,occludes", [((64, 48), 1), ((65536, 2), 1), ((2, 65536), 1), ((65537, 2), 0), ((2, 70000), 0)])
+def test_hidden_pairs_are_dropped_where_coordinates_fit(fake, size, occludes):
+    """Binning packs pixel coordinates of a record's box into 16 bits to test it against a tile's
+    occlusion bound. (gl_create_context stops at 16384; mtgl_dev_create takes any size.)"""
+    assert fake[1].fake_occludes(*size) == occludes
+
+
 # ---- the sums that decide it, restated
 
 MASK = 0xFFFFFFFF
