@@ -479,3 +479,127 @@ def test_tile_row_by_reciprocal():
         q = (local * np.uint64(0xFFFFFFFF // n)) >> np.uint64(32)
         q = np.where(local - q * n >= n, q + 1, q)
         assert np.array_equal(q, local // n), n
+
+
+# ---- the block tests of the tile kernels (k_tile.cuh) and the whole-tile test of binning (k_bin.cu)
+
+def _corner_test_f32(edges, area, xl, xh, yl, yh):
+    """corner_test: (some pixel of the rectangle may be covered, all are)."""
+    f = np.float32
+    sg = f(1) if area > 0 else f(-1)
+    some = every = area > 0 or area < 0
+    for ax, ay, A, B in edges:
+        a, b = A * sg, B * sg
+        p = [(f(x) - ax) * a for x in (xl, xh)]
+        r = [(f(y) - ay) * b for y in (yl, yh)]
+        some = some and max(p) >= min(r)
+        every = every and min(p) >= max(r)
+    return bool(some), bool(every)
+
+
+def _tri_mask_f32(edges, area, wx0, wy0):
+    """tri_mask: the covered pixels of the 8x4 block, bit 8 * row + column."""
+    f = np.float32
+    sg = f(1) if area > 0 else f(-1)
+    x, y = np.arange(wx0, wx0 + 8, dtype=f), np.arange(wy0, wy0 + 4, dtype=f)
+    m = np.ones((4, 8), bool)
+    for ax, ay, A, B in edges:
+        m &= ((x - ax) * (A * sg))[None, :] >= ((y - ay) * (B * sg))[:, None]
+    return sum(1 << (8 * r + c) for r in range(4) for c in range(8) if m[r, c])
+
+
+def _box_mask(box, wx0, wy0):
+    mnx, mny, mxx, mxy = box
+    c0, c1 = max(mnx - wx0, 0), min(mxx - wx0, 7)
+    r0, r1 = max(mny - wy0, 0), min(mxy - wy0, 3)
+    if c0 > c1 or r0 > r1:
+        return 0
+    cols = (0xFF >> (7 - c1)) & (0xFF << c0) & 0xFFFFFFFF
+    return (cols * 0x01010101 & 0xFFFFFFFF) & (0xFFFFFFFF >> (8 * (3 - r1))) & (0xFFFFFFFF << (8 * r0) & 0xFFFFFFFF)
+
+
+def _covered_tiles_int(edges, area, box, ts, W, H):
+    """box_of with OCCLUDE and take_bound's coverage: the tiles held to be covered whole, with their
+    pixels' ranges (clipped to the framebuffer); None when an edge may be inexact."""
+    mnx, mny, mxx, mxy = box
+    tx0, ty0 = -(-mnx // ts), -(-mny // ts)
+    tx1 = (W - 1) // ts if mxx == W - 1 else (mxx + 1) // ts - 1
+    ty1 = (H - 1) // ts if mxy == H - 1 else (mxy + 1) // ts - 1
+    if tx1 < tx0 or ty1 < ty0:
+        return []
+    xl, xh, yl, yh = tx0 * ts, tx1 * ts + ts - 1, ty0 * ts, ty1 * ts + ts - 1
+    steps = []
+    for ax, ay, A, B in edges:
+        if not all(abs(v) < 2 ** 24 for v in (ax, ay, A, B)):
+            return None
+        ax, ay, A, B = int(ax), int(ay), int(A), int(B)
+        a, b = (A, B) if area > 0 else (-A, -B)
+        if max(abs(xl - ax), abs(xh - ax)) * abs(a) >= 1 << 24 or max(abs(yl - ay), abs(yh - ay)) * abs(b) >= 1 << 24:
+            return None
+        right, bottom = a < 0, b >= 0
+        e00 = (xl + (ts - 1 if right else 0) - ax) * a - (yl + (ts - 1 if bottom else 0) - ay) * b
+        steps.append((e00, a * ts, b * ts))
+    out = []
+    for ty in range(ty0, ty1 + 1):
+        for tx in range(tx0, tx1 + 1):
+            x0, y0 = tx * ts, ty * ts
+            cx, cy = max(x0 + ts - (mxx + 1), 0), max(y0 + ts - (mxy + 1), 0)
+            if all(e00 + (tx - tx0) * sx - (ty - ty0) * sy + max(-(sx // ts), 0) * cx + max(sy // ts, 0) * cy >= 0
+                   for e00, sx, sy in steps):
+                out.append((x0, x0 + ts - 1 - cx, y0, y0 + ts - 1 - cy))
+    return out
+
+
+def test_block_tests_agree_with_every_pixel():
+    """Random integer triangles (small, large, slivers, both orientations, vertices far outside, where
+    the products round): per 8x4 block, `any` false means no pixel passes the per-pixel float32
+    test, `all` true that every one does, and the masks are the pixels that pass it inside the box.
+    Every tile that binning takes an occlusion bound from is covered whole, at the framebuffer's
+    right and bottom sides too."""
+    f = np.float32
+    rng = np.random.default_rng(17)
+    none = whole = mixed = bounds = edge_bounds = 0
+    for k in range(900):
+        W, H = int(rng.integers(20, 220)), int(rng.integers(20, 220))
+        scale = [8, 60, 400, 3000][k % 4]
+        far = 0 if k % 5 else int(rng.integers(-40_000_000, 40_000_000))
+        xs = [W // 2 + int(v) for v in rng.integers(-scale, scale + 1, 3)]
+        ys = [H // 2 + int(v) for v in rng.integers(-scale, scale + 1, 3)]
+        if k % 9 == 0:
+            xs[2], ys[2] = (xs[0] + xs[1]) // 2, (ys[0] + ys[1]) // 2 + int(rng.integers(-1, 2))  # sliver
+        xs[0] += far
+        X, Y = [f(v) for v in xs], [f(v) for v in ys]
+        area = (X[2] - X[0]) * (Y[1] - Y[0]) - (Y[2] - Y[0]) * (X[1] - X[0])
+        edges = _edges(*[v for p in zip(xs, ys) for v in p])
+        box = (max(min(xs), 0), max(min(ys), 0), min(max(xs), W - 1), min(max(ys), H - 1))
+        if box[0] > box[2] or box[1] > box[3]:
+            continue
+        gx, gy = np.meshgrid(np.arange(W, dtype=f), np.arange(H, dtype=f))
+        e = [(gx - ax) * A - (gy - ay) * B for ax, ay, A, B in edges]
+        if area > 0:
+            cov = (e[0] >= 0) & (e[1] >= 0) & (e[2] >= 0)
+        elif area < 0:
+            cov = (e[0] <= 0) & (e[1] <= 0) & (e[2] <= 0)
+        else:
+            cov = np.zeros((H, W), bool)
+        for _ in range(40):
+            wx0, wy0 = 8 * int(rng.integers(box[0] // 8, box[2] // 8 + 1)), 4 * int(rng.integers(box[1] // 4, box[3] // 4 + 1))
+            xl, xh = max(wx0, box[0]), min(wx0 + 7, box[2])
+            yl, yh = max(wy0, box[1]), min(wy0 + 3, box[3])
+            sub = cov[yl:yh + 1, xl:xh + 1]
+            some, every = _corner_test_f32(edges, area, xl, xh, yl, yh)
+            assert some or not sub.any(), (k, wx0, wy0)
+            assert not every or sub.all(), (k, wx0, wy0)
+            none, whole, mixed = none + (not some), whole + every, mixed + (some and not every)
+            if not (area > 0 or area < 0):
+                continue  # such a record is in no block
+            want = sum(1 << (8 * (y - wy0) + x - wx0) for y in range(yl, yh + 1) for x in range(xl, xh + 1) if cov[y, x])
+            assert _box_mask(box, wx0, wy0) & _tri_mask_f32(edges, area, wx0, wy0) == want, (k, wx0, wy0)
+        if not (area > 0 or area < 0):
+            continue
+        ts = [8, 16, 32][k % 3]
+        for x0, x1, y0, y1 in _covered_tiles_int(edges, area, box, ts, W, H) or []:
+            assert cov[y0:y1 + 1, x0:x1 + 1].all(), (k, ts, x0, y0)
+            bounds += 1
+            edge_bounds += x1 - x0 + 1 < ts or y1 - y0 + 1 < ts
+    assert none > 3000 and whole > 3000 and mixed > 3000 and bounds > 2000 and edge_bounds > 100
