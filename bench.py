@@ -744,7 +744,7 @@ def run_batch(args, spec):
         "data": "synthetic (seeded; mytinygl_gb300/workloads.py uneven_batch)",
         "config": batch_config(spec, scenes, world),
         "pipeline": {"setup_triangles_per_step": int(rec), "bin_entries_per_step": int(pairs),
-                     "tile": bst["tile_size"], "persistent_ctas": bst["ctas"],
+                     "tile": bst["tile_size"], "tile_ctas": bst["ctas"],
                      "record_capacity": bst["record_capacity"], "pair_capacity": bst["pair_capacity"],
                      "graph_replays": bst["graph_replays"], "graph_captures": bst["graph_captures"]},
         "batched_wall_frames_per_s": round(batched_wall_fps, 2),

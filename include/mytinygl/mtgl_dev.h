@@ -256,7 +256,8 @@ typedef struct mtgl_batch mtgl_batch;
 
 typedef struct {
     int32_t tile_size;       /* 8, 16 or 32 pixels; 0: the tuned default                    */
-    int32_t ctas_per_sm;     /* persistent tile CTAs per SM; 0: the tuned default           */
+    int32_t ctas_per_sm;     /* fewer tile CTAs per SM than fit step through the tiles; as
+                                many or more: a CTA per tile; 0: the tuned default          */
     float record_factor;     /* initial record capacity per input triangle; 0: default      */
     float pair_factor;       /* initial tile-pair capacity per record; 0: default           */
     int32_t use_graph;       /* 1: capture the run in a CUDA graph and replay it; 0: launch */
@@ -270,7 +271,7 @@ typedef struct {
     uint64_t batches, frames, input_triangles, setup_triangles, bin_entries, fragments;
     uint64_t graph_captures, graph_replays, overflow_reruns, kernel_launches;
     uint32_t record_capacity, pair_capacity;
-    int32_t tile_size, ctas;
+    int32_t tile_size, ctas;         /* ctas: of the last run's tile launch */
     uint64_t vertices, vertex_bytes; /* as in mtgl_stats, over the batch's passes */
     uint64_t debug_status;           /* as in mtgl_stats */
 } mtgl_batch_stats;

@@ -79,7 +79,7 @@ def main():
                 ms, st = time_config(lib, ctxs, streams, args.steps, tile_size=tile, ctas_per_sm=ctas,
                                      order_by_cost=order)
                 r = dict(tile_size=tile, ctas_per_sm=ctas, order_by_cost=order, ms=round(ms, 3),
-                         frames_per_s=round(args.frames / (ms / 1e3), 1), persistent_ctas=st["ctas"],
+                         frames_per_s=round(args.frames / (ms / 1e3), 1), tile_ctas=st["ctas"],
                          records=st["setup_triangles"] // max(1, st["batches"]),
                          pairs=st["bin_entries"] // max(1, st["batches"]))
                 results.append(r)

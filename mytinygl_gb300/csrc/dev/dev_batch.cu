@@ -460,7 +460,7 @@ int mtgl_dev_batch_launch(mtgl_batch *b)
         b->stats.vertices += p.slots;
         b->stats.vertex_bytes += p.vbytes;
     }
-    b->stats.ctas = resident;
+    b->stats.ctas = (int32_t)(limited ? std::min<uint32_t>((uint32_t)resident, b->t.ntiles) : b->t.ntiles);
     return MTGL_OK;
 }
 

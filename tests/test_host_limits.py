@@ -220,6 +220,21 @@ def test_hidden_pairs_are_dropped_where_coordinates_fit(fake, size, occludes):
     assert fake[1].fake_occludes(*size) == occludes
 
 
+@pytest.mark.parametrize("per_sm,side,ctas", [(0, 1024, 64 * 64), (4, 1024, 64 * 64), (3, 1024, 3 * 152), (1, 32, 4)])
+def test_batch_stats_count_the_launched_ctas(fake, gpu, per_sm, side, ctas):
+    """Tiles of 16 pixels, four CTAs resident per SM of 152: one per tile unless fewer than fit are
+    asked for, and never more than tiles."""
+    lib = fake[0]
+    ctx = lib.context(side, side)
+    b = lib.batch(use_graph=0, tile_size=16, ctas_per_sm=per_sm)
+    draw(ctx)
+    b.render([ctx])
+    b.wait()
+    assert b.stats()["ctas"] == ctas
+    b.destroy()
+    ctx.destroy()
+
+
 # ---- the sums that decide it, restated
 
 MASK = 0xFFFFFFFF
