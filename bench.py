@@ -4,8 +4,8 @@
 Workload (default `batch`): 256 independent frames per step — sides log-uniform 64-1024,
 triangle counts log-uniform 100-200k, each a lit UV sphere or a textured frame with ~30 %
 clipped triangles (p = 1/2), with its own modelview, lights and 256x256 mipmapped texture —
-rendered by one batched pipeline run (mtgl_batch_render: persistent tile kernel over all
-frames, CUDA graph replay), and compared with the plain per-frame path on the same frames.
+rendered by one batched pipeline run (mtgl_batch_render: one tile launch over all frames,
+CUDA graph replay), and compared with the plain per-frame path on the same frames.
 Other workloads: `textured` (1920x1080, 100k clip-straddling triangles, 512^2 trilinear
 texture, 8 point lights, EXP fog), `rop` (1920x1080, 1M small blended triangles with
 alpha, stencil and depth tests), `sphere` (800x600 lit UV sphere), `serve` (Poisson
@@ -149,9 +149,9 @@ def stage_rooflines(workload, vertices, vertex_bytes, rec, pairs, npix, tex, pha
     written once) over its measured time, and K4's issue-slot fraction: warp instructions
     per launch (ncu) over the issue slots of its measured time (SMs x 4 schedulers x clock).
       K1 vertex:  attribute bytes read + vertices x 48 (post-transform vertex written)
-      K2 setup:   vertices x 48 (read once) + records x 224 (written)
+      K2 setup:   vertices x 48 (read once) + records x 240 (written)
       K3 binning: records x 80 (box and edge words read) + pairs x 8 (written)
-      K4 tile:    pixels x 9 + pairs x 4 + records x 224 + texture bytes"""
+      K4 tile:    pixels x 9 + pairs x 4 + records x 240 + texture bytes"""
     stages = {
         "k1_vertex": (vertex_bytes + vertices * POST_VERTEX_BYTES, phase_ms.get("vertex")),
         "k2_setup": (vertices * POST_VERTEX_BYTES + rec * REC_BYTES, phase_ms.get("setup")),
@@ -757,7 +757,7 @@ def run_batch(args, spec):
         "phase_ms": {"vertex": round(tm["vertex_ms"] / passes, 4), "setup": round(tm["setup_ms"] / passes, 4),
                      "bin": round(tm["bin_ms"] / passes, 4), "tile": round(k4_ms, 4)},
         "wall_ms_per_step": round(wall * 1e3 / args.steps, 4),
-        "roofline": {"kernel": "k_tile (K4 tile raster/ROP, persistent over all frames)", "bound": "hbm",
+        "roofline": {"kernel": "k_tile_free (K4 tile raster/ROP, order-free, all frames)", "bound": "hbm",
                      "achieved": round(achieved, 2) if achieved else None, "peak": peak,
                      "peak_source": f"{peak_src} (HBM copy)", "unit": "GB/s",
                      "frac": round(achieved / peak, 5) if achieved else None,

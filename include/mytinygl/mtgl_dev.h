@@ -224,8 +224,12 @@ void *mtgl_dev_stream(mtgl_dev *d);
 
 /* Per-context options. MTGL_OPT_DEPTH_REJECTION (default 1): the tile kernel skips, per
  * warp, triangles none of whose fragments can pass GL_LESS/GL_LEQUAL/GL_NEVER while the
- * stencil test is off. Rendering is identical either way; with it off every covered
- * fragment is counted in mtgl_stats.fragments. Applies to draws queued afterwards. */
+ * stencil test is off, and binning drops them from tiles that a nearer triangle covers.
+ * Rendering is identical either way; with it off every covered fragment is counted in
+ * mtgl_stats.fragments. With it on, the count of passes whose result does not depend on the
+ * order of their triangles varies a little between runs: their tiles' lists come in whatever
+ * order they were written, and what is skipped depends on it. Applies to draws queued
+ * afterwards. */
 #define MTGL_OPT_DEPTH_REJECTION 1
 /* MTGL_OPT_MIPMAP_CHAIN (default 0): an extension with no counterpart in MyTinyGL, whose
  * glTexImage2D accepts level 0 only and whose sampler knows level 0 and one derived level
@@ -244,10 +248,10 @@ int mtgl_dev_set_option(mtgl_dev *d, int option, int value);
  * takes the pending pass (clears, then draws) of each of n contexts of one device, each
  * with its own framebuffer size and GL state, and renders them all with one run of the
  * pipeline: one vertex launch, one setup launch, one binning pass over the tiles of all
- * frames, and one persistent tile launch whose CTAs take (frame, tile) work items from a
- * device queue, costliest first. The run enqueues without host waits and is captured in a
- * CUDA graph, replayed while the batch keeps its shape. Every framebuffer ends up exactly
- * as rendering each context alone would leave it.
+ * frames, and one tile launch over them (a CTA per tile, in frame order unless the config
+ * says otherwise). The run enqueues without host waits and is captured in a CUDA graph,
+ * replayed while the batch keeps its shape. Every framebuffer ends up exactly as rendering
+ * each context alone would leave it.
  *
  * Record and tile-pair buffers have fixed capacities (set from the config, then from the
  * largest totals seen). A run that exceeds one leaves every framebuffer untouched;
@@ -263,8 +267,10 @@ typedef struct {
     int32_t use_graph;       /* 1: capture the run in a CUDA graph and replay it; 0: launch */
     int32_t order_by_cost;   /* 1: hand out the costliest tiles first; 0: in frame order    */
     int32_t readback_kernel; /* 1: colour read-backs into mapped page-locked host memory are
-                                written by a kernel (one launch per 128 frames); 0: one copy
-                                call per frame. Other destinations are always copied.       */
+                                written by the tile launch (frames of 2^12 pixels and more
+                                that the run renders) or by a kernel (the others, one launch
+                                per 128 frames); 0: one copy call per frame. Other
+                                destinations are always copied.                             */
 } mtgl_batch_config;
 
 typedef struct {

@@ -83,8 +83,9 @@ int mtgl_batch_render(mtgl_batch *b, GLState *const *ctxs, int32_t n);
  * packed RGBA8, row 0 = top) into colors[i]; NULL entries (or a NULL colors) copy nothing.
  * The copies have landed when mtgl_dev_batch_wait returns; page-locked destinations keep
  * them asynchronous. Each colors[i] must hold the frame's width * height pixels: those in
- * page-locked memory the device maps are written by a read-back kernel (one launch per 128
- * frames) unless mtgl_batch_config.readback_kernel is 0, the others are copied. */
+ * page-locked memory the device maps are written by the run's tile launch (frames of 2^12
+ * pixels and more) or by a read-back kernel (smaller ones, one launch per 128 frames) unless
+ * mtgl_batch_config.readback_kernel is 0, the others are copied. */
 int mtgl_batch_render_read(mtgl_batch *b, GLState *const *ctxs, uint32_t *const *colors, int32_t n);
 
 /* Replay a GL command stream onto ctx (made current). No counterpart in the reference.

@@ -1,6 +1,7 @@
-"""Autotuner of the batched renderer: tile size, persistent CTAs per SM, work order (costliest
-tiles first, or frame order) and the record / tile-pair capacity factors, measured on the
-uneven-batch workload on this GPU.
+"""Autotuner of the batched renderer: tile size, tile CTAs per SM, work order (costliest tiles
+first, or frame order) and the record / tile-pair capacity factors, measured on the
+uneven-batch workload on this GPU. The factors are of the same frames with depth rejection off:
+a batch's first run has to hold the pairs of frames in which nothing hides anything.
 
     python -m mytinygl_gb300.autotune [--frames 256] [--steps 5]
 
@@ -26,6 +27,7 @@ from .gl import PreparedStreams
 HERE = os.path.dirname(os.path.abspath(__file__))
 TUNED_JSON = os.path.join(HERE, "tuned.json")
 TUNED_H = os.path.join(HERE, "csrc", "dev", "tuned.h")
+MTGL_OPT_DEPTH_REJECTION = 1
 
 
 def setup(lib, scenes):
@@ -72,7 +74,7 @@ def main():
     tris = sum(W.scene_triangles(s) for s in scenes)
     results = []
     for tile in (8, 16, 32):
-        for ctas in (0, 1, 2, 4, 8):
+        for ctas in (1, 2, 4, 8):  # (0 would be the default this chooses)
             if tile == 32 and ctas > 1:
                 continue  # a 32x32 CTA is 1024 threads: one fits an SM
             for order in (1, 0):
@@ -86,8 +88,12 @@ def main():
                 print(json.dumps(r), flush=True)
     best = min(results, key=lambda r: r["ms"])
     # capacity factors: the measured totals of the best tile size with 1/8 headroom
-    rec_factor = math.ceil(best["records"] / max(1, tris) * 1.125 * 100) / 100
-    pair_factor = math.ceil(best["pairs"] / max(1, best["records"]) * 1.125 * 10) / 10
+    for c in ctxs:
+        lib.lib.mtgl_set_option(c.handle, MTGL_OPT_DEPTH_REJECTION, 0)
+    _, st = time_config(lib, ctxs, streams, 1, tile_size=best["tile_size"])
+    records, pairs = (st[k] // max(1, st["batches"]) for k in ("setup_triangles", "bin_entries"))
+    rec_factor = math.ceil(records / max(1, tris) * 1.125 * 100) / 100
+    pair_factor = math.ceil(pairs / max(1, records) * 1.125 * 10) / 10
     out = {"workload": f"uneven_batch({args.frames}, seed={args.seed})", "input_triangles": tris,
            "best": best, "record_factor": rec_factor, "pair_factor": pair_factor, "results": results}
     with open(TUNED_JSON, "w") as f:

@@ -186,8 +186,8 @@ int run_clears_only(mtgl_dev *d)
 // Capacities of a pass's records and pairs: the largest totals the context has seen, or for its
 // first passes an estimate: a record per filled triangle, three for polygon modes drawn as
 // points or lines, as many again in small passes for what clipping splits (sprites across the
-// screen's edge made up to 1.6 times their triangles) and an eighth in large ones; four pairs per record, and at least 2^18 (a few megabytes) unless the frame
-// cannot have that many. Totals beyond them cost one more run of the pass (mtgl_dev_settle).
+// screen's edge made up to 1.6 times their triangles) and an eighth in large ones; four pairs
+// per record, and at least 2^18 (a few megabytes) unless the frame cannot have that many. Totals beyond them cost one more run of the pass (mtgl_dev_settle).
 // A pass of more than 2^22 primitives, whose records may be gigabytes of which few are
 // needed, takes exact sizes instead: its two waits are nothing beside it. So does one whose
 // estimate finds no memory (flush_pass).

@@ -666,7 +666,7 @@ int launch_bin_expand(const BinArgs &a, cudaStream_t s)
     return 1;
 }
 
-// ------------------------------------------------------------------ persistent work order
+// ------------------------------------------------------------------ work order of the tile launch
 
 // coarse log2 bucket of a tile's record count: 8 steps per octave, 0 for an empty tile
 __device__ __forceinline__ uint32_t cost_bucket(uint32_t c)

@@ -58,7 +58,8 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// 32x32 bit transpose across the warp: bit i of lane l becomes bit l of lane i.
+// 32x32 bit transpose across the warp: bit i of lane l becomes bit l of lane i (block swaps of
+// halving size: Warren, "Hacker's Delight", 7-3, with lanes for words).
 __device__ __forceinline__ uint32_t warp_transpose(uint32_t v)
 {
     const uint32_t lane = threadIdx.x & 31u;

@@ -99,7 +99,6 @@ constexpr int kRecTypeShift = 4;
 // GL_NEVER. The tile kernel's tests read them with the edge
 // coefficients (same 16-byte word) instead of through the raster state.
 constexpr int kRecCtlShift = 8, kRecDepthFuncShift = 20;
-__device__ __forceinline__ uint32_t rec_type(const float *r) { return (__float_as_uint(r[R_FLAGS]) >> kRecTypeShift) & 3u; }
 
 // Lower bound of the depth of every fragment a triangle record can write in the rectangle
 // [xl, xh] x [yl, yh] of its box (inclusive pixel positions, inside the record's box).

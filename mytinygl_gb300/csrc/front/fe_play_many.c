@@ -4,9 +4,9 @@
  * No counterpart in the reference, where one thread drives one current context
  * (gl_api.c:14-23). Contexts share no front-end state and, outside an unfinished batch (one
  * writing their framebuffer or reading their resources), no back-end state either, so
- * distinct contexts play on a pool of threads, kept between calls: each thread claims the next unplayed stream
- * (longest first), makes its context current and plays it. Staging copies, index scans and state snapshots of
- * different frames then run on all host cores instead of one.
+ * distinct contexts play on a pool of threads, kept between calls: each thread claims the next
+ * unplayed stream (longest first), makes its context current and plays it. Staging copies,
+ * index scans and state snapshots of different frames then run on all host cores instead of one.
  */
 #include <errno.h>
 #include <pthread.h>
